@@ -262,7 +262,7 @@ void Sim::write_checkpoint(const std::string& dir) {
     if (mg_warm_ && mac_prev_ok_) {  // the MAC projection's warm start: a restart continues bit for bit
         std::vector<double> h((size_t)g_.N);
         sync();
-        ck(cudaMemcpy(h.data(), mac_phi_prev_.p, sizeof(double) * g_.N, cudaMemcpyDeviceToHost), "D2H");
+        ck(cudaMemcpy(h.data(), mac_phi_last_, sizeof(double) * g_.N, cudaMemcpyDeviceToHost), "D2H");
         write_vismf(dir + "/Level_0/mac_phi", 1, 0, 0, hi, grown(h, 1, n, 0, g_.zper));
     }
     {  // nodal p on the nodes 0..n in every direction (periodic duplicates wrapped)
@@ -348,6 +348,7 @@ void Sim::read_checkpoint(const std::string& dir) {
         if (!m.empty()) {
             if (mac_phi_prev_.n != (size_t)g_.N) mac_phi_prev_.alloc(g_.N);
             ck(cudaMemcpy(mac_phi_prev_.p, m.data(), sizeof(double) * g_.N, cudaMemcpyHostToDevice), "H2D");
+            mac_phi_last_ = mac_phi_prev_.p;
             mac_prev_ok_ = true;
         }
     }

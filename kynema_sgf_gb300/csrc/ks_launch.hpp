@@ -400,4 +400,25 @@ template <typename T>
 void launch_nd_bottom(Ctx& c, const NDLevelT<T>& L, double sigma, double omega, int sweeps);
 void launch_add_f32(Ctx& c, double* phi, const float* e, long long n);
 
+// ---- direct Poisson solves by Fourier transforms in x and y (ks_spectral.cu), FP64
+constexpr int kSpectralMax = 4096;  // longest transform (its two exchange buffers fit one block's shared memory)
+// The tridiagonal z systems of one operator's horizontal modes: eigenvalues
+// of the 1D stiffness (lx, ly) and mass (mx, my; nodal) stencils for kx <= nx/2
+// and ky <= ny/2, inverse pivots dinv[k][mode] and, for cyclic z, the
+// eliminated unknown's column w[k][mode] and inverse Schur complement.
+struct SpectralZ {
+    int nx, ny, nz;  // transform lengths and points per z column
+    int zper, nodal;
+    double iz2;
+    const double *lx, *ly, *mx, *my;
+    double *dinv, *w, *schur;
+};
+// radices of a transform of length n; false if n has a prime factor above 13 or exceeds kSpectralMax
+bool spectral_radices(int n, int& np, int r[12]);
+bool spectral_prepare_device();
+void launch_spectral_setup(Ctx& c, const SpectralZ& Z);
+// phi = scale * (unscaled operator)^-1 rhs; work: (nz + 1) / 2 * 2 nx ny doubles, 16-byte aligned
+void launch_spectral_solve(Ctx& c, const SpectralZ& Z, const double2* tw_x, const double2* tw_y, const double* rhs, double* phi, double* work,
+                           double scale);
+
 }  // namespace ks

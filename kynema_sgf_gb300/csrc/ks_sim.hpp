@@ -248,6 +248,7 @@ class Sim {
     void apply_predictor(bool incremental);
     void apply_corrector();
     void apply_projection(double time, double scaling, bool incremental);
+    void projection_alone(double time, double scaling, bool incremental);
     int step();
     bool godunov() const { return godunov_; }
 
@@ -410,6 +411,20 @@ class Sim {
     std::vector<double> binv_ccs_h_;
     DevBuf<double> mgbufs_, binvs_;
     DevBuf<float> mgbufs32_, binvs32_;
+    // direct start of the Poisson solves: the factors of one operator (false: not available),
+    // and the solves of a step that take it
+    bool spectral_setup(bool nodal);
+    void spectral_choose();
+    void spectral_start(const SpectralZ& Z, const double* rhs, double* phi, double coef, int np);
+    void spectral_norms(int np, double& bnorm, double& rnorm);
+    int nod_bparts_ = 0;  // block maxima of |rhs| that nd_rhs left in parts_ for the direct start
+    bool mac_direct_ = false, nod_direct_ = false;
+    bool nod_alone_ = false;  // inside projection_alone, with the nodal factors at hand
+    bool direct_start(bool solve) const { return solve && mg_warm_ && !mixed_; }
+    SpectralZ zmac_{}, znod_{};
+    DevBuf<double> spec_tab_, spec_mac_, spec_nod_;  // roots and eigenvalues; z factors
+    const double2 *tw_x_ = nullptr, *tw_y_ = nullptr;
+    const double* mac_phi_last_ = nullptr;  // where the last MAC potential is held (mac_prev_ok_)
     int mg_warm_ = 1;          // ks.mg_warm_start
     bool mac_prev_ok_ = false; // mac_phi_prev_ holds the last MAC potential
     DevBuf<double> mac_phi_prev_;
