@@ -1374,33 +1374,6 @@ __global__ void k_objective(Grid g, const double* u, int lo0, int lo1, int lo2, 
     if (threadIdx.x == 0) parts[blockIdx.x] = s * invM;
 }
 
-// disk adjoint: partial sums over the cut-off box of  sum_x (actb(x) . n) B(x),
-// B(x) = sum_points w_p g3(x - p) with the per-point weights w_p in pts[4p+3]
-__global__ void k_act_adj_dot(Grid g, const double* actb, const double* pts, int npts, double ax0, double ax1, double ax2, double eps, double x0,
-                              double y0, double z0, int lo0, int lo1, int lo2, int n0, int n1, int n2, double* parts) {
-    __shared__ double sh[256];
-    double acc = 0.0;
-    const long long M = (long long)n0 * n1 * n2;
-    const double gfac = 0.17958712212516656 / (eps * eps * eps);
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < M; t += (long long)gridDim.x * blockDim.x) {
-        const int a = (int)(t % n0);
-        const long long r = t / n0;
-        const int b = (int)(r % n1), c = (int)(r / n1);
-        const int i = lo0 + a, j = lo1 + b, k = lo2 + c;
-        const double x = x0 + (i + 0.5) * g.dx, y = y0 + (j + 0.5) * g.dy, z = z0 + (k + 0.5) * g.dz;
-        double s = 0;
-        for (int m = 0; m < npts; ++m) {
-            const double rx = (pts[4 * m] - x) / eps, ry = (pts[4 * m + 1] - y) / eps, rz = (pts[4 * m + 2] - z) / eps;
-            const double r2 = rx * rx + ry * ry + rz * rz;
-            if (r2 < 16.0) s += gfac * exp(-rx * rx - ry * ry - rz * rz) * pts[4 * m + 3];
-        }
-        const long long cc = cidx(g, i, j, k);
-        acc += s * (actb[cc] * ax0 + actb[g.N + cc] * ax1 + actb[2 * g.N + cc] * ax2);
-    }
-    acc = block_sum(acc, sh);
-    if (threadIdx.x == 0) parts[blockIdx.x] = acc;
-}
-
 // scatter of the sampled-velocity adjoint to the trilinear corners
 __global__ void k_act_sample_adj(Grid g, const double* pts, const double* wb, int npts, double x0, double y0, double z0, double* ub) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1624,13 +1597,6 @@ void launch_axpby(Ctx& c, long long n, double a, const double* x, double b, cons
 void launch_objective(Ctx& c, const Grid& g, const double* u, const int lo[3], const int hi[3], double invM, double* ub, double* parts, int* np) {
     *np = 1216;
     KS_LAUNCH(c, k_objective, *np, 256, B8 * 6.0 * g.N, g, u, lo[0], lo[1], lo[2], hi[0], hi[1], hi[2], invM, ub, parts);
-}
-void launch_act_adj_dot(Ctx& c, const Grid& g, const double* actb, const double* pts, int npts, const double ax[3], double eps, const double plo[3],
-                        const int lo[3], const int hi[3], double* parts, int* np) {
-    const int n0 = hi[0] - lo[0] + 1, n1 = hi[1] - lo[1] + 1, n2 = hi[2] - lo[2] + 1;
-    *np = 1216;
-    KS_LAUNCH(c, k_act_adj_dot, *np, 256, B8 * 3.0 * n0 * n1 * n2, g, actb, pts, npts, ax[0], ax[1], ax[2], eps, plo[0], plo[1], plo[2], lo[0],
-              lo[1], lo[2], n0, n1, n2, parts);
 }
 void launch_act_sample_adj(Ctx& c, const Grid& g, const double* pts, const double* wb, int npts, const double plo[3], double* ub) {
     KS_LAUNCH(c, k_act_sample_adj, nblocks(npts, 64), 64, B8 * 30.0 * npts, g, pts, wb, npts, plo[0], plo[1], plo[2], ub);

@@ -106,10 +106,9 @@ void Sim::adj_alloc() {
                 G2.tr[a][b][n] = nullptr;
                 if (a != b) { G2.tr[a][b][n] = q; q += fsz[a]; }
             }
-    size_t maxpts = 1;
-    for (auto& d : disks_) maxpts = std::max(maxpts, (size_t)d.nr * d.nt);
-    S->pts.alloc(4 * maxpts);
-    S->wb.alloc(3 * maxpts);
+    S->wb.alloc(3 * act_area_.size());
+    S->dparts.alloc(kActParts * disks_.size());
+    S->dq.alloc(disks_.size());
     ct_grad_.assign(disks_.size(), 0.0);
     adj_ = std::move(S);
 }
@@ -172,60 +171,37 @@ void Sim::forward_core() {
 // Reverse of the actuator forcing.  srcb = adjoint of src; the actuator field
 // enters src as rho * act.
 void Sim::adjoint_disks(const double* srcb) {
-    if (!S_.act) return;
+    if (!S_.act || disks_.empty()) return;
     AdjState& S = *adj_;
-    const double pi = 3.14159265358979323846;
-    for (size_t di = 0; di < disks_.size(); ++di) {
+    const size_t nd = disks_.size(), np = act_area_.size();
+    long long cells = 0;
+    for (auto& G : act_groups_) cells = std::max(cells, G.cells);
+    // q = sum_x actb(x) . a  B(x) of every disk, B with the per-point weights pi (r+^2 - r-^2) / nt
+    ck(cudaMemcpyAsync(actw_.p, act_area_.data(), np * sizeof(double), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
+    launch_act_adj_dot(ctx_, g_, srcb, actd_.p, (int)nd, cells, ring_.p, actw_.p, acte_.p, actr_.p, plo_, S.dparts.p);
+    launch_reduce(ctx_, S.dparts.p, kActParts, (int)nd, 0, S.dq.p);
+    std::vector<double> q(nd), wb(3 * np);
+    ck(cudaMemcpyAsync(q.data(), S.dq.p, nd * sizeof(double), cudaMemcpyDeviceToHost, ctx_.stream), "D2H");
+    sync();
+    for (size_t di = 0; di < nd; ++di) {
         const Disk& d = disks_[di];
         const double* ax = d.normal;
-        std::vector<double> hp, rpos;
-        disk_points(d, hp, rpos);
-        // q = sum_x actb(x) . a  B(x), B with the per-point weights pi (r+^2 - r-^2) / nt
-        std::vector<double> ring;
-        double bmin[3] = {1e300, 1e300, 1e300}, bmax[3] = {-1e300, -1e300, -1e300};
-        for (int ip = 0; ip < d.nr; ++ip) {
-            const double r = (ip + 0.5) * d.dr, rp = r + 0.5 * d.dr, rmn = r - 0.5 * d.dr;
-            const double wgt = pi * (rp * rp - rmn * rmn) / d.nt;
-            for (int it = 0; it < d.nt; ++it) {
-                const double* o = &rpos[3 * (ip * d.nt + it)];
-                for (int m = 0; m < 3; ++m) {
-                    ring.push_back(o[m]);
-                    bmin[m] = std::min(bmin[m], o[m]);
-                    bmax[m] = std::max(bmax[m], o[m]);
-                }
-                ring.push_back(wgt);
-            }
-        }
-        const int nring = (int)ring.size() / 4;
-        int lo[3], hi[3];
-        const double h[3] = {g_.dx, g_.dy, g_.dz};
-        const int nn[3] = {g_.nx, g_.ny, g_.nz};
-        for (int m = 0; m < 3; ++m) {
-            lo[m] = std::max(0, (int)std::floor((bmin[m] - 4.0 * d.eps - plo_[m]) / h[m]) - 1);
-            hi[m] = std::min(nn[m] - 1, (int)std::floor((bmax[m] + 4.0 * d.eps - plo_[m]) / h[m]) + 1);
-        }
-        if (hi[0] < lo[0] || hi[1] < lo[1] || hi[2] < lo[2]) continue;
-        ck(cudaMemcpyAsync(S.pts.p, ring.data(), ring.size() * sizeof(double), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
-        int np = 0;
-        launch_act_adj_dot(ctx_, g_, srcb, S.pts.p, nring, ax, d.eps, plo_, lo, hi, parts_.p, &np);
-        const double q = rho_ * reduce(np, 1, 0, nullptr);
+        q[di] *= rho_;
         // act = 0.5 ct un^2 B a:  dJ/dct += 0.5 un^2 q ;  un_bar = ct un q
         const double un = d.ref[0] * ax[0] + d.ref[1] * ax[1] + d.ref[2] * ax[2];
-        ct_grad_[di] += 0.5 * un * un * q;
-        const double unb = d.ct_now * un * q;
+        ct_grad_[di] += 0.5 * un * un * q[di];
+        const double unb = d.ct_now * un * q[di];
         // un = a . sum_p w_p u(x_p): scatter w_p unb a to the sampling stencils
-        const int npts = d.nr * d.nt;
-        std::vector<double> wb(3 * (size_t)npts);
+        double* w3 = &wb[3 * (size_t)act_h_[di].p0];
         for (int ir = 0; ir < d.nr; ++ir) {
             const double w = ((ir + 1.0) * (ir + 1.0) - (double)ir * ir) / ((double)d.nr * d.nr * d.nt);
             for (int it = 0; it < d.nt; ++it)
-                for (int m = 0; m < 3; ++m) wb[3 * (ir * d.nt + it) + m] = w * unb * ax[m];
+                for (int m = 0; m < 3; ++m) w3[3 * (ir * d.nt + it) + m] = w * unb * ax[m];
         }
-        ck(cudaMemcpyAsync(S.pts.p, hp.data(), hp.size() * sizeof(double), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
-        ck(cudaMemcpyAsync(S.wb.p, wb.data(), wb.size() * sizeof(double), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
-        launch_act_sample_adj(ctx_, g_, S.pts.p, S.wb.p, npts, plo_, S.ub.p);
-        sync();  // host vectors and S.pts are reused by the next disk
     }
+    ck(cudaMemcpyAsync(S.wb.p, wb.data(), wb.size() * sizeof(double), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
+    launch_act_sample_adj(ctx_, g_, pts_.p, S.wb.p, (int)np, plo_, S.ub.p);
+    sync();  // wb is read by the copy
 }
 
 // Reverse of one step at the current state x^n = (velocity, gp).  On entry

@@ -844,10 +844,7 @@ void Sim::alloc() {
         if (!godunov_) tconv_old_.alloc(N);
         if (gb_.flux[0][0] == nullptr) throw KsError(KS_ERR_UNSUPPORTED, "temperature transport needs the face scratch");
     }
-    size_t maxpts = 1;
-    for (auto& d : disks_) maxpts = std::max(maxpts, (size_t)d.nr * d.nt);
-    pts_.alloc(4 * maxpts);
-    samp_.alloc(3 * maxpts);
+    act_setup();
     launch_fill(ctx_, mueff_.p, mu_, g_.N);
 }
 
@@ -1020,29 +1017,94 @@ void Sim::disk_points(const Disk& d, std::vector<double>& sample, std::vector<do
     }
 }
 
-void Sim::actuator_update() {
-    if (!S_.act) return;
+// What the disks keep for the life of the handle: they do not move, so their
+// sampling points, spreading boxes and Gaussian factors are laid out once.
+void Sim::act_setup() {
     const double pi = 3.14159265358979323846;
-    launch_fill(ctx_, act_.p, 0.0, 3 * g_.N);
+    const double h[3] = {g_.dx, g_.dy, g_.dz};
+    const int nn[3] = {g_.nx, g_.ny, g_.nz};
+    std::vector<double> sample, ring;
+    long long tab = 0;
     for (auto& d : disks_) {
-        // sample points on the sampling disk (disk_ops.cpp:378-412)
-        const double* ax = d.normal;
-        const int np = d.nr * d.nt;
         std::vector<double> hp, rpos;
         disk_points(d, hp, rpos);
-        for (int p = 0; p < np; ++p) {
-            const double hh[3] = {g_.dx, g_.dy, g_.dz};
-            const int nn[3] = {g_.nx, g_.ny, g_.nz};
-            for (int m = 0; m < 3; ++m) {
-                const int c = (int)std::floor((hp[3 * p + m] - plo_[m] - 0.5 * hh[m]) / hh[m]);
-                if (c < -1 || c + 1 > nn[m]) throw KsError(KS_ERR_DECK, "actuator sample point outside the domain");
+        ActDisk A{};
+        A.p0 = (int)(ring.size() / 3);
+        A.npts = d.nr * d.nt;
+        A.tab = tab;
+        A.eps = d.eps;
+        for (int m = 0; m < 3; ++m) A.ax[m] = d.normal[m];
+        double bmin[3] = {1e300, 1e300, 1e300}, bmax[3] = {-1e300, -1e300, -1e300};
+        for (int ip = 0; ip < d.nr; ++ip) {
+            const double r = (ip + 0.5) * d.dr, rp = r + 0.5 * d.dr, rmn = r - 0.5 * d.dr;
+            for (int it = 0; it < d.nt; ++it) {
+                for (int m = 0; m < 3; ++m) {
+                    const double o = rpos[3 * (ip * d.nt + it) + m], q = hp[3 * (ip * d.nt + it) + m];
+                    bmin[m] = std::min(bmin[m], o);
+                    bmax[m] = std::max(bmax[m], o);
+                    const int c = (int)std::floor((q - plo_[m] - 0.5 * h[m]) / h[m]);
+                    if (c < -1 || c + 1 > nn[m]) act_outside_ = true;
+                }
+                act_area_.push_back(pi * (rp * rp - rmn * rmn) / d.nt);
             }
         }
-        ck(cudaMemcpyAsync(pts_.p, hp.data(), hp.size() * sizeof(double), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
-        launch_act_sample(ctx_, g_, vel_.p, pts_.p, np, plo_, samp_.p);
-        std::vector<double> sv(3 * (size_t)np);
-        ck(cudaMemcpyAsync(sv.data(), samp_.p, sv.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx_.stream), "D2H");
-        sync();
+        // cells within 4 eps of any ring point, clamped to the domain
+        bool empty = false;
+        for (int m = 0; m < 3; ++m) {
+            const int hi = std::min(nn[m] - 1, (int)std::floor((bmax[m] + 4.0 * d.eps - plo_[m]) / h[m]) + 1);
+            A.lo[m] = std::max(0, (int)std::floor((bmin[m] - 4.0 * d.eps - plo_[m]) / h[m]) - 1);
+            A.n[m] = hi - A.lo[m] + 1;
+            empty = empty || A.n[m] <= 0;
+        }
+        if (empty) A.n[0] = A.n[1] = A.n[2] = 0;
+        tab += (long long)A.npts * (A.n[0] + A.n[1] + A.n[2]);
+        sample.insert(sample.end(), hp.begin(), hp.end());
+        ring.insert(ring.end(), rpos.begin(), rpos.end());
+        // a disk joins the launch of its predecessors unless their boxes meet
+        bool joins = !act_groups_.empty();
+        for (int q = joins ? act_groups_.back().d0 : 0; joins && q < (int)act_h_.size(); ++q) {
+            bool meet = true;
+            for (int m = 0; m < 3; ++m) meet = meet && A.lo[m] < act_h_[q].lo[m] + act_h_[q].n[m] && act_h_[q].lo[m] < A.lo[m] + A.n[m];
+            joins = !meet;
+        }
+        if (!joins) act_groups_.push_back({(int)act_h_.size(), 0, 0});
+        ActGroup& G = act_groups_.back();
+        G.nd += 1;
+        G.cells = std::max(G.cells, (long long)A.n[0] * A.n[1] * A.n[2]);
+        act_h_.push_back(A);
+    }
+    if (disks_.empty()) return;
+    pts_.alloc(sample.size());
+    samp_.alloc(sample.size());
+    ring_.alloc(ring.size());
+    actw_.alloc(act_area_.size());
+    actd_.alloc(act_h_.size());
+    acte_.alloc((size_t)tab);
+    actr_.alloc((size_t)tab);
+    ck(cudaDeviceSynchronize(), "disk tables");  // alloc's memset is not ordered with the handle's stream
+    ck(cudaMemcpyAsync(pts_.p, sample.data(), sample.size() * sizeof(double), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
+    ck(cudaMemcpyAsync(ring_.p, ring.data(), ring.size() * sizeof(double), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
+    ck(cudaMemcpyAsync(actd_.p, act_h_.data(), act_h_.size() * sizeof(ActDisk), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
+    launch_act_tables(ctx_, g_, actd_.p, (int)act_h_.size(), tab, ring_.p, plo_, acte_.p, actr_.p);
+    sync();  // the host vectors are read by the copies
+}
+
+void Sim::actuator_update() {
+    if (!S_.act) return;
+    launch_fill(ctx_, act_.p, 0.0, 3 * g_.N);
+    if (disks_.empty()) return;
+    if (act_outside_) throw KsError(KS_ERR_DECK, "actuator sample point outside the domain");
+    // velocity at the points of every sampling disk (disk_ops.cpp:378-412)
+    const double pi = 3.14159265358979323846;
+    const int np = (int)act_area_.size();
+    launch_act_sample(ctx_, g_, vel_.p, pts_.p, np, plo_, samp_.p);
+    act_host_.resize(3 * (size_t)np);
+    ck(cudaMemcpyAsync(act_host_.data(), samp_.p, act_host_.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx_.stream), "D2H");
+    sync();
+    for (size_t di = 0; di < disks_.size(); ++di) {
+        Disk& d = disks_[di];
+        const double* sv = &act_host_[3 * (size_t)act_h_[di].p0];
+        const double* ax = d.normal;
         double ref[3] = {0, 0, 0};
         for (int ir = 0; ir < d.nr; ++ir) {
             const double w = ((ir + 1.0) * (ir + 1.0) - (double)ir * ir) / ((double)d.nr * d.nr * d.nt);
@@ -1060,36 +1122,21 @@ void Sim::actuator_update() {
             while (m + 1 < d.ws.size() && d.ws[m + 1] < umag) ++m;
             d.ct_now = d.ct[m] + (d.ct[m + 1] - d.ct[m]) * (umag - d.ws[m]) / (d.ws[m + 1] - d.ws[m]);
         }
+    }
+    // force magnitude of every ring point
+    for (size_t di = 0; di < disks_.size(); ++di) {
+        const Disk& d = disks_[di];
         const double aero = 0.5 * d.uinf2 * d.ct_now;
-        // ring points with per-point force magnitude
-        std::vector<double> ring;
-        double bmin[3] = {1e300, 1e300, 1e300}, bmax[3] = {-1e300, -1e300, -1e300};
+        double* w = &act_host_[act_h_[di].p0];
         for (int ip = 0; ip < d.nr; ++ip) {
             const double r = (ip + 0.5) * d.dr, rp = r + 0.5 * d.dr, rmn = r - 0.5 * d.dr;
             const double f = aero * pi * (rp * rp - rmn * rmn);
-            for (int it = 0; it < d.nt; ++it) {
-                const double* o = &rpos[3 * (ip * d.nt + it)];
-                for (int m = 0; m < 3; ++m) {
-                    ring.push_back(o[m]);
-                    bmin[m] = std::min(bmin[m], o[m]);
-                    bmax[m] = std::max(bmax[m], o[m]);
-                }
-                ring.push_back(f / d.nt);
-            }
+            for (int it = 0; it < d.nt; ++it) w[ip * d.nt + it] = f / d.nt;
         }
-        const int nring = (int)ring.size() / 4;
-        ck(cudaMemcpyAsync(pts_.p, ring.data(), ring.size() * sizeof(double), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
-        // cells within 4 eps of any ring point, clamped to the domain
-        int lo[3], hi[3];
-        const double h[3] = {g_.dx, g_.dy, g_.dz};
-        const int nn[3] = {g_.nx, g_.ny, g_.nz};
-        for (int m = 0; m < 3; ++m) {
-            lo[m] = std::max(0, (int)std::floor((bmin[m] - 4.0 * d.eps - plo_[m]) / h[m]) - 1);
-            hi[m] = std::min(nn[m] - 1, (int)std::floor((bmax[m] + 4.0 * d.eps - plo_[m]) / h[m]) + 1);
-        }
-        launch_act_spread(ctx_, g_, act_.p, pts_.p, nring, ax, d.eps, plo_, lo, hi);
-        sync();  // pts_ is reused by the next disk
     }
+    ck(cudaMemcpyAsync(actw_.p, act_host_.data(), (size_t)np * sizeof(double), cudaMemcpyHostToDevice, ctx_.stream), "H2D");
+    for (auto& G : act_groups_)
+        if (G.cells > 0) launch_act_spread(ctx_, g_, act_.p, actd_.p, G.d0, G.nd, G.cells, ring_.p, actw_.p, acte_.p, actr_.p, plo_);
 }
 
 // ---------------------------------------------------------------- MAC projection

@@ -4,6 +4,7 @@
 // sampling and Gaussian spreading.  One thread per output point; periodic
 // wrap and wall boundary conditions are applied inside the kernels (no ghost
 // cells are stored).
+#include <algorithm>
 #include <cmath>
 
 #include "ks_launch.hpp"
@@ -858,31 +859,84 @@ __global__ void k_act_sample(Grid g, const double* vel, const double* pts, int n
 }
 
 // Gaussian spreading of ring-point forces (disk_spreading.H:45-105,
-// actuator_utils.H:45-60) over the cells of the cut-off box of one disk.
-__global__ void k_act_spread(Grid g, double* act, const double* pts, int npts, double ax0, double ax1, double ax2, double eps,
-                             double x0, double y0, double z0, int lo0, int lo1, int lo2, int n0, int n1, int n2) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long M = (long long)n0 * n1 * n2;
-    if (t >= M) return;
-    const int a = (int)(t % n0);
-    const long long r = t / n0;
-    const int b = (int)(r % n1), c = (int)(r / n1);
-    const int i = lo0 + a, j = lo1 + b, k = lo2 + c;
-    if (k < 0 || k >= g.nz) return;
-    // cell centre of the unwrapped index; stored at the wrapped cell
-    const double x = x0 + (i + 0.5) * g.dx, y = y0 + (j + 0.5) * g.dy, z = z0 + (k + 0.5) * g.dz;
-    const double gfac = 0.17958712212516656 / (eps * eps * eps);
-    double s = 0;
-    for (int m = 0; m < npts; ++m) {
-        const double rx = (pts[4 * m] - x) / eps, ry = (pts[4 * m + 1] - y) / eps, rz = (pts[4 * m + 2] - z) / eps;
-        const double r2 = rx * rx + ry * ry + rz * rz;
-        if (r2 < 16.0) s += gfac * exp(-rx * rx - ry * ry - rz * rz) * pts[4 * m + 3];
+// actuator_utils.H:45-60) over the cells of the cut-off box of a disk.
+// The kernel exp(-|x - p|^2 / eps^2) is a product of three 1D factors, and
+// disks do not move: k_act_tables forms the factors of every (point, cell
+// column of one direction) once per handle, and the spread multiplies them.
+// Evaluated per (point, cell) it took three FP64 divisions and an exp, about
+// 45 FP64 issue slots for each of the 100 points of a cell, and one launch and
+// two host waits a disk: 340 us a disk of 18 cells' diameter, 5.4 ms a step of
+// a 16-disk farm.
+__global__ void k_act_tables(Grid g, const ActDisk* D, const double* pts, double x0, double y0, double z0, double* E, float* R) {
+    const ActDisk d = D[blockIdx.y];
+    const int S = d.n[0] + d.n[1] + d.n[2];
+    const double gfac = 0.17958712212516656 / (d.eps * d.eps * d.eps);
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < d.npts * S; t += gridDim.x * blockDim.x) {
+        const int m = t / S;
+        int q = t - m * S, dir = 0;
+        while (q >= d.n[dir]) q -= d.n[dir++];
+        const double o = dir == 0 ? x0 : (dir == 1 ? y0 : z0), h = hd(g, dir);
+        const double r = (pts[3 * (d.p0 + m) + dir] - (o + (d.lo[dir] + q + 0.5) * h)) / d.eps;
+        E[d.tab + t] = (dir == 0 ? gfac : 1.0) * exp(-r * r);
+        R[d.tab + t] = (float)(r * r);
     }
+}
+
+// Sum over a disk's points of w_m g3(x - p_m) at cell (a, b, c) of its box.
+// The cut-off |x - p|^2 < 16 eps^2 is decided on the FP32 squares, whose sum is
+// off by less than 1e-5, and within 0.01 of it on the FP64 distance itself.
+__device__ inline double act_sum(const Grid& g, const ActDisk& d, const double* pts, const double* w, const double* E, const float* R, double x0,
+                                 double y0, double z0, int a, int b, int c) {
+    const int S = d.n[0] + d.n[1] + d.n[2];
+    const int ob = d.n[0] + b, oc = d.n[0] + d.n[1] + c;
+    double s = 0;
+    for (int m = 0; m < d.npts; ++m) {
+        const long long q = d.tab + (long long)m * S;
+        const float r2 = R[q + a] + R[q + ob] + R[q + oc];
+        if (r2 > 16.01f) continue;
+        if (r2 > 15.99f) {
+            const double* p = pts + 3 * (d.p0 + m);
+            const double rx = (p[0] - (x0 + (d.lo[0] + a + 0.5) * g.dx)) / d.eps, ry = (p[1] - (y0 + (d.lo[1] + b + 0.5) * g.dy)) / d.eps,
+                         rz = (p[2] - (z0 + (d.lo[2] + c + 0.5) * g.dz)) / d.eps;
+            if (!(rx * rx + ry * ry + rz * rz < 16.0)) continue;
+        }
+        s += E[q + a] * E[q + ob] * (E[q + oc] * w[d.p0 + m]);
+    }
+    return s;
+}
+
+// One launch spreads the disks d0 .. d0 + gridDim.y - 1, whose boxes are
+// disjoint; overlapping disks go in launches of their own, in disk order.
+__global__ void k_act_spread(Grid g, double* act, const ActDisk* D, int d0, const double* pts, const double* w, const double* E, const float* R,
+                             double x0, double y0, double z0) {
+    const ActDisk d = D[d0 + blockIdx.y];
+    const int M = d.n[0] * d.n[1] * d.n[2];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= M) return;
+    const int a = t % d.n[0], r = t / d.n[0], b = r % d.n[1], c = r / d.n[1];
+    const double s = act_sum(g, d, pts, w, E, R, x0, y0, z0, a, b, c);
     if (s == 0.0) return;
-    const long long cc = cidx(g, wrapn(i, g.nx), wrapn(j, g.ny), k);
-    act[cc] += s * ax0;
-    act[g.N + cc] += s * ax1;
-    act[2 * g.N + cc] += s * ax2;
+    const long long cc = cidx(g, d.lo[0] + a, d.lo[1] + b, d.lo[2] + c);
+    act[cc] += s * d.ax[0];
+    act[g.N + cc] += s * d.ax[1];
+    act[2 * g.N + cc] += s * d.ax[2];
+}
+
+// disk adjoint: per disk (blockIdx.y) block sums over its box of
+// sum_x (actb(x) . n) B(x), B(x) = sum_m w_m g3(x - p_m)
+__global__ void k_act_adj_dot(Grid g, const double* actb, const ActDisk* D, const double* pts, const double* w, const double* E, const float* R,
+                              double x0, double y0, double z0, double* parts) {
+    const ActDisk d = D[blockIdx.y];
+    const int M = d.n[0] * d.n[1] * d.n[2];
+    double acc = 0.0;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < M; t += gridDim.x * blockDim.x) {
+        const int a = t % d.n[0], r = t / d.n[0], b = r % d.n[1], c = r / d.n[1];
+        const double s = act_sum(g, d, pts, w, E, R, x0, y0, z0, a, b, c);
+        const long long cc = cidx(g, d.lo[0] + a, d.lo[1] + b, d.lo[2] + c);
+        acc += s * (actb[cc] * d.ax[0] + actb[g.N + cc] * d.ax[1] + actb[2 * g.N + cc] * d.ax[2]);
+    }
+    acc = block_reduce<0>(acc);
+    if (threadIdx.x == 0) parts[blockIdx.y * gridDim.x + blockIdx.x] = acc;
 }
 
 }  // namespace
@@ -1050,13 +1104,21 @@ void launch_sub_ratio(Ctx& c, double* a, long long n, const double* s, double de
 void launch_act_sample(Ctx& c, const Grid& g, const double* vel, const double* pts, int npts, const double plo[3], double* out) {
     KS_LAUNCH(c, k_act_sample, nblocks(npts, 64), 64, B8 * 6 * npts, g, vel, pts, npts, plo[0], plo[1], plo[2], out);
 }
-void launch_act_spread(Ctx& c, const Grid& g, double* act, const double* pts, int npts, const double ax[3], double eps, const double plo[3],
-                       const int lo[3], const int hi[3]) {
-    const int n0 = hi[0] - lo[0] + 1, n1 = hi[1] - lo[1] + 1, n2 = hi[2] - lo[2] + 1;
-    if (n0 <= 0 || n1 <= 0 || n2 <= 0) return;
-    const long long M = (long long)n0 * n1 * n2;
-    KS_LAUNCH(c, k_act_spread, nblocks(M, BS), BS, B8 * 6 * M, g, act, pts, npts, ax[0], ax[1], ax[2], eps, plo[0], plo[1], plo[2], lo[0],
-              lo[1], lo[2], n0, n1, n2);
+void launch_act_tables(Ctx& c, const Grid& g, const ActDisk* D, int nd, long long entries, const double* pts, const double plo[3], double* E,
+                       float* R) {
+    const long long b = (entries / std::max(1, nd) + BS - 1) / BS;
+    const dim3 grid((unsigned)std::max(1LL, std::min(1024LL, b)), (unsigned)nd);
+    KS_LAUNCH(c, k_act_tables, grid, BS, 12.0 * entries, g, D, pts, plo[0], plo[1], plo[2], E, R);
+}
+void launch_act_spread(Ctx& c, const Grid& g, double* act, const ActDisk* D, int d0, int nd, long long cells, const double* pts, const double* w,
+                       const double* E, const float* R, const double plo[3]) {
+    const dim3 grid(nblocks(cells, 128), (unsigned)nd);
+    KS_LAUNCH(c, k_act_spread, grid, 128, B8 * 6 * cells * nd, g, act, D, d0, pts, w, E, R, plo[0], plo[1], plo[2]);
+}
+void launch_act_adj_dot(Ctx& c, const Grid& g, const double* actb, const ActDisk* D, int nd, long long cells, const double* pts, const double* w,
+                        const double* E, const float* R, const double plo[3], double* parts) {
+    const dim3 grid(kActParts, (unsigned)nd);
+    KS_LAUNCH(c, k_act_adj_dot, grid, 128, B8 * 3 * cells * nd, g, actb, D, pts, w, E, R, plo[0], plo[1], plo[2], parts);
 }
 
 }  // namespace ks

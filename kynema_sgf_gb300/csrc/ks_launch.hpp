@@ -194,8 +194,24 @@ void launch_ke(Ctx& c, const Grid& g, const double* vel, double rho, double* par
 void launch_sub_ratio(Ctx& c, double* a, long long n, const double* s, double den, double* parts = nullptr, int* np = nullptr);
 void launch_reduce(Ctx& c, const double* partials, int nparts, int ncomp, int op_max, double* out);
 void launch_act_sample(Ctx& c, const Grid& g, const double* vel, const double* pts, int npts, const double plo[3], double* out);
-void launch_act_spread(Ctx& c, const Grid& g, double* act, const double* pts, int npts, const double ax[3], double eps,
-                       const double plo[3], const int lo[3], const int hi[3]);
+// Actuator disks (device records).  A disk's spreading box lo, n of cells; its
+// points p0 .. p0 + npts - 1 of the ring-point array; its 1D Gaussian factors
+// from entry tab of the tables, npts rows of n[0] + n[1] + n[2].
+struct ActDisk {
+    int lo[3], n[3];
+    int p0, npts;
+    long long tab;
+    double ax[3], eps;
+};
+constexpr int kActParts = 128;  // block sums per disk of launch_act_adj_dot
+void launch_act_tables(Ctx& c, const Grid& g, const ActDisk* D, int nd, long long entries, const double* pts, const double plo[3], double* E,
+                       float* R);
+// disks d0 .. d0 + nd - 1 (disjoint boxes of at most `cells` cells), point weights w
+void launch_act_spread(Ctx& c, const Grid& g, double* act, const ActDisk* D, int d0, int nd, long long cells, const double* pts, const double* w,
+                       const double* E, const float* R, const double plo[3]);
+// kActParts block sums for each of the nd disks, disk-major
+void launch_act_adj_dot(Ctx& c, const Grid& g, const double* actb, const ActDisk* D, int nd, long long cells, const double* pts, const double* w,
+                        const double* E, const float* R, const double plo[3], double* parts);
 
 // ---- Godunov (ks_godunov.cu)
 // Godunov face scratch; each array holds FP64 or FP32 values (fp32 flag of
@@ -336,8 +352,6 @@ void launch_adj_coriolis(Ctx& c, const Grid& g, const double* srcb, const Scalar
 void launch_adj_nodal_post(Ctx& c, const Grid& g, const double* psi, const double* ub, double* out);
 void launch_axpby(Ctx& c, long long n, double a, const double* x, double b, const double* y, double* out);
 void launch_objective(Ctx& c, const Grid& g, const double* u, const int lo[3], const int hi[3], double invM, double* ub, double* parts, int* np);
-void launch_act_adj_dot(Ctx& c, const Grid& g, const double* actb, const double* pts, int npts, const double ax[3], double eps, const double plo[3],
-                        const int lo[3], const int hi[3], double* parts, int* np);
 void launch_act_sample_adj(Ctx& c, const Grid& g, const double* pts, const double* wb, int npts, const double plo[3], double* ub);
 
 // ---- multigrid (ks_mg.cu); T = double (FP64 path) or float (cycles of the

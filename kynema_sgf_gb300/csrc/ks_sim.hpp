@@ -214,7 +214,8 @@ struct AdjState {
     DevBuf<double> fu, fgp, fp;     // forward state at the end of an adjoint run
     DevBuf<double> snaps;           // binomial checkpoints, 6N values per slot
     int nslots = 0;
-    DevBuf<double> pts, wb;         // disk points / sample adjoints
+    DevBuf<double> wb;              // sample adjoints
+    DevBuf<double> dparts, dq;      // per-disk block sums and sums
     int box_lo[3] = {0, 0, 0}, box_hi[3] = {-1, -1, -1};
     bool box_set = false;
     double J = 0.0;
@@ -430,7 +431,21 @@ class Sim {
     DevBuf<double> mac_phi_prev_;
     double nod_bnorm_ = 0.0;   // |rhs| of a warm-started nodal solve (0: zero start)
     DevBuf<double> parts_, red_;
-    DevBuf<double> pts_, samp_;
+    // actuator disks (act_setup): sampling points and the velocity there, ring
+    // points, their force (or area) weights, disk records, 1D Gaussian factors
+    // and their squared distances
+    DevBuf<double> pts_, samp_, ring_, actw_, acte_;
+    DevBuf<float> actr_;
+    DevBuf<ActDisk> actd_;
+    std::vector<ActDisk> act_h_;
+    struct ActGroup {  // consecutive disks with disjoint boxes of at most `cells` cells
+        int d0, nd;
+        long long cells;
+    };
+    std::vector<ActGroup> act_groups_;
+    std::vector<double> act_area_, act_host_;
+    bool act_outside_ = false;  // a sampling point lies outside the domain
+    void act_setup();
     double* hred_ = nullptr;  // pinned
 };
 
