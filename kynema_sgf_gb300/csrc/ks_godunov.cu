@@ -18,6 +18,8 @@
 // taken on the integer pipe (ks_common.cuh).  Post-MAC states of rho*u are rho
 // times the traces of u (the PPM limiter and the traces are homogeneous of
 // degree one in the advected field).
+#include <algorithm>
+
 #include "ks_decide.cuh"
 #include "ks_launch.hpp"
 
@@ -513,13 +515,30 @@ __global__ void __launch_bounds__(128) k_cf_col(Op op, int chunk) {
     }
 }
 
+// Faces a thread of the column kernels marches.  A long march carries more
+// (the cell before a chunk is formed again: about 1.7 faces' work in k_ppm_col,
+// 0.7 in k_cf_col), a short one leaves more warps: an SM sub-partition needs
+// about 3.4 of them in FP64, whose step is a serial chain of 40 to 130 FP64
+// instructions, and twice as many in FP32, which waits on loads.  So the
+// marches are cut to leave 2048 (FP64) or 4096 (FP32) warps, between lo and hi
+// faces.  Measured, k_ppm_col / k_adv_trans_col: 32^3 129 / 69 us at 32 / 16
+// faces, 21 / 12.5 at 2 / 1; 64^3 141 / 84 against 60 / 41 at 4; 96^3 177 / 113
+// against 155 / 113 at 16; FP32 128x128x64 58 / 71 against 37 / 43 at 8; on
+// 256x256x128 32 / 16 are the best.
+template <typename T>
+inline int march_chunk(const Grid& g, int lo, int hi) {
+    const long long rows = 1 + (long long)g.ny * (g.nz + 1) / 32768;  // marches are counted on the second grid dimension
+    const long long m = g.N / (32LL * (sizeof(T) == 4 ? 4096 : 2048));
+    return (int)std::min<long long>(hi, std::max<long long>(std::max<long long>(lo, rows), m));
+}
+
 template <typename Op>
 static void launch_cf(Ctx& c, const char* name_x, const char* name_col, const Op& op, double bytes) {
     const Grid& g = op.g;
     if (op.d == 0) {
         KS_LAUNCH_NAMED(c, name_x, k_cf_x<Op>, nblocks(g.N, 256), 256, bytes, op);
     } else {
-        constexpr int chunk = 16;
+        const int chunk = march_chunk<typename Op::T>(g, 1, 16);
         const int nf = op.d == 1 ? g.ny : nzfaces(g), no = op.d == 1 ? g.nz : g.ny;
         const int bx = g.nx >= 128 ? 128 : 32 * ((g.nx + 31) / 32);
         const dim3 grid((unsigned)((g.nx + bx - 1) / bx), (unsigned)(no * ((nf + chunk - 1) / chunk)));
@@ -694,7 +713,6 @@ static T* tp(void* p) {
 }
 
 // stage 1 on the d-faces: the x kernel for d = 0, the column march otherwise
-constexpr int PPM_CHUNK = 32;
 template <typename T, int NC, int MODE, int EDGES>
 static void launch_ppm(Ctx& c, const Grid& g, int d, const T* vel, const T* umac, double dt, double rho, const PpmOut<T, NC>& O,
                        double bytes) {
@@ -706,7 +724,8 @@ static void launch_ppm(Ctx& c, const Grid& g, int d, const T* vel, const T* umac
         KS_LAUNCH(c, (k_ppm_x<T, NC, MODE, EDGES>), nblocks(warps * 32, BS), BS, bytes, A, s, T(rho), O);
     } else {
         const int nf = (d == 2) ? nzfaces(g) : g.ny;
-        const int nch = (nf + PPM_CHUNK - 1) / PPM_CHUNK, chunk = (nf + nch - 1) / nch;
+        const int most = march_chunk<T>(g, 2, 32);
+        const int nch = (nf + most - 1) / most, chunk = (nf + nch - 1) / nch;
         const int bx = g.nx >= BS ? BS : 32 * ((g.nx + 31) / 32);
         const dim3 grid((unsigned)((g.nx + bx - 1) / bx), (unsigned)((d == 1 ? g.nz : g.ny) * nch));
         KS_LAUNCH(c, (k_ppm_col<T, NC, MODE, EDGES>), grid, bx, bytes, A, s, T(rho), O, chunk);
