@@ -452,35 +452,57 @@ __global__ void __launch_bounds__(256) k_ppm_x(PpmArgs<T> A, T s, T rho, PpmOut<
 // velocities and states on its own transverse faces).  The low-side state of
 // face c + e_d and the high-side state of face c share it, so the kernels
 // below form each cell's corrections once: x faces take the low cell's from
-// the previous lane of the warp (lane 0 and the periodic wrap form their
-// own); y and z faces march a chunk of 16 faces along d and carry it.
+// the thread before; y and z faces march a chunk of 16 faces along d and carry it.
 //
 // An op supplies T, K (values per cell), the grid g and face direction d,
 //   cell(i, j, k, c[K]): the cell's corrections,
 //   face(f, kf, wl, wh, cl[K], ch[K]): the face's output from the low and
 //     high cells' corrections (kf the face's z index, wl / wh a wall face
 //     without a cell below / above).
+//
+// A block of k_cf_x holds `rows` whole x rows, or `seg` cells of a row longer
+// than a block, and passes the low cell's corrections through shared memory, so
+// only the first cell of a segment forms its low neighbour's.  (Passed between
+// the lanes of a warp, lane 0 of every warp formed a second cell's, which costs
+// the warp a second pass of its FP64 instructions: k_adv_trans_x 1563 us and
+// k_adv_flux_x 1380 us on 256x256x128 in FP64, 1.55 times the column kernels;
+// now 1000 and 858.)
 template <typename Op>
-__global__ void __launch_bounds__(256, sizeof(typename Op::T) == 4 ? 3 : 2) k_cf_x(Op op) {
+__global__ void __launch_bounds__(256, sizeof(typename Op::T) == 4 ? 3 : 2) k_cf_x(Op op, int rows, int seg, int nseg) {
     using T = typename Op::T;
     constexpr int K = Op::K;
+    __shared__ T sh[K][256];
     const Grid& g = op.g;
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const bool live = t < g.N;
-    int i = 0, j = 0, k = 0;
-    T ch[K], cl[K];
-    for (int n = 0; n < K; ++n) ch[n] = T(0);
-    if (live) {
-        const unsigned u = (unsigned)t, r = u / (unsigned)g.nx;
-        i = (int)(u - r * (unsigned)g.nx);
-        k = (int)(r / (unsigned)g.ny);
-        j = (int)(r - (unsigned)k * (unsigned)g.ny);
-        op.cell(i, j, k, ch);
+    const int t = threadIdx.x;
+    int row, i;
+    bool live;
+    if (nseg == 1) {
+        const int r = t / g.nx;
+        i = t - r * g.nx;
+        row = blockIdx.x * rows + r;
+        live = r < rows && row < g.ny * g.nz;
+    } else {
+        row = blockIdx.x / nseg;
+        i = (blockIdx.x - row * nseg) * seg + t;
+        live = t < seg && i < g.nx;
     }
-    for (int n = 0; n < K; ++n) cl[n] = __shfl_up_sync(0xffffffffu, ch[n], 1);
+    const int k = row / g.ny, j = row - k * g.ny;
+    T ch[K], cl[K];
+    if (live) {
+        op.cell(i, j, k, ch);
+#pragma unroll
+        for (int n = 0; n < K; ++n) sh[n][t] = ch[n];
+    }
+    __syncthreads();
     if (!live) return;
-    if ((threadIdx.x & 31) == 0 || i == 0) op.cell(i == 0 ? g.nx - 1 : i - 1, j, k, cl);
-    op.face(t, k, false, false, cl, ch);
+    if (nseg > 1 && t == 0) {
+        op.cell(i == 0 ? g.nx - 1 : i - 1, j, k, cl);
+    } else {
+        const int q = i == 0 ? t + g.nx - 1 : t - 1;
+#pragma unroll
+        for (int n = 0; n < K; ++n) cl[n] = sh[n][q];
+    }
+    op.face((long long)row * g.nx + i, k, false, false, cl, ch);
 }
 
 template <typename Op>
@@ -536,7 +558,10 @@ template <typename Op>
 static void launch_cf(Ctx& c, const char* name_x, const char* name_col, const Op& op, double bytes) {
     const Grid& g = op.g;
     if (op.d == 0) {
-        KS_LAUNCH_NAMED(c, name_x, k_cf_x<Op>, nblocks(g.N, 256), 256, bytes, op);
+        const int nseg = (g.nx + 255) / 256, seg = (g.nx + nseg - 1) / nseg, rows = nseg == 1 ? 256 / g.nx : 1;
+        const long long lines = (long long)g.ny * g.nz;
+        const unsigned blocks = (unsigned)(nseg == 1 ? (lines + rows - 1) / rows : lines * nseg);
+        KS_LAUNCH_NAMED(c, name_x, k_cf_x<Op>, blocks, 32 * ((seg * rows + 31) / 32), bytes, op, rows, seg, nseg);
     } else {
         const int chunk = march_chunk<typename Op::T>(g, 1, 16);
         const int nf = op.d == 1 ? g.ny : nzfaces(g), no = op.d == 1 ? g.nz : g.ny;
