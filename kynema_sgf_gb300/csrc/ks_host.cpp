@@ -1509,7 +1509,7 @@ void Sim::diff_alloc() {
     }
     dbuf_.alloc(tot);
     dtmp_.alloc(3 * (size_t)g_.N);
-    dparts_.alloc((size_t)std::max(divtau_tile_blocks(g_), 2 * diff_cell_blocks(g_)));
+    dparts_.alloc((size_t)std::max(divtau_blocks(g_), 2 * diff_cell_blocks(g_)));
     double* q = dbuf_.p;
     for (size_t l = 0; l < cc_.size(); ++l) {
         DiffLevel L{};
@@ -1587,7 +1587,7 @@ void Sim::diffuse_solve(double dtd) {
         launch_divtau_jacobi(ctx_, g_, vel_.p, mueff_.p, wg_.p, vel_tmp_.p, L0.dinv, dtmp_.p, rho_, dtd, L0.omega, parts);
         std::swap(vel_.p, dtmp_.p);
     };
-    const int np = divtau_tile_blocks(g_);
+    const int np = divtau_blocks(g_);
     int it = 0;
     double r0 = 0.0, rn = 0.0, target = 0.0;
     while (true) {
@@ -1654,7 +1654,7 @@ void Sim::apply_predictor(bool incremental) {
     if (wallmodel_) launch_wall_grad(ctx_, g_, vel_old_.p, mueff_.p, wg_.p, shear_, utau_ * utau_, um_[0], um_[1], vmag_, rho_);
     double* fl[9];
     for (int m = 0; m < 9; ++m) fl[m] = static_cast<double*>(gb_.flux[m / 3][m % 3]);
-    launch_divtau(ctx_, g_, vel_old_.p, mueff_.p, wg_.p, divtau_.p, 1, src_.p, forces_.p, nullptr, nullptr, dt, rho_, fl, mixed_);
+    launch_divtau(ctx_, g_, vel_old_.p, mueff_.p, wg_.p, divtau_.p, 1, src_.p, forces_.p, nullptr, nullptr, dt, rho_, mixed_);
     if (temp_) {  // the temperature's diff_term(Old) (no temperature sources)
         if (tzlo_ == 1)
             launch_theta_wall_grad(ctx_, g_, vel_old_.p, theta_old_.p, alpha_.p, tgz_.p, shear_, utau_, kappa_, std::log(zref_ / z0t_), vmag_,
@@ -1673,7 +1673,7 @@ void Sim::apply_predictor(bool incremental) {
     if (S_.bous) sources(vel_old_.p, theta_nph_.p);
     launch_predictor_rhs(ctx_, g_, vel_old_.p, conv_.p, src_.p, divtau_.p, vel_.p, dt, rho_, diff_fac());
     if (diff_type_ == 0) {  // explicit RK2 correction (incflo_advance.cpp:388-400)
-        launch_divtau(ctx_, g_, vel_.p, mueff_.p, wg_.p, vel_tmp_.p, 2, nullptr, nullptr, vel_.p, divtau_.p, dt, rho_, fl, mixed_);
+        launch_divtau(ctx_, g_, vel_.p, mueff_.p, wg_.p, vel_tmp_.p, 2, nullptr, nullptr, vel_.p, divtau_.p, dt, rho_, mixed_);
         std::swap(vel_.p, vel_tmp_.p);
     } else {  // icns().solve(dt_diff) (incflo_advance.cpp:376-386)
         diffuse_solve(diff_type_ == 2 ? dt : 0.5 * dt);
@@ -1695,7 +1695,7 @@ void Sim::mol_predictor(bool incremental) {
     for (int m = 0; m < 9; ++m) fl[m] = static_cast<double*>(gb_.flux[m / 3][m % 3]);
     // diff_term(Old) enters predictor_rhs with factor 1 / 0.5 / 0 (implicit: not formed)
     const double fac = diff_fac();
-    if (fac != 0.0) launch_divtau(ctx_, g_, vel_old_.p, mueff_.p, wg_.p, divtau_.p, 0, nullptr, nullptr, nullptr, nullptr, dt, rho_, fl);
+    if (fac != 0.0) launch_divtau(ctx_, g_, vel_old_.p, mueff_.p, wg_.p, divtau_.p, 0, nullptr, nullptr, nullptr, nullptr, dt, rho_);
     if (temp_) {
         if (tzlo_ == 1)
             launch_theta_wall_grad(ctx_, g_, vel_old_.p, theta_old_.p, alpha_.p, tgz_.p, shear_, utau_, kappa_, std::log(zref_ / z0t_), vmag_,

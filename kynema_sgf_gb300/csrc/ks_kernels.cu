@@ -403,11 +403,9 @@ constexpr int TTX = 32, TTY = 4, TTZ = 4;
 constexpr int THX = TTX + 2, THY = TTY + 2, THZ = TTZ + 2;
 constexpr int TNH = THX * THY * THZ;
 constexpr int TNFX = (TTX + 1) * TTY * TTZ, TNFY = TTX * (TTY + 1) * TTZ, TNFZ = TTX * TTY * (TTZ + 1);
-// dynamic shared memory of the tile kernel staging and computing in type T
-template <typename T>
-constexpr size_t tau_smem() { return sizeof(T) * (4 * (size_t)TNH + 3 * ((size_t)TNFX + TNFY + TNFZ)); }
+constexpr size_t tau_smem() { return sizeof(float) * (4 * (size_t)TNH + 3 * ((size_t)TNFX + TNFY + TNFZ)); }
 
-// Epilogue of the tiled tensor-diffusion kernel (acc = divtau(vel) of a cell):
+// Epilogue of the tensor-diffusion kernels (acc = divtau(vel) of a cell):
 //   0: out = acc
 //   1: out = acc, forces = (src + acc) / rho
 //   2: out = base + 0.5 dt (acc - dold) / rho                        (explicit RK2 correction)
@@ -424,12 +422,12 @@ struct TauEpi {
     double irho;  // 1 / rho, formed on the host
 };
 
-// T: type of the staged values, the face fluxes and their arithmetic (double;
-// float for the mixed-precision form, modes 0-2 only).  The inputs are FP64
-// and rounded once when staged; the epilogue runs in FP64.
-template <typename T>
+// FP32 form (mixed precision, modes 0-2): staged values, face fluxes and their
+// arithmetic are FP32, the FP64 inputs rounded once when staged; the epilogue
+// runs in FP64.
 __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const double* vel, const double* mueff, const double* wg, double* out,
                                                                TauEpi E) {
+    using T = float;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     T* sm = reinterpret_cast<T*>(sm_raw);
     T* sV = sm;                // [3][THZ][THY][THX]
@@ -504,9 +502,8 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
     const int tx = tid % TTX, ty = (tid / TTX) % TTY, tz = tid / (TTX * TTY);
     const int i = i0 + tx, j = j0 + ty, k = k0 + tz;
     const bool live = i < g.nx && j < g.ny && k < g.nz;
-    const double rho = E.rho, dt = E.dt, irho = E.irho;
+    const double dt = E.dt, irho = E.irho;
     const long long N = g.N, t = live ? cidx(g, i, j, k) : 0;
-    double rmax = 0.0;
     for (int n = 0; n < 3 && live; ++n) {
         const int ax = (tz * TTY + ty) * (TTX + 1) + tx;
         const int ay = (tz * (TTY + 1) + ty) * TTX + tx;
@@ -521,27 +518,280 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
         } else if (E.mode == 1) {
             out[m] = acc;
             E.forces[m] = (E.src[m] + acc) * irho;
-        } else if (E.mode == 2) {
-            out[m] = E.base[m] + 0.5 * dt * (acc - E.dold[m]) * irho;
-        } else if (E.mode == 3) {
-            out[m] = (rho * E.base[m] + dt * (0.5 * (E.conv_o[m] + E.conv_n[m]) + 0.5 * E.dold[m] + 0.5 * acc + E.src[m])) * irho;
         } else {
-            const double x = (double)sV[n * TNH + hidx(tx + 1, ty + 1, tz + 1)];
-            const double r = E.base[m] - rho * x + dt * acc;
-            rmax = nmax(rmax, fabs(r));
-            out[m] = E.mode == 7 ? x + E.omega * E.dinv[m] * r : r;
+            out[m] = E.base[m] + 0.5 * dt * (acc - E.dold[m]) * irho;
         }
     }
+}
+
+// ---- FP64 form: columns marched in z.  The kernel is bound by FP64 issue, so
+// it spends as few FP64 instructions a cell as the term allows:
+// - a face's transverse derivatives are means of its two cells' central
+//   differences, so each cell's differences are formed once (nine subtractions,
+//   three of them merged in pairs into the part of the divergence that a
+//   direction's face needs) and both faces of the cell in a direction add them;
+// - grid spacings are ratios folded into one FMA per component, and the face
+//   viscosity carries 1 / h^2 of the flux's own direction, so a flux enters the
+//   divergence by a subtraction alone;
+// - a march keeps the z faces and the in-plane differences of the next layer.
+// 72 FP64 instructions a cell and 6 for the halo, where the tile kernel's
+// per-face differences, repeated on the tile's halo, took about 130.
+// A block owns 32 x TY columns and keeps three layers of the velocity (with a
+// one-cell halo) and two of the viscosity in shared memory; the layer after
+// next is loaded while the current one is computed.  Its warps: one per row of
+// columns; one each for the row below and above (the cell differences the y
+// faces need, and the upper row's faces); one for the columns left (lanes 0 ..)
+// and right (lanes 16 ..) of the block.
+// On 256x256x128: 2.25 ms as tiles (96 % of the FP64 issue rate), 1.56 ms now
+// (89 %); 96^3 284 -> 178 us.
+template <int TY>
+struct TauPlanes {
+    double V[3][3][TY + 2][34];   // [layer mod 3][component]: row and column 0 are the halo
+    double M[2][TY + 2][34];      // [layer mod 2]
+    double QX[3][TY][34];         // cell differences for x faces: divergence part, du/dy, du/dz
+    double QY[3][TY + 2][32];     // for y faces: divergence part, dv/dx, dv/dz
+    double FX[3][TY][33], FY[3][TY + 1][32];
+};
+struct TauCoef {                  // spacing ratios (see k_divtau_col)
+    double gx, gy, gz;            // 1 / (2 h^2)
+    double xy, xz, yx, yz, zx, zy;  // transverse weights: hx / (4 hy) on x faces, ...
+    double lx, ly, lz;            // -hx / (8 hy), -hy / (8 hx), -hz / (8 hx)
+    double ryz, rxz, rxy;         // hy / hz, hx / hz, hx / hy
+};
+inline TauCoef tau_coef(const Grid& g) {
+    const double x = g.dx, y = g.dy, z = g.dz;
+    return TauCoef{0.5 * g.idx * g.idx, 0.5 * g.idy * g.idy, 0.5 * g.idz * g.idz, 0.25 * x / y, 0.25 * x / z, 0.25 * y / x, 0.25 * y / z,
+                   0.25 * z / x,        0.25 * z / y,        -0.125 * x / y,      -0.125 * y / x, -0.125 * z / x, y / z, x / z, x / y};
+}
+
+template <int TY>
+__global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef K, const double* vel, const double* mueff, const double* wg, double* out,
+                                                             TauEpi E, int kc) {
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    TauPlanes<TY>& S = *reinterpret_cast<TauPlanes<TY>*>(sm_raw);
+    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * TY, k0 = blockIdx.z * kc, k1 = min(k0 + kc, g.nz);
+    const long long N = g.N;
+    const int sz = g.nx * g.ny;
+    // ---- staging: thread tid loads one column of the (TY + 2) x 34 footprint
+    // (a block may be wider than the grid: x and y wrap fully)
+    const bool loads = tid < (TY + 2) * 34;
+    const int lx = tid % 34, ly = tid / 34;
+    const int col = loads ? (((j0 + ly - 1) % g.ny + g.ny) % g.ny) * g.nx + ((i0 + lx - 1) % g.nx + g.nx) % g.nx : 0;
+    struct Cell {
+        double v[3], m;
+    };
+    auto fetch = [&](int k) {  // layer -1 and nz are the ghosts VelDiff gives
+        Cell c;
+        const int kk = g.zper ? (k < 0 ? k + g.nz : (k >= g.nz ? k - g.nz : k)) : (k < 0 ? 0 : (k >= g.nz ? g.nz - 1 : k));
+        const double* p = vel + (long long)kk * sz + col;
+        for (int n = 0; n < 3; ++n) c.v[n] = p[n * N];
+        c.m = mueff[(long long)kk * sz + col];
+        if (!g.zper && (k < 0 || k >= g.nz)) {
+            c.v[2] = bitsd(dbits(c.v[2]) ^ ~kMag);
+            if (k < 0 && g.zlo == ZWALLMODEL)
+                for (int n = 0; n < 2; ++n) c.v[n] -= wg[(long long)n * sz + col] * g.dz;
+        }
+        return c;
+    };
+    auto stage = [&](const Cell& c, int s, int k) {
+        for (int n = 0; n < 3; ++n) S.V[s][n][ly][lx] = c.v[n];
+        S.M[k & 1][ly][lx] = c.m;
+    };
+    int sm = 0, sc = 1, sp = 2;  // slots of layers k - 1, k, k + 1
+    double mu = 0.0;             // viscosity of layer k - 1, then k, of the thread's column
+    if (loads) {
+        const Cell c = fetch(k0 - 1);
+        stage(c, sm, k0 - 1);
+    }
+    __syncthreads();
+    const bool mainw = w < TY;
+    const int y = w + 1, x = l + 1;
+    if (mainw) mu = S.M[(k0 - 1) & 1][y][x];
+    __syncthreads();
+    if (loads) {
+        const Cell a = fetch(k0), b = fetch(k0 + 1);
+        stage(a, sc, k0);
+        stage(b, sp, k0 + 1);
+    }
+    __syncthreads();
+    // in-plane differences of a layer: du/dx, dv/dy, their part of the
+    // divergence in units of du/dx, dw/dx, dw/dy
+    struct Plane {
+        double dx, dy, c, wx, wy, v[3];
+    };
+    auto plane = [&](int s) {
+        Plane q;
+        for (int n = 0; n < 3; ++n) q.v[n] = S.V[s][n][y][x];
+        q.dx = S.V[s][0][y][x + 1] - S.V[s][0][y][x - 1];
+        q.dy = S.V[s][1][y + 1][x] - S.V[s][1][y - 1][x];
+        q.c = q.dx + K.rxy * q.dy;
+        q.wx = S.V[s][2][y][x + 1] - S.V[s][2][y][x - 1];
+        q.wy = S.V[s][2][y + 1][x] - S.V[s][2][y - 1][x];
+        return q;
+    };
+    auto zflux = [&](const Plane& a, const Plane& b, double msum, double F[3]) {
+        const double G = msum * K.gz, G43 = msum * (K.gz * (4.0 / 3.0));
+        F[0] = G * ((b.v[0] - a.v[0]) + K.zx * (a.wx + b.wx));
+        F[1] = G * ((b.v[1] - a.v[1]) + K.zy * (a.wy + b.wy));
+        F[2] = G43 * ((b.v[2] - a.v[2]) + K.lz * (a.c + b.c));
+    };
+    // differences across z and in the plane that the x faces (and y faces) of cell (yy, xx) need
+    auto xcell = [&](int yy, int xx, double dy, double q[3]) {
+        q[0] = dy + K.ryz * (S.V[sp][2][yy][xx] - S.V[sm][2][yy][xx]);
+        q[1] = S.V[sc][0][yy + 1][xx] - S.V[sc][0][yy - 1][xx];
+        q[2] = S.V[sp][0][yy][xx] - S.V[sm][0][yy][xx];
+    };
+    auto ycell = [&](int yy, int xx, double dx, double q[3]) {
+        q[0] = dx + K.rxz * (S.V[sp][2][yy][xx] - S.V[sm][2][yy][xx]);
+        q[1] = S.V[sc][1][yy][xx + 1] - S.V[sc][1][yy][xx - 1];
+        q[2] = S.V[sp][1][yy][xx] - S.V[sm][1][yy][xx];
+    };
+    auto xflux = [&](int yy, int xx, int m, double F[3]) {  // low x face of footprint cell (yy, xx)
+        const double ms = S.M[m][yy][xx] + S.M[m][yy][xx - 1], G = ms * K.gx, G43 = ms * (K.gx * (4.0 / 3.0));
+        F[0] = G43 * ((S.V[sc][0][yy][xx] - S.V[sc][0][yy][xx - 1]) + K.lx * (S.QX[0][yy - 1][xx] + S.QX[0][yy - 1][xx - 1]));
+        F[1] = G * ((S.V[sc][1][yy][xx] - S.V[sc][1][yy][xx - 1]) + K.xy * (S.QX[1][yy - 1][xx] + S.QX[1][yy - 1][xx - 1]));
+        F[2] = G * ((S.V[sc][2][yy][xx] - S.V[sc][2][yy][xx - 1]) + K.xz * (S.QX[2][yy - 1][xx] + S.QX[2][yy - 1][xx - 1]));
+    };
+    auto yflux = [&](int yy, int xx, int m, double F[3]) {  // low y face
+        const double ms = S.M[m][yy][xx] + S.M[m][yy - 1][xx], G = ms * K.gy, G43 = ms * (K.gy * (4.0 / 3.0));
+        F[0] = G * ((S.V[sc][0][yy][xx] - S.V[sc][0][yy - 1][xx]) + K.yx * (S.QY[1][yy][xx - 1] + S.QY[1][yy - 1][xx - 1]));
+        F[1] = G43 * ((S.V[sc][1][yy][xx] - S.V[sc][1][yy - 1][xx]) + K.ly * (S.QY[0][yy][xx - 1] + S.QY[0][yy - 1][xx - 1]));
+        F[2] = G * ((S.V[sc][2][yy][xx] - S.V[sc][2][yy - 1][xx]) + K.yz * (S.QY[2][yy][xx - 1] + S.QY[2][yy - 1][xx - 1]));
+    };
+    Plane pc{};
+    double fz[3] = {0.0, 0.0, 0.0};
+    if (mainw) {
+        const Plane pm = plane(sm);
+        pc = plane(sc);
+        const double m0 = S.M[k0 & 1][y][x];
+        zflux(pm, pc, mu + m0, fz);
+        mu = m0;
+    }
+    const int i = i0 + l, j = j0 + w;
+    const bool live = mainw && i < g.nx && j < g.ny;
+    const int sr = l & 15, sx = l < 16 ? 0 : 33;  // the side warp's row and column
+    const bool side = w == TY + 2 && sr < TY;
+    const double rho = E.rho, dt = E.dt, irho = E.irho;
+    long long rmax = 0;
+    for (int k = k0; k < k1; ++k) {
+        const int m = k & 1;
+        Cell nxt{};
+        const bool more = loads && k + 1 < k1;
+        if (more) nxt = fetch(k + 2);
+        // ---- cell differences of layer k, z fluxes on its upper faces
+        Plane pn{};
+        double fzn[3] = {0.0, 0.0, 0.0}, q[3];
+        if (mainw) {
+            pn = plane(sp);
+            const double mn = S.M[m ^ 1][y][x];
+            zflux(pc, pn, mu + mn, fzn);
+            mu = mn;
+            xcell(y, x, pc.dy, q);
+            for (int n = 0; n < 3; ++n) S.QX[n][w][x] = q[n];
+            ycell(y, x, pc.dx, q);
+            for (int n = 0; n < 3; ++n) S.QY[n][y][l] = q[n];
+        } else if (w < TY + 2) {
+            const int yy = w == TY ? 0 : TY + 1;
+            ycell(yy, x, S.V[sc][0][yy][x + 1] - S.V[sc][0][yy][x - 1], q);
+            for (int n = 0; n < 3; ++n) S.QY[n][yy][l] = q[n];
+        } else if (side) {
+            xcell(sr + 1, sx, S.V[sc][1][sr + 2][sx] - S.V[sc][1][sr][sx], q);
+            for (int n = 0; n < 3; ++n) S.QX[n][sr][sx] = q[n];
+        }
+        __syncthreads();
+        // ---- fluxes on the low x and y faces
+        double fx[3], fy[3];
+        if (mainw) {
+            xflux(y, x, m, fx);
+            yflux(y, x, m, fy);
+            for (int n = 0; n < 3; ++n) {
+                S.FX[n][w][l] = fx[n];
+                S.FY[n][w][l] = fy[n];
+            }
+        } else if (w == TY + 1) {
+            yflux(TY + 1, x, m, fy);
+            for (int n = 0; n < 3; ++n) S.FY[n][TY][l] = fy[n];
+        } else if (side && sx) {
+            xflux(sr + 1, 33, m, fx);
+            for (int n = 0; n < 3; ++n) S.FX[n][sr][32] = fx[n];
+        }
+        __syncthreads();
+        // ---- divergence and the mode's epilogue
+        if (live) {
+            const long long t = ((long long)k * g.ny + j) * g.nx + i;
+#pragma unroll
+            for (int n = 0; n < 3; ++n) {
+                const double acc = ((S.FX[n][w][l + 1] - fx[n]) + (S.FY[n][w + 1][l] - fy[n])) + (fzn[n] - fz[n]);
+                const long long o = n * N + t;
+                if (E.mode == 0) {
+                    out[o] = acc;
+                } else if (E.mode == 1) {
+                    out[o] = acc;
+                    E.forces[o] = (E.src[o] + acc) * irho;
+                } else if (E.mode == 2) {
+                    out[o] = E.base[o] + 0.5 * dt * (acc - E.dold[o]) * irho;
+                } else if (E.mode == 3) {
+                    out[o] = (rho * E.base[o] + dt * (0.5 * (E.conv_o[o] + E.conv_n[o]) + 0.5 * E.dold[o] + 0.5 * acc + E.src[o])) * irho;
+                } else {
+                    const double r = E.base[o] - rho * pc.v[n] + dt * acc;
+                    rmax = imax_abs(rmax, r);
+                    out[o] = E.mode == 7 ? pc.v[n] + E.omega * E.dinv[o] * r : r;
+                }
+            }
+        }
+        pc = pn;
+        for (int n = 0; n < 3; ++n) fz[n] = fzn[n];
+        // layer k + 2 replaces layer k - 1 (read before the first barrier) and
+        // the viscosity of layer k (before the second)
+        if (more) stage(nxt, sm, k + 2);
+        const int s = sm;
+        sm = sc;
+        sc = sp;
+        sp = s;
+        __syncthreads();
+    }
     if (!E.parts) return;  // uniform over the block
-    for (int o = 16; o > 0; o >>= 1) rmax = nmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-    __shared__ double wmax[TTX * TTY * TTZ / 32];
-    if ((tid & 31) == 0) wmax[tid >> 5] = rmax;
+    for (int o = 16; o > 0; o >>= 1) {
+        const long long b = __shfl_xor_sync(0xffffffffu, rmax, o);
+        rmax = b > rmax ? b : rmax;
+    }
+    __shared__ long long wmax[TY];
+    if (mainw && l == 0) wmax[w] = rmax;
     __syncthreads();
     if (tid == 0) {
-        double b = 0.0;
-        for (int w = 0; w < TTX * TTY * TTZ / 32; ++w) b = nmax(b, wmax[w]);
-        E.parts[(blockIdx.z * (long long)gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = b;
+        for (int r = 0; r < TY; ++r) rmax = wmax[r] > rmax ? wmax[r] : rmax;
+        E.parts[(blockIdx.z * (long long)gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = bitsd(rmax);
     }
+}
+
+// Launch shape: rows a block and layers a march.  A march does about 0.6
+// layers' work more than its layers (the low z face and two staged layers), and
+// an SM runs two blocks at a time, so the march is the one whose blocks, dealt
+// to 304 places, finish first: 96^3 takes 12 layers (177 us; 210 at 1, 232 at
+// 16), 128x128x64 16 (232; 217 at 4), 64^3 4 (66; 101 at
+// 12, 253 at 32), 256x256x128 16 (1571; 1544 at 8, 1886 at 1).  Blocks of 4
+// rows only where those of 8 leave places empty: 32x32x16 12 us against 16.
+struct TauShape {
+    int ty, kc;
+    dim3 grid;
+};
+inline TauShape tau_shape(const Grid& g) {
+    TauShape s{8, 1, dim3(1, 1, 1)};
+    const int bx = (g.nx + 31) / 32;
+    if ((long long)bx * ((g.ny + 7) / 8) * g.nz < 304) s.ty = 4;  // small grids: more blocks
+    const int by = (g.ny + s.ty - 1) / s.ty;
+    double best = 0.0;
+    for (int kc = 1; kc <= 16 && kc <= g.nz; ++kc) {
+        const long long blocks = (long long)bx * by * ((g.nz + kc - 1) / kc);
+        const double cost = (double)((blocks + 303) / 304) * (kc + 0.6);
+        if (kc == 1 || cost < best) {
+            best = cost;
+            s.kc = kc;
+        }
+    }
+    s.grid = dim3((unsigned)bx, (unsigned)by, (unsigned)((g.nz + s.kc - 1) / s.kc));
+    return s;
 }
 
 // predictor_rhs (src/equation_systems/CompRHSOps.H:32-141); fac = 1 explicit,
@@ -1015,35 +1265,42 @@ void launch_divtau_faces(Ctx& c, const Grid& g, const double* vel, const double*
     KS_LAUNCH(c, k_tau_div, nblocks(g.N, BS), BS, B8 * per_cell * g.N, g, F, out, mode, src, forces, base, dold, dt, rho);
 }
 
+static void launch_divtau_col(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, const TauEpi& E,
+                              double bytes) {
+    const TauShape s = tau_shape(g);
+    const TauCoef K = tau_coef(g);
+    if (s.ty == 4) {
+        KS_LAUNCH_SMEM(c, k_divtau_col<4>, s.grid, 32 * 7, sizeof(TauPlanes<4>), bytes, g, K, vel, mueff, wg, out, E, s.kc);
+    } else {
+        cudaFuncSetAttribute(k_divtau_col<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TauPlanes<8>));
+        KS_LAUNCH_SMEM(c, k_divtau_col<8>, s.grid, 32 * 11, sizeof(TauPlanes<8>), bytes, g, K, vel, mueff, wg, out, E, s.kc);
+    }
+}
+static_assert(sizeof(TauPlanes<4>) <= 48 * 1024, "needs no shared memory attribute");
 void launch_divtau(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, int mode,
-                   const double* src, double* forces, const double* base, const double* dold, double dt, double rho, double* const fl[9],
-                   int fp32) {
-    (void)fl;  // the tiled kernel keeps its face fluxes in shared memory
-    const dim3 grid((g.nx + TTX - 1) / TTX, (g.ny + TTY - 1) / TTY, (g.nz + TTZ - 1) / TTZ);
+                   const double* src, double* forces, const double* base, const double* dold, double dt, double rho, int fp32) {
     const double per_cell = 4 + 3 + (mode == 1 ? 6 : 0) + (mode == 2 ? 6 : 0);
     TauEpi E{mode, src, base, dold, nullptr, nullptr, nullptr, forces, nullptr, dt, rho, 0.0, 1.0 / rho};
     if (fp32) {
-        cudaFuncSetAttribute(k_divtau_tile<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tau_smem<float>());
-        KS_LAUNCH_SMEM(c, k_divtau_tile<float>, grid, TTX * TTY * TTZ, tau_smem<float>(), B8 * per_cell * g.N, g, vel, mueff, wg, out, E);
+        const dim3 grid((g.nx + TTX - 1) / TTX, (g.ny + TTY - 1) / TTY, (g.nz + TTZ - 1) / TTZ);
+        KS_LAUNCH_SMEM(c, k_divtau_tile, grid, TTX * TTY * TTZ, tau_smem(), B8 * per_cell * g.N, g, vel, mueff, wg, out, E);
     } else {
-        cudaFuncSetAttribute(k_divtau_tile<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tau_smem<double>());
-        KS_LAUNCH_SMEM(c, k_divtau_tile<double>, grid, TTX * TTY * TTZ, tau_smem<double>(), B8 * per_cell * g.N, g, vel, mueff, wg, out, E);
+        launch_divtau_col(c, g, vel, mueff, wg, out, E, B8 * per_cell * g.N);
     }
 }
 void launch_divtau_corrector(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, const double* vel_old,
                              const double* conv_old, const double* conv_new, const double* dold, const double* src, double dt, double rho) {
-    cudaFuncSetAttribute(k_divtau_tile<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tau_smem<double>());
-    const dim3 grid((g.nx + TTX - 1) / TTX, (g.ny + TTY - 1) / TTY, (g.nz + TTZ - 1) / TTZ);
     TauEpi E{3, src, vel_old, dold, conv_old, conv_new, nullptr, nullptr, nullptr, dt, rho, 0.0, 1.0 / rho};
-    KS_LAUNCH_SMEM(c, k_divtau_tile<double>, grid, TTX * TTY * TTZ, tau_smem<double>(), B8 * 22.0 * g.N, g, vel, mueff, wg, out, E);
+    launch_divtau_col(c, g, vel, mueff, wg, out, E, B8 * 22.0 * g.N);
 }
-int divtau_tile_blocks(const Grid& g) { return ((g.nx + TTX - 1) / TTX) * ((g.ny + TTY - 1) / TTY) * ((g.nz + TTZ - 1) / TTZ); }
+int divtau_blocks(const Grid& g) {
+    const TauShape s = tau_shape(g);
+    return (int)(s.grid.x * s.grid.y * s.grid.z);
+}
 void launch_divtau_jacobi(Ctx& c, const Grid& g, const double* x, const double* mueff, const double* wg, const double* b, const double* dinv,
                           double* out, double rho, double dtd, double omega, double* parts) {
-    cudaFuncSetAttribute(k_divtau_tile<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tau_smem<double>());
-    const dim3 grid((g.nx + TTX - 1) / TTX, (g.ny + TTY - 1) / TTY, (g.nz + TTZ - 1) / TTZ);
     TauEpi E{omega > 0.0 ? 7 : 8, nullptr, b, nullptr, nullptr, nullptr, dinv, nullptr, parts, dtd, rho, omega, 1.0 / rho};
-    KS_LAUNCH_SMEM(c, k_divtau_tile<double>, grid, TTX * TTY * TTZ, tau_smem<double>(), B8 * ((omega > 0.0 ? 13.0 : 10.0) * g.N), g, x, mueff, wg, out, E);
+    launch_divtau_col(c, g, x, mueff, wg, out, E, B8 * ((omega > 0.0 ? 13.0 : 10.0) * g.N));
 }
 void launch_predictor_rhs(Ctx& c, const Grid& g, const double* vo, const double* conv, const double* src, const double* dtau, double* vel,
                           double dt, double rho, double fac) {

@@ -152,24 +152,23 @@ void launch_wall_grad(Ctx& c, const Grid& g, const double* vel_old, const double
                       double um0, double um1, double vmag, double rho);
 // out = divtau(vel) ; mode 0: plain, mode 1: forces = (src + divtau)/rho also written,
 // mode 2: out = base + 0.5*dt*(divtau(vel) - dold)/rho (RK2 correction into out).
-// Fused shared-memory tiles; face_scratch is not used.
+// Fused: no face arrays touch memory.
 // fp32 = 1 (modes 0-2): staging, face fluxes and divergence in FP32 (mixed-precision form), epilogue in FP64
 void launch_divtau(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, int mode,
-                   const double* src, double* forces, const double* base, const double* dold, double dt, double rho,
-                   double* const face_scratch[9], int fp32 = 0);
+                   const double* src, double* forces, const double* base, const double* dold, double dt, double rho, int fp32 = 0);
 // the same result through face-flux arrays in caller-provided scratch (9 arrays:
 // N cells for x and y faces, nx*ny*(nz+1) for z faces) and a divergence pass
 void launch_divtau_faces(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, int mode,
                          const double* src, double* forces, const double* base, const double* dold, double dt, double rho,
                          double* const face_scratch[9]);
-// MOL corrector_rhs (explicit) fused into the tiled divtau of vel:
+// MOL corrector_rhs (explicit) fused into the divtau of vel:
 // out = (rho u_old + dt (0.5 (conv_old + conv_new) + 0.5 (dold + divtau(vel)) + src)) / rho
 void launch_divtau_corrector(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, const double* vel_old,
                              const double* conv_old, const double* conv_new, const double* dold, const double* src, double dt, double rho);
 // Tensor-diffusion solve passes on any level grid g: out = x + omega dinv (b - rho x + dtd divtau(x))
 // (omega > 0, a Jacobi sweep) or out = b - rho x + dtd divtau(x) (omega = 0, the residual), with
-// block maxima of the residual's magnitude in parts (divtau_tile_blocks(g) entries) when parts is set.
-int divtau_tile_blocks(const Grid& g);
+// block maxima of the residual's magnitude in parts (divtau_blocks(g) entries) when parts is set.
+int divtau_blocks(const Grid& g);
 void launch_divtau_jacobi(Ctx& c, const Grid& g, const double* x, const double* mueff, const double* wg, const double* b, const double* dinv,
                           double* out, double rho, double dtd, double omega, double* parts);
 // predictor_rhs: vel = (rho vel_old + dt (conv + src + fac divtau)) / rho
