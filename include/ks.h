@@ -187,12 +187,13 @@ int ks_fma_peak(int fp64, double* gflops);
  * legacy default stream), with the boundary treatment of the advance: x and y
  * periodic; z periodic or slip walls, or a wall-model bottom whose wall-normal
  * tangential-velocity gradient is given in wall_grad (2 x nx*ny, device).
- * Its face-flux scratch lives in a static device array sized for at most
- * KS_NOALLOC_MAX_CELLS cells (about 24 MB, held by every GPU that loads the
- * library until exit); larger grids are rejected with KS_ERR_ARG.  The first
- * call on a device looks up that array's address with that device current;
- * make that first call before any stream capture.  All calls share the
- * array: calls whose kernels overlap on the GPU race, order them.  A CUDA
+ * One launch.  A call whose output overlaps an input keeps face fluxes in a
+ * static device array sized for at most KS_NOALLOC_MAX_CELLS cells (about 24
+ * MB, held by every GPU that loads the library until exit); larger grids are
+ * rejected with KS_ERR_ARG.  The first such call on a device looks up that
+ * array's address with that device current; make it before any stream
+ * capture.  All such calls share the array: those whose kernels overlap on
+ * the GPU race, order them.  A CUDA
  * error already pending on the calling thread is left in place and the call
  * returns KS_ERR_CUDA without launching; calls after cudaDeviceReset are not
  * supported. */
