@@ -94,10 +94,6 @@ using CellFO = CellFOT<double>;
 
 inline unsigned nblocks(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
-// max that keeps a NaN operand (fmax drops it): a non-finite residual or CFL
-// maximum must reach the host's finiteness checks
-__host__ __device__ inline double nmax(double a, double b) { return (a != a || b != b) ? a + b : (a > b ? a : b); }
-
 // ---- FP64 decisions on the integer pipe.
 // On this GPU every FP64 instruction -- DFMA, DADD, DMUL, and also the
 // compares (DSETP) and min/max (DMNMX) -- issues at one sixty-fourth of the
@@ -109,8 +105,18 @@ __host__ __device__ inline double nmax(double a, double b) { return (a != a || b
 // are not ordered like IEEE does; a NaN field still reaches the host through
 // the arithmetic it enters and the residual / CFL maxima (imax_abs keeps it).
 #ifdef __CUDACC__
-__device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
-__device__ __forceinline__ double bitsd(long long b) { return __longlong_as_double(b); }
+// The casts are opaque moves: given __double_as_longlong the compiler recognises
+// masks and comparisons of the pattern and turns them back into FP64 compares.
+__device__ __forceinline__ long long dbits(double x) {
+    long long b;
+    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+    return b;
+}
+__device__ __forceinline__ double bitsd(long long b) {
+    double x;
+    asm("mov.b64 %0, %1;" : "=d"(x) : "l"(b));
+    return x;
+}
 constexpr long long kMag = 0x7fffffffffffffffLL;
 // signed integer with the order of the doubles
 __device__ __forceinline__ long long okey(double x) {
@@ -127,7 +133,12 @@ __device__ __forceinline__ bool ige0(double x) { return okey(x) >= -1; }  // x >
 __device__ __forceinline__ bool ilt(double a, double b) { return okey(a) < okey(b); }
 __device__ __forceinline__ double imin(double a, double b) { return okey(a) < okey(b) ? a : b; }
 __device__ __forceinline__ double imax(double a, double b) { return okey(a) > okey(b) ? a : b; }
-__device__ __forceinline__ double iabs(double x) { return bitsd(dbits(x) & kMag); }
+// Magnitudes and signs are taken on the high word: the compiler turns the same
+// masks on the 64-bit pattern back into fabs, copysign and negation, which
+// issue as FP64 instructions.
+__device__ __forceinline__ double hiword(double x, int hi) { return __hiloint2double(hi, __double2loint(x)); }
+__device__ __forceinline__ double iabs(double x) { return hiword(x, __double2hiint(x) & 0x7fffffff); }
+__device__ __forceinline__ double ineg(double x) { return hiword(x, __double2hiint(x) ^ (int)0x80000000); }
 // |x| < c for c > 0
 __device__ __forceinline__ bool iabs_lt(double x, double c) { return (dbits(x) & kMag) < dbits(c); }
 // |a| < |b|
@@ -136,8 +147,17 @@ __device__ __forceinline__ bool iabs_lt2(double a, double b) { return (dbits(a) 
 __device__ __forceinline__ bool isame_sign(double a, double b) {
     return (dbits(a) ^ dbits(b)) >= 0 && (dbits(a) & kMag) != 0 && (dbits(b) & kMag) != 0;
 }
-// copysign(m, s) for m >= 0
-__device__ __forceinline__ double isign(double m, double s) { return bitsd(dbits(m) | (dbits(s) & ~kMag)); }
+// copysign(m, s)
+__device__ __forceinline__ double isign(double m, double s) {
+    return hiword(m, (__double2hiint(m) & 0x7fffffff) | (__double2hiint(s) & (int)0x80000000));
+}
+// max that keeps a NaN operand (fmax drops it): a non-finite residual or CFL
+// maximum must reach the host's finiteness checks
+__device__ __forceinline__ double nmax(double a, double b) {
+    if ((dbits(a) & kMag) > 0x7ff0000000000000LL) return a;
+    if ((dbits(b) & kMag) > 0x7ff0000000000000LL) return b;
+    return imax(a, b);
+}
 // running max of |x| kept as bits: NaN patterns order above infinity, so a
 // NaN operand survives to the host
 __device__ __forceinline__ long long imax_abs(long long m, double x) {

@@ -14,7 +14,7 @@ __device__ inline bool same_sign(double a, double b) { return isame_sign(a, b); 
 __device__ inline bool same_sign(float a, float b) { return a * b > 0.0f; }
 __device__ inline bool abs_lt(double a, double b) { return iabs_lt2(a, b); }  // |a| < |b|
 __device__ inline bool abs_lt(float a, float b) { return fabsf(a) < fabsf(b); }
-__device__ inline double mag_sign(double m, double s) { return isign(iabs(m), s); }  // |m| with the sign of s
+__device__ inline double mag_sign(double m, double s) { return isign(m, s); }  // |m| with the sign of s
 __device__ inline float mag_sign(float m, float s) { return copysignf(fabsf(m), s); }
 __device__ inline double clip2(double e, double a, double b) { return imin(imax(e, imin(a, b)), imax(a, b)); }
 __device__ inline float clip2(float e, float a, float b) { return fminf(fmaxf(e, fminf(a, b)), fmaxf(a, b)); }
@@ -32,7 +32,7 @@ __device__ inline bool below_small_abs(double u) { return iabs_lt(u, kSmallVel);
 __device__ inline bool below_small_abs(float u) { return fabsf(u) < (float)kSmallVel; }
 __device__ inline double absv(double x) { return iabs(x); }
 __device__ inline float absv(float x) { return fabsf(x); }
-__device__ inline double neg_if(bool c, double x) { return c ? bitsd(dbits(x) ^ ~kMag) : x; }
+__device__ inline double neg_if(bool c, double x) { return hiword(x, __double2hiint(x) ^ (c ? (int)0x80000000 : 0)); }
 __device__ inline float neg_if(bool c, float x) { return c ? -x : x; }
 __device__ inline double min2(double a, double b) { return imin(a, b); }
 __device__ inline float min2(float a, float b) { return fminf(a, b); }
@@ -42,6 +42,38 @@ __device__ inline bool lt(double a, double b) { return ilt(a, b); }  // a < b
 __device__ inline bool lt(float a, float b) { return a < b; }
 __device__ inline bool nonzero(double x) { return (dbits(x) & kMag) != 0; }
 __device__ inline bool nonzero(float x) { return x != 0.0f; }
+
+// The FP64 forms below spend fewer FP64 instructions: scaling by a power of two
+// is an addition to the exponent field (a result below the normal range becomes
+// zero), and a choice is made before the arithmetic it selects, for an
+// instruction that is predicated off still takes its FP64 issue slot.
+constexpr long long kExp1 = 1LL << 52;
+__device__ inline double twice(double x) { return hiword(x, __double2hiint(x) + 0x00100000); }  // x finite, not 0
+__device__ inline double half_fin(double x) {  // x finite
+    const int h = __double2hiint(x);
+    return (h & 0x7fffffff) >= 0x00200000 ? hiword(x, h - 0x00100000) : 0.0;
+}
+__device__ inline double half_of(double x) {  // infinities and NaN are kept
+    return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000 ? x : half_fin(x);
+}
+
+// van Leer (monotonized-central) limited slope of the middle cell of (a, b, c)
+// from l = b - a, r = c - b and d = c - a: copysign(min(|d / 2|, |2 l|, |2 r|), d)
+// where l r > 0, else 0.  (A non-finite neighbour reaches the edge through its
+// value and difference, whatever the slope.)
+__device__ inline double vls3(double l, double r, double d) {
+    if (!same_sign(l, r)) return 0.0;
+    const double m = abs_lt(l, r) ? l : r;
+    if ((dbits(d) & kMag) < (dbits(m) & kMag) + 2 * kExp1) return half_fin(d);
+    return mag_sign(twice(m), d);
+}
+__device__ inline float vls3(float l, float r, float d) {
+    const float dsc = 0.5f * d, dsl = 2.0f * l, dsr = 2.0f * r;
+    if (!same_sign(dsl, dsr)) return 0.0f;
+    float m = abs_lt(dsl, dsr) ? dsl : dsr;
+    m = abs_lt(dsc, m) ? dsc : m;
+    return mag_sign(m, dsc);
+}
 
 #endif
 

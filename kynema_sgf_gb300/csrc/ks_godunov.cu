@@ -31,71 +31,106 @@ constexpr int BS = 256;
 
 inline long long nfaces(const Grid& g, int d) { return (long long)g.nx * g.ny * (d == 2 ? nzfaces(g) : g.nz); }
 
-// van Leer limited slope of the middle cell of (a, b, c):
-// copysign(min(|dsc|, |dsl|, |dsr|), dsc) where dsl dsr > 0, else 0
-template <typename T>
-__device__ inline T vls(T a, T b, T c) {
-    const T dsc = T(0.5) * (c - a), dsl = T(2) * (b - a), dsr = T(2) * (c - b);
-    if (!same_sign(dsl, dsr)) return T(0);
-    T m = abs_lt(dsl, dsr) ? dsl : dsr;
-    m = abs_lt(dsc, m) ? dsc : m;
-    return mag_sign(m, dsc);
+// The FP64 forms of the edge, the parabola and the trace share differences with
+// their neighbours: 12 FP64 instructions a component of a pre-MAC cell with the
+// slope (vls3), where the plain forms take 21.  Slopes and limited parabolas
+// are the same bits as the plain forms; edges and traces differ in their last
+// bit or two.
+//
+// unlimited PPM edge value between cells with values a0, a1 = a0 + l and
+// slopes s0, s1, clipped to the two cells
+__device__ inline double ppm_edge(double a0, double a1, double l, double s0, double s1) {
+    return clip2(fma(-1.0 / 6.0, s1 - s0, fma(0.5, l, a0)), a0, a1);
 }
-
-// unlimited PPM edge value between cells with values a0, a1 and slopes s0, s1,
-// clipped to the two cells
-template <typename T>
-__device__ inline T ppm_edge(T a0, T a1, T s0, T s1) {
-    return clip2(T(0.5) * (a0 + a1) - T(1.0 / 6.0) * (s1 - s0), a0, a1);
+__device__ inline float ppm_edge(float a0, float a1, float, float s0, float s1) {
+    return clip2(0.5f * (a0 + a1) - float(1.0 / 6.0) * (s1 - s0), a0, a1);
 }
 
 // Edge value on the face with index k along d from the cell values
-// a(k-2), a(k-1), a(k), a(k+1) and the slopes s(k-1), s(k).  Wall-bounded z:
+// a(k-2), a(k-1), a(k), a(k+1), l = a(k) - a(k-1) and the slopes s(k-1), s(k).  Wall-bounded z:
 // the wall faces take the boundary (ghost) value, the faces one cell inside
 // the one-sided fourth-order formula clipped to the two adjacent cells.
 template <typename T>
-__device__ inline T edge_at(bool walls, int k, int nz, T am2, T am1, T a0, T ap1, T sm1, T s0) {
+__device__ inline T edge_at(bool walls, int k, int nz, T am2, T am1, T a0, T ap1, T l, T sm1, T s0) {
     if (walls) {
         if (k == 0) return am1;
         if (k == nz) return a0;
         if (k == 1) return clip2(T(-0.2) * am2 + T(0.75) * am1 + T(0.5) * a0 - T(0.05) * ap1, am1, a0);
         if (k == nz - 1) return clip2(T(-0.2) * ap1 + T(0.75) * a0 + T(0.5) * am1 - T(0.05) * am2, a0, am1);
     }
-    return ppm_edge(am1, a0, sm1, s0);
+    return ppm_edge(am1, a0, l, sm1, s0);
 }
 
 // limited parabola of a cell (Colella-Woodward 1984): (sm, sp) from its two
 // edges and the cell value s0.  3 s0 - 2 sm = s0 + 2 (s0 - sm), and
-// 3 s0 - 2 sp = s0 - 2 (sp - s0).
-template <typename T>
-__device__ inline void cw84(T s0, T& sm, T& sp) {
-    const T dp = sp - s0, dm = s0 - sm;
+// 3 s0 - 2 sp = s0 - 2 (sp - s0).  FP64: dp = sp - s0 and dm = s0 - sm of the
+// limited parabola are returned for the trace.
+__device__ inline void cw84(float s0, float& sm, float& sp, float&, float&) {
+    const float dp = sp - s0, dm = s0 - sm;
     if (!same_sign(dp, dm)) {
         sp = s0;
         sm = s0;
         return;
     }
-    const T dp2 = T(2) * dp, dm2 = T(2) * dm;
+    const float dp2 = 2.0f * dp, dm2 = 2.0f * dm;
     if (!abs_lt(dp, dm2)) sp = s0 + dm2;
     else if (!abs_lt(dm, dp2)) sm = s0 - dp2;
+}
+__device__ inline void cw84(double s0, double& sm, double& sp, double& dm, double& dp) {
+    dp = sp - s0;
+    dm = s0 - sm;
+    if (!same_sign(dp, dm)) {
+        sp = sm = s0;
+        dp = dm = 0.0;
+        return;
+    }
+    const long long mp = dbits(dp) & kMag, mm = dbits(dm) & kMag;
+    const bool hi = mp >= mm + kExp1, lo = !hi && mm >= mp + kExp1;
+    if (hi) dp = twice(dm);
+    if (lo) dm = twice(dp);
+    const double t = s0 + (hi ? dp : ineg(dm));
+    sp = hi ? t : sp;
+    sm = lo ? t : sm;
 }
 
 // Average of the limited parabola (sm, s0, sp) over the part of the cell that
 // crosses its high face (hi = true) or low face in dt, sig = |u| dt / h:
 //   high: sp - h D + h g s6,   low: sm + h D + h g s6,
-// h = sig / 2, g = 1 - 2 sig / 3, D = sp - sm, s6 = 6 s0 - 3 (sm + sp).
+// h = sig / 2, g = 1 - 2 sig / 3, D = sp - sm = dp + dm,
+// s6 = 6 s0 - 3 (sm + sp) = 3 (dm - dp).  TraceCoef holds h and h g (FP32) or
+// 3 h g = h (3 - 4 h) (FP64) for u = |u| and s = dt / h.
 template <typename T>
-struct TraceCoef {
-    T h, hg;
-    __device__ inline TraceCoef(T sig) {
-        h = T(0.5) * sig;
-        hg = h * (T(1) - T(2.0 / 3.0) * sig);
+struct TraceCoef;
+template <>
+struct TraceCoef<float> {
+    float h, hg;
+    __device__ inline TraceCoef(float u, float s) {
+        const float sig = u * s;
+        h = 0.5f * sig;
+        hg = h * (1.0f - float(2.0 / 3.0) * sig);
     }
 };
-template <typename T>
-__device__ inline T ppm_trace(bool hi, T sm, T s0, T sp, const TraceCoef<T>& c) {
-    const T D = sp - sm, s6 = T(6) * s0 - T(3) * (sm + sp);
+template <>
+struct TraceCoef<double> {
+    double h, hg;
+    __device__ inline TraceCoef(double u, double s) {
+        h = u * half_of(s);
+        hg = h * fma(-4.0, h, 3.0);
+    }
+};
+__device__ inline float ppm_trace(bool hi, float sm, float s0, float sp, const TraceCoef<float>& c) {
+    const float D = sp - sm, s6 = 6.0f * s0 - 3.0f * (sm + sp);
     return c.hg * s6 + (neg_if(hi, c.h) * D + (hi ? sp : sm));
+}
+__device__ inline double ppm_trace(bool hi, double sm, double s0, double sp, const TraceCoef<double>& c) {
+    return fma(c.hg, fma(2.0, s0, -(sm + sp)), fma(neg_if(hi, c.h), sp - sm, hi ? sp : sm));
+}
+// the same with the parabola's dm, dp at hand (cw84)
+__device__ inline float ppm_trace(bool hi, float sm, float s0, float sp, float, float, const TraceCoef<float>& c) {
+    return ppm_trace(hi, sm, s0, sp, c);
+}
+__device__ inline double ppm_trace(bool hi, double sm, double, double sp, double dm, double dp, const TraceCoef<double>& c) {
+    return fma(c.hg, dm - dp, fma(neg_if(hi, c.h), dm + dp, hi ? sp : sm));
 }
 
 // Wall face treatment (SetZEdgeBCs): tangential components take the interior
@@ -112,10 +147,24 @@ __device__ inline void zbc(const Grid& g, int k, int n, T& lo, T& hi) {
 
 // upwind state with AMReX-Hydro's small_vel: the mean of both states where
 // |vel| < small_vel
-template <typename T>
-__device__ inline T upwind(T vel, T lo, T hi) {
-    if (below_small_abs(vel)) return T(0.5) * (lo + hi);
-    return ge0(vel) ? lo : hi;
+__device__ inline double upwind(double vel, double lo, double hi) {
+    // half the sum of the chosen state with itself, or of both: one FP64
+    // instruction, where the mean formed beside the choice (a predicated
+    // instruction still takes its issue slot) costs two
+    const bool m = below_small_abs(vel), up = ge0(vel);
+    return half_of((m || up ? lo : hi) + (m || !up ? hi : lo));
+}
+// the same for NC components of a face: one branch to the means, which are rare
+template <typename T, int NC, typename St>
+__device__ inline void upwind_n(T vel, const T (&lo)[NC], const T (&hi)[NC], const St& st) {
+    if (below_small_abs(vel)) {
+#pragma unroll
+        for (int n = 0; n < NC; ++n) st(n, T(0.5) * (lo[n] + hi[n]));
+        return;
+    }
+    const bool up = ge0(vel);
+#pragma unroll
+    for (int n = 0; n < NC; ++n) st(n, up ? lo[n] : hi[n]);
 }
 template <typename T>
 __device__ inline T riemann(T lo, T hi) {
@@ -123,6 +172,22 @@ __device__ inline T riemann(T lo, T hi) {
     const bool ltm = (le0(lo) && ge0(hi)) || below_small_abs(sum);
     return ltm ? T(0) : (ge0(sum) ? lo : hi);
 }
+
+// Side a face's upwinded state is formed from: the low cell's where vel >= 0,
+// the mean of both where |vel| < small_vel, the cell inside the domain on a
+// wall face (zbc: both states are that cell's there, the normal component's
+// zero).  One side's state is corrected, not both.  FP64, bound by issue, loads
+// that side alone and branches to the mean (256x256x128, k_adv_trans_col 785 us
+// against 1078 with both loaded and the mean selected); FP32, bound by memory,
+// loads both and selects (512x512x256, k_adv_flux_col 2.64 ms against 2.79).
+struct UpSide {
+    bool low, mean;
+    template <typename T>
+    __device__ inline UpSide(T vel, bool wl, bool wh) {
+        mean = !wl && !wh && below_small_abs(vel);
+        low = !wl && (wh || ge0(vel));
+    }
+};
 
 template <typename T>
 struct P3 {
@@ -137,7 +202,7 @@ struct C3 {
 // MODE 0 (pre-MAC): the characteristic speed of a cell is its velocity
 // component d, so one trace per cell (its downwind face; the other face
 // takes the cell value).  Computes the unlimited edges from the slopes and
-// stores them (reused by the post-MAC pass), writes the left/right states, the
+// stores them where a reverse step will read them, writes the left/right states, the
 // Riemann-solved advective velocity and the two transverse components
 // upwinded with it.
 // MODE 1 (post-MAC): the speed is the MAC velocity of the face, so one trace
@@ -158,7 +223,7 @@ struct PpmArgs {
 
 template <typename T, int NC>
 struct PpmOut {
-    T* E[3];   // unlimited edges (MODE 0 writes them for the adjoint)
+    T* E[3];   // unlimited edges (MODE 0 writes them for the reverse mode; null without one)
     T* PM[3];  // limited parabola (sm, sp) of every cell (MODE 0 writes, MODE 1 EDGES = 0 reads)
     T* PP[3];
     T* LO[3];  // left / right states
@@ -176,7 +241,7 @@ __device__ inline void face_states_mac(T u, T s, T pm, T p0, T pp, T qm, T q0, T
     h = q0;
     const bool up = above_small(u), dn = below_msmall(u);
     if (up || dn) {
-        const TraceCoef<T> c(absv(u) * s);
+        const TraceCoef<T> c(absv(u), s);
         const T t = ppm_trace(up, up ? pm : qm, up ? p0 : q0, up ? pp : qp, c);
         if (up) l = t;
         else h = t;
@@ -215,9 +280,9 @@ __global__ void __launch_bounds__(256) k_ppm_col(PpmArgs<T> A, T s, T rho, PpmOu
     };
     auto fid = [&](int m) -> long long { return d == 1 ? fidx(g, 1, i, m, o) : fidx(g, 2, i, o, m); };
     auto cellid = [&](int m) -> long long { return d == 1 ? cidx(g, i, m, o) : cidx(g, i, o, m); };  // 0 <= m < nl
-    // per component at face m: a(m-1), a(m), a(m+1), the slope s(m), the edge
+    // per component at face m: a(m-1), a(m), a(m+1), r0 = a(m+1) - a(m), the slope s(m), the edge
     // e(m), and cell m-1's high-face trace (MODE 0) or limited parabola (MODE 1)
-    T am1[NC], a0[NC], ap1[NC], sl0[NC], e0[NC], lo0[NC], pm[NC], pp[NC];
+    T am1[NC], a0[NC], ap1[NC], sl0[NC], e0[NC], lo0[NC], pm[NC], pp[NC], r0[NC];
     {
         T u = T(0);
         if (MODE == 0) u = val(d, m0 - 1);
@@ -240,17 +305,19 @@ __global__ void __launch_bounds__(256) k_ppm_col(PpmArgs<T> A, T s, T rho, PpmOu
             } else {
                 const T x3 = val(n, m0 - 3), x2 = val(n, m0 - 2);
                 ap1[n] = val(n, m0 + 1);
-                const T s2 = vls(x3, x2, am1[n]), s1 = vls(x2, am1[n], a0[n]);
-                sl0[n] = vls(am1[n], a0[n], ap1[n]);
-                em1 = edge_at(walls, m0 - 1, g.nz, x3, x2, am1[n], a0[n], s2, s1);
-                e0[n] = edge_at(walls, m0, g.nz, x2, am1[n], a0[n], ap1[n], s1, sl0[n]);
+                const T l2 = am1[n] - x2, l1 = a0[n] - am1[n];
+                r0[n] = ap1[n] - a0[n];
+                const T s2 = vls3(x2 - x3, l2, am1[n] - x3), s1 = vls3(l2, l1, a0[n] - x2);
+                sl0[n] = vls3(l1, r0[n], ap1[n] - am1[n]);
+                em1 = edge_at(walls, m0 - 1, g.nz, x3, x2, am1[n], a0[n], l2, s2, s1);
+                e0[n] = edge_at(walls, m0, g.nz, x2, am1[n], a0[n], ap1[n], l1, s1, sl0[n]);
             }
-            T sm = em1, sp = e0[n];
-            cw84(am1[n], sm, sp);
+            T sm = em1, sp = e0[n], dm, dp;
+            cw84(am1[n], sm, sp, dm, dp);
             pm[n] = sm;
             pp[n] = sp;
             lo0[n] = am1[n];
-            if (MODE == 0 && above_small(u)) lo0[n] = ppm_trace(true, sm, am1[n], sp, TraceCoef<T>(absv(u) * s));
+            if (MODE == 0 && above_small(u)) lo0[n] = ppm_trace(true, sm, am1[n], sp, dm, dp, TraceCoef<T>(absv(u), s));
         }
     }
     for (int m = m0; m < m1; ++m) {
@@ -262,26 +329,28 @@ __global__ void __launch_bounds__(256) k_ppm_col(PpmArgs<T> A, T s, T rho, PpmOu
                 ap1[n] = val(n, m + 1);
             } else {
                 ap2[n] = val(n, m + 2);
-                s1[n] = vls(a0[n], ap1[n], ap2[n]);
-                e1[n] = edge_at(walls, m + 1, g.nz, am1[n], a0[n], ap1[n], ap2[n], sl0[n], s1[n]);
+                const T r1 = ap2[n] - ap1[n];
+                s1[n] = vls3(r0[n], r1, ap2[n] - a0[n]);
+                e1[n] = edge_at(walls, m + 1, g.nz, am1[n], a0[n], ap1[n], ap2[n], r0[n], sl0[n], s1[n]);
+                r0[n] = r1;
             }
         }
         T lo[NC], hi[NC];
         if (MODE == 0) {
             const T u = sel(a0, d);  // cell m's velocity component d
             const bool up = above_small(u), dn = below_msmall(u);
-            const TraceCoef<T> c(absv(u) * s);
+            const TraceCoef<T> c(absv(u), s);
 #pragma unroll
             for (int n = 0; n < NC; ++n) {
-                T sm = e0[n], sp = e1[n];
-                cw84(a0[n], sm, sp);
+                T sm = e0[n], sp = e1[n], dm, dp;
+                cw84(a0[n], sm, sp, dm, dp);
                 if (m < nl) {  // the post-MAC pass reads the limited parabola of every cell
                     O.PM[n][cellid(m)] = sm;
                     O.PP[n][cellid(m)] = sp;
                 }
                 T h = a0[n], lnext = a0[n];
                 if (up || dn) {
-                    const T t = ppm_trace(up, sm, a0[n], sp, c);
+                    const T t = ppm_trace(up, sm, a0[n], sp, dm, dp, c);
                     if (up) lnext = t;
                     else h = t;
                 }
@@ -305,7 +374,8 @@ __global__ void __launch_bounds__(256) k_ppm_col(PpmArgs<T> A, T s, T rho, PpmOu
                 } else {
                     sm = e0[n];
                     sp = e1[n];
-                    cw84(a0[n], sm, sp);
+                    T dm, dp;
+                    cw84(a0[n], sm, sp, dm, dp);
                 }
                 T l, h;
                 face_states_mac(u, s, pm[n], am1[n], pp[n], sm, a0[n], sp, l, h);
@@ -327,18 +397,16 @@ __global__ void __launch_bounds__(256) k_ppm_col(PpmArgs<T> A, T s, T rho, PpmOu
         for (int n = 0; n < NC; ++n) {
             O.LO[n][f] = lo[n];
             O.HI[n][f] = hi[n];
-            if (MODE == 0) O.E[n][f] = e0[n];
+            if (MODE == 0 && O.E[n]) O.E[n][f] = e0[n];
         }
         if (MODE == 0) {
             const T a = riemann(sel(lo, d), sel(hi, d));
             O.ad[f] = a;
-#pragma unroll
-            for (int n = 0; n < NC; ++n)
-                if (n != d) O.TE[n][f] = upwind(a, lo[n], hi[n]);
+            upwind_n(a, lo, hi, [&](int n, T v) {
+                if (n != d) O.TE[n][f] = v;
+            });
         } else {
-            const T u = (T)A.umac[f];
-#pragma unroll
-            for (int n = 0; n < NC; ++n) O.TE[n][f] = upwind(u, lo[n], hi[n]);
+            upwind_n((T)A.umac[f], lo, hi, [&](int n, T v) { O.TE[n][f] = v; });
         }
 #pragma unroll
         for (int n = 0; n < NC; ++n) {
@@ -383,11 +451,11 @@ __global__ void __launch_bounds__(256) k_ppm_x(PpmArgs<T> A, T s, T rho, PpmOut<
     if (MODE == 0) u = ld(0, c);
     else u = (T)A.umac[fc];
     const bool up = above_small(u), dn = below_msmall(u);
-    const TraceCoef<T> tc(absv(u) * s);
+    const TraceCoef<T> tc(absv(u), s);
     T pmv[NC], ppv[NC];
     for (int n = 0; n < NC; ++n) {
         const T a0 = ld(n, c);
-        T am1, sm, sp;
+        T am1, sm, sp, dm, dp;
         if (LOADE) {  // the limited parabola of the lane's cell, stored by the pre-MAC pass
             sm = O.PM[n][fc];
             sp = O.PP[n][fc];
@@ -396,21 +464,21 @@ __global__ void __launch_bounds__(256) k_ppm_x(PpmArgs<T> A, T s, T rho, PpmOut<
         } else {
             am1 = ld(n, c - 1);
             const T ap1 = ld(n, c + 1);
-            const T sl = vls(am1, a0, ap1);
+            const T l = a0 - am1, sl = vls3(l, ap1 - a0, ap1 - am1);
             const T slm = __shfl_up_sync(FULL, sl, 1);
-            const T e0 = ppm_edge(am1, a0, slm, sl);
+            const T e0 = ppm_edge(am1, a0, l, slm, sl);
             const T e1 = __shfl_down_sync(FULL, e0, 1);
             ev[n] = e0;
             sm = e0;
             sp = e1;
-            cw84(a0, sm, sp);
+            cw84(a0, sm, sp, dm, dp);
         }
         pmv[n] = sm;
         ppv[n] = sp;
         if (MODE == 0) {
             T h = a0, lnext = a0;
             if (up || dn) {
-                const T t = ppm_trace(up, sm, a0, sp, tc);
+                const T t = ppm_trace(up, sm, a0, sp, dm, dp, tc);
                 if (up) lnext = t;
                 else h = t;
             }
@@ -430,7 +498,7 @@ __global__ void __launch_bounds__(256) k_ppm_x(PpmArgs<T> A, T s, T rho, PpmOut<
         O.LO[n][fc] = lo[n];
         O.HI[n][fc] = hi[n];
         if (MODE == 0) {  // x faces and cells share the index: face c is owned with cell c
-            O.E[n][fc] = ev[n];
+            if (O.E[n]) O.E[n][fc] = ev[n];
             O.PM[n][fc] = pmv[n];
             O.PP[n][fc] = ppv[n];
         }
@@ -438,11 +506,11 @@ __global__ void __launch_bounds__(256) k_ppm_x(PpmArgs<T> A, T s, T rho, PpmOut<
     if (MODE == 0) {
         const T a = riemann(lo[0], hi[0]);
         O.ad[fc] = a;
-#pragma unroll
-        for (int n = 1; n < NC; ++n) O.TE[n][fc] = upwind(a, lo[n], hi[n]);
+        upwind_n(a, lo, hi, [&](int n, T v) {
+            if (n > 0) O.TE[n][fc] = v;
+        });
     } else {
-#pragma unroll
-        for (int n = 0; n < NC; ++n) O.TE[n][fc] = upwind(u, lo[n], hi[n]);
+        upwind_n(u, lo, hi, [&](int n, T v) { O.TE[n][fc] = v; });
     }
 }
 
@@ -537,23 +605,6 @@ __global__ void __launch_bounds__(128) k_cf_col(Op op, int chunk) {
     }
 }
 
-// Faces a thread of the column kernels marches.  A long march carries more
-// (the cell before a chunk is formed again: about 1.7 faces' work in k_ppm_col,
-// 0.7 in k_cf_col), a short one leaves more warps: an SM sub-partition needs
-// about 3.4 of them in FP64, whose step is a serial chain of 40 to 130 FP64
-// instructions, and twice as many in FP32, which waits on loads.  So the
-// marches are cut to leave 2048 (FP64) or 4096 (FP32) warps, between lo and hi
-// faces.  Measured, k_ppm_col / k_adv_trans_col: 32^3 129 / 69 us at 32 / 16
-// faces, 21 / 12.5 at 2 / 1; 64^3 141 / 84 against 60 / 41 at 4; 96^3 177 / 113
-// against 155 / 113 at 16; FP32 128x128x64 58 / 71 against 37 / 43 at 8; on
-// 256x256x128 32 / 16 are the best.
-template <typename T>
-inline int march_chunk(const Grid& g, int lo, int hi) {
-    const long long rows = 1 + (long long)g.ny * (g.nz + 1) / 32768;  // marches are counted on the second grid dimension
-    const long long m = g.N / (32LL * (sizeof(T) == 4 ? 4096 : 2048));
-    return (int)std::min<long long>(hi, std::max<long long>(std::max<long long>(lo, rows), m));
-}
-
 template <typename Op>
 static void launch_cf(Ctx& c, const char* name_x, const char* name_col, const Op& op, double bytes) {
     const Grid& g = op.g;
@@ -588,11 +639,20 @@ struct PmTransOp {
         c[0] = cb * (ad_b[f1] + ad_b[f0]) * (edge_b[f1] - edge_b[f0]);
     }
     __device__ inline void face(long long f, int kf, bool wl, bool wh, const T cl[1], const T ch[1]) const {
-        T l = lo[f], h = hi[f];
-        if (!wl) l -= cl[0];
-        if (!wh) h -= ch[0];
-        if (d == 2) zbc(g, kf, n, l, h);
-        out[f] = upwind(ad_a[f], l, h);
+        if constexpr (sizeof(T) == 8) {  // one component: both states cost less than the branch
+            T l = lo[f], h = hi[f];
+            if (!wl) l -= cl[0];
+            if (!wh) h -= ch[0];
+            if (d == 2) zbc(g, kf, n, l, h);
+            out[f] = upwind(ad_a[f], l, h);
+        } else {
+            const UpSide s(ad_a[f], wl, wh);
+            const T l = lo[f], h = hi[f];
+            T st;
+            if (s.mean) st = T(0.5) * ((l - cl[0]) + (h - ch[0]));
+            else st = (s.low ? l : h) - (s.low ? cl[0] : ch[0]);
+            out[f] = (wl || wh) && n == 2 ? T(0) : st;
+        }
     }
 };
 
@@ -615,8 +675,7 @@ struct PmFinalOp {
     __device__ inline void cell(int i, int j, int k, T c[1]) const {
         const long long p1 = fidx(g, b1, i + (b1 == 0), j + (b1 == 1), k + (b1 == 2)), m1 = fidx(g, b1, i, j, k);
         const long long p2 = fidx(g, b2, i + (b2 == 0), j + (b2 == 1), k + (b2 == 2)), m2 = fidx(g, b2, i, j, k);
-        const CellFOT<T, T> F{forces, g};
-        T s = hdt * F(d, i, j, k);
+        T s = hdt * forces[d * g.N + cidx(g, i, j, k)];
         s -= c1 * (AD.p[b1][p1] + AD.p[b1][m1]) * (T1[p1] - T1[m1]);
         s -= c2 * (AD.p[b2][p2] + AD.p[b2][m2]) * (T2[p2] - T2[m2]);
         c[0] = s;
@@ -647,27 +706,53 @@ struct AdvTransOp {
         const long long p1 = fidx(g, b1, i + (b1 == 0), j + (b1 == 1), k + (b1 == 2)), m1 = fidx(g, b1, i, j, k);
         const long long p2 = fidx(g, b2, i + (b2 == 0), j + (b2 == 1), k + (b2 == 2)), m2 = fidx(g, b2, i, j, k);
         const T v1p = (T)vb1[p1], v1m = (T)vb1[m1], v2p = (T)vb2[p2], v2m = (T)vb2[m2];
-        const T r1 = rho * cb1 * (v1p - v1m), r2 = rho * cb2 * (v2p - v2m);
-        const VelFPT<T, T> q{vel, g, T(1)};
-        for (int n = 0; n < NC; ++n) {
-            const T qc = q(n, i, j, k);
-            c[n] = qc * r1 - cb1 * (v1p * E1.p[n][p1] - v1m * E1.p[n][m1]);
-            c[NC + n] = qc * r2 - cb2 * (v2p * E2.p[n][p2] - v2m * E2.p[n][m2]);
+        const long long t = cidx(g, i, j, k);
+        if constexpr (sizeof(T) == 8) {
+            const T w1p = cb1 * v1p, w1m = cb1 * v1m, w2p = cb2 * v2p, w2m = cb2 * v2m;
+            const T r1 = rho * (w1p - w1m), r2 = rho * (w2p - w2m);
+            for (int n = 0; n < NC; ++n) {
+                const T qc = vel[n * g.N + t];
+                c[n] = fma(qc, r1, fma(w1m, E1.p[n][m1], -(w1p * E1.p[n][p1])));
+                c[NC + n] = fma(qc, r2, fma(w2m, E2.p[n][m2], -(w2p * E2.p[n][p2])));
+            }
+        } else {
+            const T r1 = rho * cb1 * (v1p - v1m), r2 = rho * cb2 * (v2p - v2m);
+            for (int n = 0; n < NC; ++n) {
+                const T qc = vel[n * g.N + t];
+                c[n] = qc * r1 - cb1 * (v1p * E1.p[n][p1] - v1m * E1.p[n][m1]);
+                c[NC + n] = qc * r2 - cb2 * (v2p * E2.p[n][p2] - v2m * E2.p[n][m2]);
+            }
         }
     }
-    __device__ inline void face(long long f, int kf, bool wl, bool wh, const T cl[K], const T ch[K]) const {
-        const T u = (T)ua[f];
-        const bool usmall = below_small_abs(u), upos = ge0(u);
-        auto pick = [&](T l, T h) { return usmall ? T(0.5) * (l + h) : (upos ? l : h); };
-        for (int n = 0; n < NC; ++n) {
-            const T l0 = LO.p[n][f], h0 = HI.p[n][f];
-            T l = wl ? l0 : l0 + cl[n], h = wh ? h0 : h0 + ch[n];
-            if (d == 2) zbc(g, kf, n, l, h);
-            O1.p[n][f] = pick(l, h);
-            l = wl ? l0 : l0 + cl[NC + n];
-            h = wh ? h0 : h0 + ch[NC + n];
-            if (d == 2) zbc(g, kf, n, l, h);
-            O2.p[n][f] = pick(l, h);
+    __device__ inline void face(long long f, int, bool wl, bool wh, const T cl[K], const T ch[K]) const {
+        const UpSide s((T)ua[f], wl, wh);
+        if constexpr (sizeof(T) == 8) {
+            if (s.mean) {
+                for (int n = 0; n < NC; ++n) {
+                    const T l = LO.p[n][f], h = HI.p[n][f];
+                    O1.p[n][f] = T(0.5) * ((l + cl[n]) + (h + ch[n]));
+                    O2.p[n][f] = T(0.5) * ((l + cl[NC + n]) + (h + ch[NC + n]));
+                }
+                return;
+            }
+            for (int n = 0; n < NC; ++n) {
+                const T q = s.low ? LO.p[n][f] : HI.p[n][f];
+                const bool zero = (wl || wh) && n == 2;
+                O1.p[n][f] = zero ? T(0) : q + (s.low ? cl[n] : ch[n]);
+                O2.p[n][f] = zero ? T(0) : q + (s.low ? cl[NC + n] : ch[NC + n]);
+            }
+        } else {
+            for (int n = 0; n < NC; ++n) {
+                const T l = LO.p[n][f], h = HI.p[n][f], q = s.low ? l : h;
+                T s1 = q + (s.low ? cl[n] : ch[n]), s2 = q + (s.low ? cl[NC + n] : ch[NC + n]);
+                if (s.mean) {
+                    s1 = T(0.5) * ((l + cl[n]) + (h + ch[n]));
+                    s2 = T(0.5) * ((l + cl[NC + n]) + (h + ch[NC + n]));
+                }
+                const bool zero = (wl || wh) && n == 2;
+                O1.p[n][f] = zero ? T(0) : s1;
+                O2.p[n][f] = zero ? T(0) : s2;
+            }
         }
     }
 };
@@ -691,23 +776,44 @@ struct AdvFluxOp {
         const long long p1 = fidx(g, b1, i + (b1 == 0), j + (b1 == 1), k + (b1 == 2)), m1 = fidx(g, b1, i, j, k);
         const long long p2 = fidx(g, b2, i + (b2 == 0), j + (b2 == 1), k + (b2 == 2)), m2 = fidx(g, b2, i, j, k);
         const T v1p = (T)U.p[b1][p1], v1m = (T)U.p[b1][m1], v2p = (T)U.p[b2][p2], v2m = (T)U.p[b2][m2];
-        const T r = rho * (c1 * (v1p - v1m) + c2 * (v2p - v2m));
-        const VelFPT<T, T> q{vel, g, T(1)};
-        const CellFOT<T, T> Fo{forces, g};
-        for (int n = 0; n < NC; ++n) {
-            const T x1 = T1.p[n][p1] * v1p - T1.p[n][m1] * v1m, x2 = T2.p[n][p2] * v2p - T2.p[n][m2] * v2m;
-            c[n] = hdt * Fo(n, i, j, k) + ((q(n, i, j, k) * r - c1 * x1) - c2 * x2);
+        const long long t = cidx(g, i, j, k);
+        if constexpr (sizeof(T) == 8) {
+            const T w1p = c1 * v1p, w1m = c1 * v1m, w2p = c2 * v2p, w2m = c2 * v2m;
+            const T r = rho * ((w1p - w1m) + (w2p - w2m));
+            for (int n = 0; n < NC; ++n) {
+                T x = fma(vel[n * g.N + t], r, hdt * forces[n * g.N + t]);
+                x = fma(-w1p, T1.p[n][p1], x);
+                x = fma(w1m, T1.p[n][m1], x);
+                x = fma(-w2p, T2.p[n][p2], x);
+                c[n] = fma(w2m, T2.p[n][m2], x);
+            }
+        } else {
+            const T r = rho * (c1 * (v1p - v1m) + c2 * (v2p - v2m));
+            for (int n = 0; n < NC; ++n) {
+                const T x1 = T1.p[n][p1] * v1p - T1.p[n][m1] * v1m, x2 = T2.p[n][p2] * v2p - T2.p[n][m2] * v2m;
+                c[n] = hdt * forces[n * g.N + t] + ((vel[n * g.N + t] * r - c1 * x1) - c2 * x2);
+            }
         }
     }
-    __device__ inline void face(long long f, int kf, bool wl, bool wh, const T cl[K], const T ch[K]) const {
+    __device__ inline void face(long long f, int, bool wl, bool wh, const T cl[K], const T ch[K]) const {
         const T um = (T)U.p[d][f];
-        const bool usmall = below_small_abs(um), upos = ge0(um);
-        for (int n = 0; n < NC; ++n) {
-            T stl = wl ? T(0) : LO.p[n][f] + cl[n];
-            T sth = wh ? T(0) : HI.p[n][f] + ch[n];
-            if (d == 2) zbc(g, kf, n, stl, sth);
-            const T st = usmall ? T(0.5) * (stl + sth) : (upos ? stl : sth);
-            Fl.p[n][f] = um * st;
+        const UpSide s(um, wl, wh);
+        if constexpr (sizeof(T) == 8) {
+            if (s.mean) {
+                for (int n = 0; n < NC; ++n) Fl.p[n][f] = um * (T(0.5) * ((LO.p[n][f] + cl[n]) + (HI.p[n][f] + ch[n])));
+                return;
+            }
+            for (int n = 0; n < NC; ++n) {
+                const T st = (s.low ? LO.p[n][f] : HI.p[n][f]) + (s.low ? cl[n] : ch[n]);
+                Fl.p[n][f] = um * ((wl || wh) && n == 2 ? T(0) : st);
+            }
+        } else {
+            for (int n = 0; n < NC; ++n) {
+                const T l = LO.p[n][f], h = HI.p[n][f];
+                T st = (s.low ? l : h) + (s.low ? cl[n] : ch[n]);
+                if (s.mean) st = T(0.5) * ((l + cl[n]) + (h + ch[n]));
+                Fl.p[n][f] = um * ((wl || wh) && n == 2 ? T(0) : st);
+            }
         }
     }
 };
@@ -758,12 +864,12 @@ static void launch_ppm(Ctx& c, const Grid& g, int d, const T* vel, const T* umac
 }
 
 template <typename T>
-static void premac_t(Ctx& c, const Grid& g, const T* vel, const T* forces, double dt, GodunovBufs& B, double* mac[3]) {
+static void premac_t(Ctx& c, const Grid& g, const T* vel, const T* forces, double dt, GodunovBufs& B, double* mac[3], int edges) {
     const double BT = (double)sizeof(T), B8 = 8.0;
     for (int d = 0; d < 3; ++d) {
         PpmOut<T, 3> O{};
         for (int n = 0; n < 3; ++n) {
-            O.E[n] = tp<T>(B.edge[d][n]);
+            O.E[n] = edges ? tp<T>(B.edge[d][n]) : nullptr;
             O.PM[n] = tp<T>(B.pm[d][n]);
             O.PP[n] = tp<T>(B.pp[d][n]);
             O.LO[n] = tp<T>(B.lo[d][n]);
@@ -771,7 +877,7 @@ static void premac_t(Ctx& c, const Grid& g, const T* vel, const T* forces, doubl
             O.TE[n] = tp<T>(B.tedge[d][n]);
         }
         O.ad = tp<T>(B.ad[d]);
-        launch_ppm<T, 3, 0, 1>(c, g, d, vel, (const T*)nullptr, dt, 1.0, O, BT * 3.0 * g.N + BT * 12.0 * nfaces(g, d));
+        launch_ppm<T, 3, 0, 1>(c, g, d, vel, (const T*)nullptr, dt, 1.0, O, BT * 9.0 * g.N + BT * (9.0 + 3.0 * edges) * nfaces(g, d));
     }
     // (a, b, n): states on a-faces of component n corrected along b
     const int tpl[6][3] = {{1, 2, 0}, {2, 1, 0}, {0, 2, 1}, {2, 0, 1}, {0, 1, 2}, {1, 0, 2}};
@@ -894,13 +1000,13 @@ static void to_single(Ctx& c, const double* a, float* b, long long n) {
 }
 
 void launch_premac(Ctx& c, const Grid& g, const double* vel, const double* forces, double dt, GodunovBufs& B, double* mac[3], int fp32,
-                   GodunovIn32* in32) {
+                   GodunovIn32* in32, int edges) {
     if (fp32) {
         to_single(c, vel, in32->vel, 3 * g.N);
         to_single(c, forces, in32->forces, 3 * g.N);
-        premac_t<float>(c, g, in32->vel, in32->forces, dt, B, mac);
+        premac_t<float>(c, g, in32->vel, in32->forces, dt, B, mac, edges);
     } else {
-        premac_t<double>(c, g, vel, forces, dt, B, mac);
+        premac_t<double>(c, g, vel, forces, dt, B, mac, edges);
     }
 }
 

@@ -1652,8 +1652,6 @@ void Sim::apply_predictor(bool incremental) {
     launch_smagorinsky(ctx_, g_, vel_old_.p, mueff_.p, S_, alpha_.p, mixed_);
     sources(vel_old_.p, theta_old_.p);  // BoussinesqBuoyancy: theta at Old
     if (wallmodel_) launch_wall_grad(ctx_, g_, vel_old_.p, mueff_.p, wg_.p, shear_, utau_ * utau_, um_[0], um_[1], vmag_, rho_);
-    double* fl[9];
-    for (int m = 0; m < 9; ++m) fl[m] = static_cast<double*>(gb_.flux[m / 3][m % 3]);
     launch_divtau(ctx_, g_, vel_old_.p, mueff_.p, wg_.p, divtau_.p, 1, src_.p, forces_.p, nullptr, nullptr, dt, rho_, mixed_);
     if (temp_) {  // the temperature's diff_term(Old) (no temperature sources)
         if (tzlo_ == 1)
@@ -1662,7 +1660,7 @@ void Sim::apply_predictor(bool incremental) {
         launch_tdiff(ctx_, g_, theta_old_.p, alpha_.p, tbc(), tdiff_.p, 0, nullptr, nullptr, nullptr, nullptr, nullptr, dt, rho_, 0.0);
     }
     double* mac[3] = {umac_[0].p, umac_[1].p, umac_[2].p};
-    launch_premac(ctx_, g_, vel_old_.p, forces_.p, dt, gb_, mac, mixed_, mixed_ ? &in32_ : nullptr);
+    launch_premac(ctx_, g_, vel_old_.p, forces_.p, dt, gb_, mac, mixed_, mixed_ ? &in32_ : nullptr, adj_ ? 1 : 0);
     mac_project();
     if (temp_) temperature_predictor(dt);
     const double* cmac[3] = {umac_[0].p, umac_[1].p, umac_[2].p};

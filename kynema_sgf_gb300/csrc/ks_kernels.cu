@@ -147,6 +147,56 @@ __global__ void k_smag(Grid g, const double* vel, double* mueff, double mu, doub
     if (alpha) alpha[t] = mu_pr + iprt * mut;
 }
 
+// FP64 form: columns marched in z, the column's own values carried and the
+// neighbour offsets formed once, as the FP64 issue of about 27 instructions and
+// a square root (7.5 more) should bound it, not the index maps of the 18 reads
+// of the thread-per-cell form (256x256x128: 1400 us, 575 now).
+__global__ void __launch_bounds__(128) k_smag_col(Grid g, const double* vel, double* mueff, double mu, double rhofac, double* alpha, double mu_pr,
+                                                  double iprt, int kc) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+    if (i >= g.nx) return;
+    const int k0 = blockIdx.z * kc, k1 = min(k0 + kc, g.nz);
+    const long long N = g.N;
+    const int sz = g.nx * g.ny;
+    const int xp = i + 1 == g.nx ? 1 - g.nx : 1, xm = i == 0 ? g.nx - 1 : -1;
+    const int yp = (j + 1 == g.ny ? 1 - g.ny : 1) * g.nx, ym = (j == 0 ? g.ny - 1 : -1) * g.nx;
+    const VelFPT<double, double> V{vel, g, 1.0};
+    const double hx = 0.5 * g.idx, hy = 0.5 * g.idy, hz = 0.5 * g.idz;
+    const double* p = vel + (long long)k0 * sz + j * g.nx + i;
+    double dn[3], at[3];
+    for (int n = 0; n < 3; ++n) {
+        dn[n] = V(n, i, j, k0 - 1);
+        at[n] = p[n * N];
+    }
+    for (int k = k0; k < k1; ++k, p += sz) {
+        double up[3], gz[3], sxy, syz, szx;
+        for (int n = 0; n < 3; ++n) up[n] = k + 1 < g.nz ? p[n * N + sz] : V(n, i, j, k + 1);
+        const double ux = hx * (p[xp] - p[xm]), vy = hy * (p[N + yp] - p[N + ym]);
+        sxy = hy * (p[yp] - p[ym]) + hx * (p[N + xp] - p[N + xm]);
+        const double wx = p[2 * N + xp] - p[2 * N + xm], wy = p[2 * N + yp] - p[2 * N + ym];
+        if (!g.zper && (k == 0 || k == g.nz - 1)) {  // one-sided through the wall (ghost) value
+            double a = 1.0 / 3.0, b = 1.0, c = -4.0 / 3.0;
+            if (k == g.nz - 1) { a = 4.0 / 3.0; b = -1.0; c = -1.0 / 3.0; }
+            for (int n = 0; n < 3; ++n) gz[n] = (a * up[n] + b * at[n] + c * dn[n]) * g.idz;
+            syz = gz[1] + hy * wy;
+            szx = hx * wx + gz[0];
+        } else {
+            syz = hz * (up[1] - dn[1]) + hy * wy;
+            szx = hx * wx + hz * (up[0] - dn[0]);
+            gz[2] = hz * (up[2] - dn[2]);
+        }
+        const double s = sqrt(2.0 * (ux * ux + vy * vy + gz[2] * gz[2]) + (sxy * sxy + syz * syz + szx * szx));
+        const double mut = rhofac * s;
+        const long long t = ((long long)k * g.ny + j) * g.nx + i;
+        mueff[t] = mu + mut;
+        if (alpha) alpha[t] = mu_pr + iprt * mut;
+        for (int n = 0; n < 3; ++n) {
+            dn[n] = at[n];
+            at[n] = up[n];
+        }
+    }
+}
+
 // Mixed-precision form: the same FP32 strain rate from a shared-memory tile of
 // 32 x 4 x 4 cells whose one-cell halo (fill-patch ghosts included) is staged
 // once, so each velocity value is loaded and rounded about 2.4 times per cell
@@ -214,21 +264,24 @@ struct SrcCoef {
     double c[3];
     double M[3][3];
     double rho, bous_g[3], T_ref;
-    int cor, act, bous;
 };
+// Which terms run is a template argument: as a run-time flag each absent term
+// still took its FP64 issue slots, predicated off (22 for 12 a cell: 351 us on
+// 256x256x128, 247 now).
+template <int COR, int ACT, int BOUS>
 __global__ void k_sources(Grid g, const double* vel, const double* gp, const double* act, double* src, SrcCoef s, const double* theta) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= g.N) return;
     const long long N = g.N;
     double f[3];
     for (int n = 0; n < 3; ++n) f[n] = s.c[n] - gp[n * N + t];
-    if (s.cor) {
+    if (COR) {
         const double u0 = vel[t], u1 = vel[N + t], u2 = vel[2 * N + t];
         for (int n = 0; n < 3; ++n) f[n] += s.M[n][0] * u0 + s.M[n][1] * u1 + s.M[n][2] * u2;
     }
-    if (s.act)
+    if (ACT)
         for (int n = 0; n < 3; ++n) f[n] += s.rho * act[n * N + t];
-    if (s.bous) {  // BoussinesqBuoyancy.cpp:22-50: rho g beta (T0 - theta)
+    if (BOUS) {  // BoussinesqBuoyancy.cpp:22-50: rho g beta (T0 - theta)
         const double dT = s.T_ref - theta[t];
         for (int n = 0; n < 3; ++n) f[n] += s.bous_g[n] * dT;
     }
@@ -542,8 +595,7 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
 // columns; one each for the row below and above (the cell differences the y
 // faces need, and the upper row's faces); one for the columns left (lanes 0 ..)
 // and right (lanes 16 ..) of the block.
-// On 256x256x128: 2.25 ms as tiles (96 % of the FP64 issue rate), 1.56 ms now
-// (89 %); 96^3 284 -> 178 us.
+// On 256x256x128: 2.25 ms as tiles (96 % of the FP64 issue rate), 1.50 ms now.
 template <int TY>
 struct TauPlanes {
     double V[3][3][TY + 2][34];   // [layer mod 3][component]: row and column 0 are the halo
@@ -564,7 +616,9 @@ inline TauCoef tau_coef(const Grid& g) {
                    0.25 * z / x,        0.25 * z / y,        -0.125 * x / y,      -0.125 * y / x, -0.125 * z / x, y / z, x / z, x / y};
 }
 
-template <int TY>
+// MODE (TauEpi) is a template argument: the other modes' instructions, predicated
+// off, took 7 of 92 FP64 issue slots a cell.
+template <int TY, int MODE>
 __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef K, const double* vel, const double* mueff, const double* wg, double* out,
                                                              TauEpi E, int kc) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
@@ -588,7 +642,7 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
         for (int n = 0; n < 3; ++n) c.v[n] = p[n * N];
         c.m = mueff[(long long)kk * sz + col];
         if (!g.zper && (k < 0 || k >= g.nz)) {
-            c.v[2] = bitsd(dbits(c.v[2]) ^ ~kMag);
+            c.v[2] = ineg(c.v[2]);
             if (k < 0 && g.zlo == ZWALLMODEL)
                 for (int n = 0; n < 2; ++n) c.v[n] -= wg[(long long)n * sz + col] * g.dz;
         }
@@ -672,7 +726,7 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
     const bool live = mainw && i < g.nx && j < g.ny;
     const int sr = l & 15, sx = l < 16 ? 0 : 33;  // the side warp's row and column
     const bool side = w == TY + 2 && sr < TY;
-    const double rho = E.rho, dt = E.dt, irho = E.irho;
+    const double hdr = 0.5 * E.dt * E.irho;
     long long rmax = 0;
     for (int k = k0; k < k1; ++k) {
         const int m = k & 1;
@@ -724,19 +778,19 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
             for (int n = 0; n < 3; ++n) {
                 const double acc = ((S.FX[n][w][l + 1] - fx[n]) + (S.FY[n][w + 1][l] - fy[n])) + (fzn[n] - fz[n]);
                 const long long o = n * N + t;
-                if (E.mode == 0) {
+                if constexpr (MODE == 0) {
                     out[o] = acc;
-                } else if (E.mode == 1) {
+                } else if constexpr (MODE == 1) {
                     out[o] = acc;
-                    E.forces[o] = (E.src[o] + acc) * irho;
-                } else if (E.mode == 2) {
-                    out[o] = E.base[o] + 0.5 * dt * (acc - E.dold[o]) * irho;
-                } else if (E.mode == 3) {
-                    out[o] = (rho * E.base[o] + dt * (0.5 * (E.conv_o[o] + E.conv_n[o]) + 0.5 * E.dold[o] + 0.5 * acc + E.src[o])) * irho;
+                    E.forces[o] = (E.src[o] + acc) * E.irho;
+                } else if constexpr (MODE == 2) {
+                    out[o] = E.base[o] + hdr * (acc - E.dold[o]);
+                } else if constexpr (MODE == 3) {
+                    out[o] = (E.rho * E.base[o] + E.dt * (0.5 * (E.conv_o[o] + E.conv_n[o]) + 0.5 * E.dold[o] + 0.5 * acc + E.src[o])) * E.irho;
                 } else {
-                    const double r = E.base[o] - rho * pc.v[n] + dt * acc;
+                    const double r = E.base[o] - E.rho * pc.v[n] + E.dt * acc;
                     rmax = imax_abs(rmax, r);
-                    out[o] = E.mode == 7 ? pc.v[n] + E.omega * E.dinv[o] * r : r;
+                    out[o] = MODE == 7 ? pc.v[n] + E.omega * E.dinv[o] * r : r;
                 }
             }
         }
@@ -751,17 +805,19 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
         sp = s;
         __syncthreads();
     }
-    if (!E.parts) return;  // uniform over the block
-    for (int o = 16; o > 0; o >>= 1) {
-        const long long b = __shfl_xor_sync(0xffffffffu, rmax, o);
-        rmax = b > rmax ? b : rmax;
-    }
-    __shared__ long long wmax[TY];
-    if (mainw && l == 0) wmax[w] = rmax;
-    __syncthreads();
-    if (tid == 0) {
-        for (int r = 0; r < TY; ++r) rmax = wmax[r] > rmax ? wmax[r] : rmax;
-        E.parts[(blockIdx.z * (long long)gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = bitsd(rmax);
+    if constexpr (MODE >= 7) {
+        if (!E.parts) return;  // uniform over the block
+        for (int o = 16; o > 0; o >>= 1) {
+            const long long b = __shfl_xor_sync(0xffffffffu, rmax, o);
+            rmax = b > rmax ? b : rmax;
+        }
+        __shared__ long long wmax[TY];
+        if (mainw && l == 0) wmax[w] = rmax;
+        __syncthreads();
+        if (tid == 0) {
+            for (int r = 0; r < TY; ++r) rmax = wmax[r] > rmax ? wmax[r] : rmax;
+            E.parts[(blockIdx.z * (long long)gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = bitsd(rmax);
+        }
     }
 }
 
@@ -796,11 +852,11 @@ inline TauShape tau_shape(const Grid& g) {
 
 // predictor_rhs (src/equation_systems/CompRHSOps.H:32-141); fac = 1 explicit,
 // 1/2 Crank-Nicolson, 0 implicit
-__global__ void k_pred_rhs(long long N3, const double* vo, const double* conv, const double* src, const double* dt_, double* vel, double dt,
-                           double rho, double irho, double fac) {
+__global__ void k_pred_rhs(long long N3, const double* vo, const double* conv, const double* src, const double* dt_, double* vel, double dtr,
+                           double fac) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= N3) return;
-    vel[t] = (rho * vo[t] + dt * (conv[t] + src[t] + fac * dt_[t])) * irho;
+    vel[t] = vo[t] + dtr * ((conv[t] + src[t]) + fac * dt_[t]);  // dtr = dt / rho, formed on the host
 }
 
 // ---------------------------------------------------------------- projection
@@ -1006,16 +1062,16 @@ __global__ void k_mac_divmax(Grid g, const double* um, const double* vm, const d
     if (threadIdx.x == 0) { parts[blockIdx.x] = a; parts[np + blockIdx.x] = b; }
 }
 
-__global__ void k_mac_correct(Grid g, const double* phi, double* um, double* vm, double* wm, double beta) {
+// bx = beta / dx, ...
+__global__ void k_mac_correct(Grid g, const double* phi, double* um, double* vm, double* wm, double bx, double by, double bz) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= g.N) return;
     int i, j, k;
     cell_of(g, t, i, j, k);
     const double p0 = phi[t];
-    um[t] -= beta * (p0 - phi[cidx(g, wrapn(i - 1, g.nx), j, k)]) * g.idx;
-    vm[t] -= beta * (p0 - phi[cidx(g, i, wrapn(j - 1, g.ny), k)]) * g.idy;
-    if (g.zper) wm[t] -= beta * (p0 - phi[cidx(g, i, j, wrapn(k - 1, g.nz))]) * g.idz;
-    else if (k > 0) wm[t] -= beta * (p0 - phi[cidx(g, i, j, k - 1)]) * g.idz;
+    um[t] -= bx * (p0 - phi[cidx(g, wrapn(i - 1, g.nx), j, k)]);
+    vm[t] -= by * (p0 - phi[cidx(g, i, wrapn(j - 1, g.ny), k)]);
+    if (g.zper || k > 0) wm[t] -= bz * (p0 - phi[cidx(g, i, j, k == 0 ? g.nz - 1 : k - 1)]);
 }
 
 // ---------------------------------------------------------------- reductions
@@ -1212,7 +1268,12 @@ void launch_smagorinsky(Ctx& c, const Grid& g, const double* vel, double* mueff,
         KS_LAUNCH(c, k_smag_tile, grid, SMX * SMY * SMZ, bytes, g, vel, mueff, s.mu, s.rho, s.smag_fac, alpha, s.mu_pr, s.iprt);
     } else if (fp32)
         KS_LAUNCH(c, k_smag<float>, nblocks(g.N, BS), BS, bytes, g, vel, mueff, s.mu, s.rho, s.smag_fac, s.smag, alpha, s.mu_pr, s.iprt);
-    else
+    else if (s.smag) {
+        // layers a march: 16, fewer where that leaves less than 2048 warps
+        const int kc = (int)std::min<long long>(16, std::max<long long>(1, g.N / 65536));
+        const dim3 grid((unsigned)((g.nx + 127) / 128), (unsigned)g.ny, (unsigned)((g.nz + kc - 1) / kc));
+        KS_LAUNCH(c, k_smag_col, grid, std::min(128, 32 * ((g.nx + 31) / 32)), bytes, g, vel, mueff, s.mu, s.rho * s.smag_fac, alpha, s.mu_pr, s.iprt, kc);
+    } else
         KS_LAUNCH(c, k_smag<double>, nblocks(g.N, BS), BS, bytes, g, vel, mueff, s.mu, s.rho, s.smag_fac, s.smag, alpha, s.mu_pr, s.iprt);
 }
 // src = rho (-gp/rho + geostrophic + Coriolis(u_old) + body + actuator + Boussinesq + ABLForcing)
@@ -1225,9 +1286,6 @@ void launch_sources(Ctx& c, const Grid& g, const double* vel_old, const double* 
                     const double* theta) {
     SrcCoef k{};
     k.rho = s.rho;
-    k.cor = s.cor;
-    k.act = s.act;
-    k.bous = s.bous;
     k.T_ref = s.T_ref;
     for (int n = 0; n < 3; ++n) {
         double a = 0.0;
@@ -1240,7 +1298,11 @@ void launch_sources(Ctx& c, const Grid& g, const double* vel_old, const double* 
             k.M[n][m] = s.rho * s.corfac *
                         (s.sinphi * (s.east[n] * s.north[m] - s.north[n] * s.east[m]) + s.hfac * s.cosphi * (s.up[n] * s.east[m] - s.east[n] * s.up[m]));
     }
-    KS_LAUNCH(c, k_sources, nblocks(g.N, BS), BS, B8 * (6 + 3 * s.cor + 3 * s.act + s.bous) * g.N, g, vel_old, gp, act, src, k, theta);
+    using Kern = void (*)(Grid, const double*, const double*, const double*, double*, SrcCoef, const double*);
+    static const Kern kern[8] = {k_sources<0, 0, 0>, k_sources<1, 0, 0>, k_sources<0, 1, 0>, k_sources<1, 1, 0>,
+                                 k_sources<0, 0, 1>, k_sources<1, 0, 1>, k_sources<0, 1, 1>, k_sources<1, 1, 1>};
+    const Kern run = kern[(s.cor ? 1 : 0) + (s.act ? 2 : 0) + (s.bous ? 4 : 0)];
+    KS_LAUNCH_NAMED(c, "k_sources", run, nblocks(g.N, BS), BS, B8 * (6 + 3 * s.cor + 3 * s.act + s.bous) * g.N, g, vel_old, gp, act, src, k, theta);
 }
 void launch_plane_sums(Ctx& c, const Grid& g, const double* vel, double* parts, int* np) {
     *np = parts_for((long long)g.nx * g.ny);
@@ -1265,15 +1327,29 @@ void launch_divtau_faces(Ctx& c, const Grid& g, const double* vel, const double*
     KS_LAUNCH(c, k_tau_div, nblocks(g.N, BS), BS, B8 * per_cell * g.N, g, F, out, mode, src, forces, base, dold, dt, rho);
 }
 
-static void launch_divtau_col(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, const TauEpi& E,
-                              double bytes) {
+template <int MODE>
+static void launch_divtau_mode(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, const TauEpi& E,
+                               double bytes) {
     const TauShape s = tau_shape(g);
     const TauCoef K = tau_coef(g);
+    const auto k4 = k_divtau_col<4, MODE>;
+    const auto k8 = k_divtau_col<8, MODE>;
     if (s.ty == 4) {
-        KS_LAUNCH_SMEM(c, k_divtau_col<4>, s.grid, 32 * 7, sizeof(TauPlanes<4>), bytes, g, K, vel, mueff, wg, out, E, s.kc);
+        KS_LAUNCH_SMEM_NAMED(c, "k_divtau_col", k4, s.grid, 32 * 7, sizeof(TauPlanes<4>), bytes, g, K, vel, mueff, wg, out, E, s.kc);
     } else {
-        cudaFuncSetAttribute(k_divtau_col<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TauPlanes<8>));
-        KS_LAUNCH_SMEM(c, k_divtau_col<8>, s.grid, 32 * 11, sizeof(TauPlanes<8>), bytes, g, K, vel, mueff, wg, out, E, s.kc);
+        cudaFuncSetAttribute(k8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TauPlanes<8>));
+        KS_LAUNCH_SMEM_NAMED(c, "k_divtau_col", k8, s.grid, 32 * 11, sizeof(TauPlanes<8>), bytes, g, K, vel, mueff, wg, out, E, s.kc);
+    }
+}
+static void launch_divtau_col(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, const TauEpi& E,
+                              double bytes) {
+    switch (E.mode) {
+        case 0: launch_divtau_mode<0>(c, g, vel, mueff, wg, out, E, bytes); break;
+        case 1: launch_divtau_mode<1>(c, g, vel, mueff, wg, out, E, bytes); break;
+        case 2: launch_divtau_mode<2>(c, g, vel, mueff, wg, out, E, bytes); break;
+        case 3: launch_divtau_mode<3>(c, g, vel, mueff, wg, out, E, bytes); break;
+        case 7: launch_divtau_mode<7>(c, g, vel, mueff, wg, out, E, bytes); break;
+        default: launch_divtau_mode<8>(c, g, vel, mueff, wg, out, E, bytes); break;
     }
 }
 static_assert(sizeof(TauPlanes<4>) <= 48 * 1024, "needs no shared memory attribute");
@@ -1304,7 +1380,7 @@ void launch_divtau_jacobi(Ctx& c, const Grid& g, const double* x, const double* 
 }
 void launch_predictor_rhs(Ctx& c, const Grid& g, const double* vo, const double* conv, const double* src, const double* dtau, double* vel,
                           double dt, double rho, double fac) {
-    KS_LAUNCH(c, k_pred_rhs, nblocks(3 * g.N, BS), BS, B8 * 15 * g.N, 3 * g.N, vo, conv, src, dtau, vel, dt, rho, 1.0 / rho, fac);
+    KS_LAUNCH(c, k_pred_rhs, nblocks(3 * g.N, BS), BS, B8 * 15 * g.N, 3 * g.N, vo, conv, src, dtau, vel, dt / rho, fac);
 }
 void launch_proj_pre(Ctx& c, const Grid& g, double* vel, const double* vo, const double* gp, double scaling, double rho, int add_gp,
                      int sub_old) {
@@ -1340,7 +1416,7 @@ void launch_mac_divmax(Ctx& c, const Grid& g, const double* um, const double* vm
     KS_LAUNCH(c, k_mac_divmax, *np, BS, B8 * (2 * g.N + g.NFz), g, um, vm, wm, parts, *np);
 }
 void launch_mac_correct(Ctx& c, const Grid& g, const double* phi, double* um, double* vm, double* wm, double beta) {
-    KS_LAUNCH(c, k_mac_correct, nblocks(g.N, BS), BS, B8 * 7 * g.N, g, phi, um, vm, wm, beta);
+    KS_LAUNCH(c, k_mac_correct, nblocks(g.N, BS), BS, B8 * 7 * g.N, g, phi, um, vm, wm, beta * g.idx, beta * g.idy, beta * g.idz);
 }
 void launch_cfl(Ctx& c, const Grid& g, const double* vel, const double* src, const double* mu, double rho, double* parts, int* np) {
     *np = parts_for(g.N);

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <map>
 #include <string>
@@ -107,14 +108,32 @@ struct Ctx {
     } while (0)
 
 // the same with dynamic shared memory
-#define KS_LAUNCH_SMEM(c, kern, grid, block, smem, bytes, ...)        \
-    do {                                                               \
-        const bool ks_p_ = (c).prof_match(#kern);                      \
-        if (ks_p_) (c).prof_begin(#kern, (double)(bytes));             \
-        kern<<<(grid), (block), (smem), (c).stream>>>(__VA_ARGS__);    \
-        if (ks_p_) (c).prof_end();                                     \
-        ++(c).launches;                                                \
+#define KS_LAUNCH_SMEM_NAMED(c, name, kern, grid, block, smem, bytes, ...) \
+    do {                                                                    \
+        const bool ks_p_ = (c).prof_match(name);                            \
+        if (ks_p_) (c).prof_begin(name, (double)(bytes));                   \
+        kern<<<(grid), (block), (smem), (c).stream>>>(__VA_ARGS__);         \
+        if (ks_p_) (c).prof_end();                                          \
+        ++(c).launches;                                                     \
     } while (0)
+#define KS_LAUNCH_SMEM(c, kern, grid, block, smem, bytes, ...) KS_LAUNCH_SMEM_NAMED(c, #kern, kern, grid, block, smem, bytes, __VA_ARGS__)
+
+// Faces a thread of the column kernels marches.  A long march carries more
+// (the cell before a chunk is formed again: about 1.7 faces' work in k_ppm_col,
+// 0.7 in k_cf_col), a short one leaves more warps: an SM sub-partition needs
+// about 3.4 of them in FP64, whose step is a serial chain of 40 to 130 FP64
+// instructions, and twice as many in FP32, which waits on loads.  So the
+// marches are cut to leave 2048 (FP64) or 4096 (FP32) warps, between lo and hi
+// faces.  Measured, k_ppm_col / k_adv_trans_col: 32^3 129 / 69 us at 32 / 16
+// faces, 21 / 12.5 at 2 / 1; 64^3 141 / 84 against 60 / 41 at 4; 96^3 177 / 113
+// against 155 / 113 at 16; FP32 128x128x64 58 / 71 against 37 / 43 at 8; on
+// 256x256x128 32 / 16 are the best.
+template <typename T>
+inline int march_chunk(const Grid& g, int lo, int hi) {
+    const long long rows = 1 + (long long)g.ny * (g.nz + 1) / 32768;  // marches are counted on the second grid dimension
+    const long long m = g.N / (32LL * (sizeof(T) == 4 ? 4096 : 2048));
+    return (int)std::min<long long>(hi, std::max<long long>(std::max<long long>(lo, rows), m));
+}
 
 struct Scalars {  // values fed to the pointwise kernels
     double rho, irho, mu, smag_fac;
@@ -233,8 +252,9 @@ struct GodunovIn32 {
     float* forces;  // 3 N
     float* mac[3];  // face arrays
 };
+// edges: also store the unlimited PPM edges (a reverse step reads them)
 void launch_premac(Ctx& c, const Grid& g, const double* vel_old, const double* forces, double dt, GodunovBufs& B, double* mac[3],
-                   int fp32, GodunovIn32* in32);
+                   int fp32, GodunovIn32* in32, int edges);
 void launch_advection(Ctx& c, const Grid& g, const double* vel_old, const double* forces, const double* mac[3], double dt, double rho,
                       GodunovBufs& B, double* conv, int fp32, GodunovIn32* in32);
 // Godunov fluxes and conv = -div(flux) of rho s for a cell scalar s with forces fs = src + diff (FP64);

@@ -182,10 +182,19 @@ __global__ void k_cc_gsrb(CCLevelT<T> L, CCCoef<T> w, int color, int kc) {
 // stencil.  A thread then owns the cell pair (2 i2, 2 i2 + 1) of a row, as in
 // k_cc_gsrb, so that every lane of a warp evaluates the same colour (half the
 // FP64 work); zc = -1: every cell is evaluated.
-template <typename T>
+// TO32: the destination r32, z32.  (As a run-time choice its conversion took an
+// FP64 issue slot of every cell, predicated off, as did the other branch of the
+// z neighbours' sum: 182 us a residual on 256x256x128, 163 now.)
+template <typename T, int TO32>
 __global__ void k_cc_resid(CCLevelT<T> L, CCCoef<T> w, int kc, double* parts, float* r32, float* z32, int zc) {
     const int sy = L.nx, sz = L.nx * L.ny;
     const int nch = (L.nz + kc - 1) / kc;
+    // the sum of a cell's z neighbours (a Neumann wall's is dropped)
+    auto zsum = [&](const T* p, int c, int k) {
+        const int up = k + 1 == L.nz ? (1 - L.nz) * sz : sz, dn = k == 0 ? (L.nz - 1) * sz : -sz;
+        const T a = L.zper || k > 0 ? p[c + dn] : T(0), b = L.zper || k + 1 < L.nz ? p[c + up] : T(0);
+        return a + b;
+    };
     if (zc >= 0) {
         const int hx = L.nx >> 1;
         const unsigned M2 = (unsigned)(hx * L.ny * nch);
@@ -202,13 +211,7 @@ __global__ void k_cc_resid(CCLevelT<T> L, CCCoef<T> w, int kc, double* parts, fl
                 const int dxp = i + 1 == L.nx ? 1 - L.nx : 1, dxm = i == 0 ? L.nx - 1 : -1;
                 const T sx = p[c + dxp] + p[c + dxm];
                 const T syv = p[c + dyp] + p[c + dym];
-                T szv;
-                if (L.zper) {
-                    const int kp = k + 1 == L.nz ? 0 : k + 1, km = k == 0 ? L.nz - 1 : k - 1;
-                    szv = p[c + (kp - k) * sz] + p[c + (km - k) * sz];
-                } else {
-                    szv = (k == 0 ? T(0) : p[c - sz]) + (k + 1 == L.nz ? T(0) : p[c + sz]);
-                }
+                const T szv = zsum(p, c, k);
                 T gx = w.gx0, gy = w.gy0, gz = w.gz0, dg = w.dg0;
                 if (!L.zper && (k == 0 || k + 1 == L.nz)) {
                     const bool one = L.nz == 1;
@@ -248,12 +251,7 @@ __global__ void k_cc_resid(CCLevelT<T> L, CCCoef<T> w, int kc, double* parts, fl
             u.pc = p[c];
             u.sx = p[c + dxp] + p[c + dxm];
             u.sy = p[c + dyp] + p[c + dym];
-            if (L.zper) {
-                const int kp = k + 1 == L.nz ? 0 : k + 1, km = k == 0 ? L.nz - 1 : k - 1;
-                u.sz = p[c + (kp - k) * sz] + p[c + (km - k) * sz];
-            } else {
-                u.sz = (k == 0 ? T(0) : p[c - sz]) + (k + 1 == L.nz ? T(0) : p[c + sz]);
-            }
+            u.sz = zsum(p, c, k);
             return u;
         };
         Ld cur = fetch(k0);
@@ -272,7 +270,7 @@ __global__ void k_cc_resid(CCLevelT<T> L, CCCoef<T> w, int kc, double* parts, fl
             const T S = gx * cur.sx + gy * cur.sy + gz * cur.sz;
             const T v = cur.r - dg * (cur.pc - S);
             cur = nxt;
-            if (r32) {
+            if constexpr (TO32) {
                 r32[c] = (float)v;
                 z32[c] = 0.0f;
             } else {
@@ -467,8 +465,11 @@ inline NdCoef<T> nd_coef(const NDLevelT<T>& L, double sigma, double omega) {
 // about half the FP64 operations of the node-by-node sums; the residual is
 // one FMA chain from rhs with the sigma-scaled weights.
 // MODE 0: out = in + omega (rhs - A in) / diag.  MODE 1: the same plus block
-// maxima of |rhs - A in|.  MODE 2: res = rhs - A phi plus block maxima.
-template <typename T, int MODE>
+// maxima of |rhs - A in|.  MODE 2: res = rhs - A phi plus block maxima.  MODE 3:
+// MODE 2 to the FP32 cycle's right-hand side r32.  FZ: the face weights are zero
+// (equal spacings).  Both are template arguments because a term that is
+// predicated off takes its FP64 issue slots all the same: five of 19 a node.
+template <typename T, int MODE, int FZ>
 __global__ void k_nd_col(NDLevelT<T> L, NdCoef<T> w, const T* in, T* out, int kc, double* parts, float* r32 = nullptr,
                          float* z32 = nullptr) {
     const int sz = L.nx * L.ny;
@@ -504,18 +505,16 @@ __global__ void k_nd_col(NDLevelT<T> L, NdCoef<T> w, const T* in, T* out, int kc
             res = w.c3 * (Exm + Exp) + res;
             res = w.c1 * (Eym + Eyp) + res;
             res = w.c0 * (Pm + Pp) + res;
-            if (!L.faces_zero) {
+            if constexpr (!FZ) {
                 res = w.c12 * Ex0 + res;
                 res = w.c10 * Ey0 + res;
                 res = w.c4 * (Cm + Cp) + res;
             }
-            if (MODE == 2) {
-                if (r32) {  // residual to the FP32 cycle's right-hand side (as in k_cc_resid)
-                    r32[idx] = (float)res;
-                    z32[idx] = 0.0f;
-                } else {
-                    L.res[idx] = res;
-                }
+            if constexpr (MODE == 3) {
+                r32[idx] = (float)res;
+                z32[idx] = 0.0f;
+            } else if constexpr (MODE == 2) {
+                L.res[idx] = res;
             } else {
                 out[idx] = w.oinv * res + C0;
             }
@@ -1067,21 +1066,22 @@ void launch_cc_resid(Ctx& c, const CCLevelT<T>& L, double beta, double* parts, i
     if (L.nx % 2) zero_color = -1;  // the pair form needs an even row
     const int n = parts_for((long long)(zero_color >= 0 ? L.nx / 2 : L.nx) * L.ny * ((L.nz + kc - 1) / kc));
     if (np) *np = n;
-    KS_LAUNCH(c, k_cc_resid<T>, n, BS, sizeof(T) * 3.0 * ncc(L), L, cc_coef(L), kc, parts, (float*)nullptr, (float*)nullptr, zero_color);
+    KS_LAUNCH_NAMED(c, "k_cc_resid<T>", (k_cc_resid<T, 0>), n, BS, sizeof(T) * 3.0 * ncc(L), L, cc_coef(L), kc, parts, (float*)nullptr, (float*)nullptr, zero_color);
 }
 void launch_cc_resid32(Ctx& c, const CCLevelT<double>& L, double beta, float* r32, float* z32, double* parts, int* np) {
     (void)beta;
     const int kc = cc_chunk(L);
     const int n = parts_for((long long)L.nx * L.ny * ((L.nz + kc - 1) / kc));
     *np = n;
-    KS_LAUNCH(c, k_cc_resid<double>, n, BS, 8.0 * 2.0 * ncc(L) + 8.0 * ncc(L), L, cc_coef(L), kc, parts, r32, z32, -1);
+    KS_LAUNCH_NAMED(c, "k_cc_resid<double>", (k_cc_resid<double, 1>), n, BS, 8.0 * 2.0 * ncc(L) + 8.0 * ncc(L), L, cc_coef(L), kc, parts, r32, z32, -1);
 }
 void launch_nd_resid32(Ctx& c, const NDLevelT<double>& L, double sigma, float* r32, float* z32, double* parts, int* np) {
     const int kc = nd_chunk(L);
     const int n = parts_for(nd_cols(L, kc));
     *np = n;
-    KS_LAUNCH(c, (k_nd_col<double, 2>), n, BS, 8.0 * 2.0 * nnd(L) + 8.0 * nnd(L), L, nd_coef(L, sigma, 0.0), (const double*)L.phi,
-              (double*)nullptr, kc, parts, r32, z32);
+    const auto run = L.faces_zero ? k_nd_col<double, 3, 1> : k_nd_col<double, 3, 0>;
+    KS_LAUNCH_NAMED(c, "(k_nd_col<double,2>)", run, n, BS, 8.0 * 2.0 * nnd(L) + 8.0 * nnd(L), L, nd_coef(L, sigma, 0.0), (const double*)L.phi,
+                    (double*)nullptr, kc, parts, r32, z32);
 }
 // full coarsening (2 in every direction) or a semicoarsened pair, whose
 // ratios the hierarchy's construction has checked to be 1 or 2 with F.n = r C.n
@@ -1130,7 +1130,9 @@ void launch_nd_jacobi(Ctx& c, const NDLevelT<T>& L, double sigma, double omega, 
         else
             KS_LAUNCH(c, k_nd_col2<0>, nblocks(nd_cols(L, kc), BS), BS, bytes, L, nd_coef(L, sigma, omega), in, out, kc, nullptr);
     } else {
-        KS_LAUNCH(c, (k_nd_col<T, 0>), nblocks(nd_cols(L, kc), BS), BS, bytes, L, nd_coef(L, sigma, omega), in, out, kc, nullptr);
+        const auto run = L.faces_zero ? k_nd_col<T, 0, 1> : k_nd_col<T, 0, 0>;
+        KS_LAUNCH_NAMED(c, "(k_nd_col<T,0>)", run, nblocks(nd_cols(L, kc), BS), BS, bytes, L, nd_coef(L, sigma, omega), in, out, kc, nullptr,
+                        nullptr, nullptr);
     }
 }
 template <typename T>
@@ -1147,10 +1149,13 @@ void launch_nd_resid(Ctx& c, const NDLevelT<T>& L, double sigma, double* parts, 
     }
     const int n = parts_for(nd_cols(L, kc));
     if (np) *np = n;
-    if constexpr (sizeof(T) == 4)
+    if constexpr (sizeof(T) == 4) {
         KS_LAUNCH(c, k_nd_col2<2>, n, BS, bytes, L, nd_coef(L, sigma, 0.0), (const T*)L.phi, (T*)nullptr, kc, parts);
-    else
-        KS_LAUNCH(c, (k_nd_col<T, 2>), n, BS, bytes, L, nd_coef(L, sigma, 0.0), (const T*)L.phi, (T*)nullptr, kc, parts);
+    } else {
+        const auto run = L.faces_zero ? k_nd_col<T, 2, 1> : k_nd_col<T, 2, 0>;
+        KS_LAUNCH_NAMED(c, "(k_nd_col<T,2>)", run, n, BS, bytes, L, nd_coef(L, sigma, 0.0), (const T*)L.phi, (T*)nullptr, kc, parts, nullptr,
+                        nullptr);
+    }
 }
 template <typename T>
 void launch_nd_restrict(Ctx& c, const NDLevelT<T>& F, const NDLevelT<T>& C) {
@@ -1176,7 +1181,8 @@ void launch_nd_jacobi_norm(Ctx& c, const NDLevelT<double>& L, double sigma, doub
     const int kc = nd_chunk(L);
     const int n = parts_for(nd_cols(L, kc));
     *np = n;
-    KS_LAUNCH(c, (k_nd_col<double, 1>), n, BS, 8.0 * 3.0 * nnd(L), L, nd_coef(L, sigma, omega), in, out, kc, parts);
+    const auto run = L.faces_zero ? k_nd_col<double, 1, 1> : k_nd_col<double, 1, 0>;
+    KS_LAUNCH_NAMED(c, "(k_nd_col<double,1>)", run, n, BS, 8.0 * 3.0 * nnd(L), L, nd_coef(L, sigma, omega), in, out, kc, parts, nullptr, nullptr);
 }
 void launch_nd_zero_start(Ctx& c, const NDLevelT<double>& L, double sigma, double omega, double* out, float* r32, float* z32, double* parts,
                           int* np) {

@@ -17,6 +17,7 @@
 // also forms predictor_rhs.
 #include <cfloat>
 
+#include "ks_decide.cuh"
 #include "ks_launch.hpp"
 
 namespace ks {
@@ -25,18 +26,17 @@ namespace {
 
 constexpr int BS = 256;
 
-// MC slope of a cell from its two neighbours.  edge = -1 / +1 marks the cell
-// next to a low / high ext_dir or hoextrap domain face, whose ghost holds the
-// face value: the central difference becomes the one-sided quadratic
-// (q+ + 3 q0 - 4 qb)/3 or (4 qb - 3 q0 - q-)/3.
-__device__ inline double mc_slope(double qm, double q0, double qp, int edge) {
-    const double dl = 2.0 * (q0 - qm), dr = 2.0 * (qp - q0);
-    double dc = 0.5 * (qp - qm);
-    if (edge < 0) dc = (qp + 3.0 * q0 - 4.0 * qm) / 3.0;
-    else if (edge > 0) dc = (4.0 * qp - 3.0 * q0 - qm) / 3.0;
-    double s = fmin(fabs(dl), fmin(fabs(dc), fabs(dr)));
-    if (!(dr * dl > 0.0)) s = 0.0;
-    return dc > 0.0 ? s : -s;
+// MC slope of a cell with value q0 from its two neighbours, l = q0 - qm and
+// r = qp - q0 (vls3).  edge = -1 / +1 marks the cell next to a low / high
+// ext_dir or hoextrap domain face, whose ghost holds the face value: the
+// central difference becomes the one-sided quadratic (q+ + 3 q0 - 4 qb)/3 or
+// (4 qb - 3 q0 - q-)/3.
+__device__ inline double mc_slope(double qm, double q0, double qp, double l, double r, int edge) {
+    if (edge == 0) return vls3(l, r, qp - qm);
+    const double dc = edge < 0 ? (qp + 3.0 * q0 - 4.0 * qm) / 3.0 : (4.0 * qp - 3.0 * q0 - qm) / 3.0;
+    if (!same_sign(l, r)) return 0.0;
+    const double m = twice(abs_lt(l, r) ? l : r);
+    return igt0(dc) ? iabs(abs_lt(dc, m) ? dc : m) : ineg(iabs(abs_lt(dc, m) ? dc : m));
 }
 
 // Every velocity component is ext_dir (normal) or hoextrap (tangential) at a
@@ -49,17 +49,18 @@ __device__ inline int z_edge(const Grid& g, int d, int k) {
 // ExtrapVelToFaces choice: zero where the states diverge or their mean is
 // below small_vel = 1e-10, else the upwind state
 __device__ inline double mol_pick(double umns, double upls) {
-    if (umns < 0.0 && upls > 0.0) return 0.0;
-    const double avg = 0.5 * (upls + umns);
-    if (fabs(avg) < 1.0e-10) return 0.0;
-    return avg >= 0.0 ? umns : upls;
+    if (ilt0(umns) && igt0(upls)) return 0.0;
+    const double sum = upls + umns;
+    if (iabs_lt(sum, 2.0e-10)) return 0.0;
+    return ige0(sum) ? umns : upls;
 }
 
 // compute_convective_fluxes choice: the upwind state, the mean of both where
 // |u_mac| <= small_vel = FLT_EPSILON
 __device__ inline double mol_upwind(double u, double qmns, double qpls) {
     const double small_vel = (double)FLT_EPSILON;
-    return u > small_vel ? qmns : (u < -small_vel ? qpls : 0.5 * (qmns + qpls));
+    const bool up = dbits(u) > dbits(small_vel), dn = okey(u) < okey(-small_vel);
+    return half_of((dn ? qpls : qmns) + (up ? qmns : qpls));
 }
 
 __device__ inline double* pick3(int n, double* a, double* b, double* c) { return n == 0 ? a : (n == 1 ? b : c); }
@@ -70,7 +71,10 @@ __device__ inline double* pick3(int n, double* a, double* b, double* c) { return
 // them; KIND 2 the fluxes of rho s for a cell scalar s (AdvOp_MOL.H:38-118),
 // hoextrap at z walls like a tangential component.  Each computes the MC slope of every cell once per component: the
 // x kernel takes the slope of cell i - 1 from the neighbouring lane of its warp,
-// the y and z kernels march along a column of MOL_CHUNK faces and carry it.
+// the y and z kernels march along a column of faces and carry it.  Signs and
+// magnitudes are decided on the integer pipe and rho multiplies the face's
+// velocity, once for its three components (128x128x64: 142, 105 and 114 us for the x, y and
+// z kernels with FP64 compares and every load scaled, 43, 43 and 47 now).
 
 // x faces: each warp covers 31 consecutive faces of one x row.  Lane l forms
 // the slope of cell i = 31 s + l - 1 (s: the warp's segment of the row);
@@ -90,83 +94,95 @@ __global__ void k_mol_x(Grid g, const double* vel, double rho, const double* mac
     const bool face = lane > 0 && i < g.nx;
     const int ic = min(i, g.nx - 1);  // lanes past the row end read in range and write nothing
     const long long t = ((long long)k * g.ny + j) * g.nx + (face ? i : 0);
-    const VelFP Q{vel, g, KIND ? rho : 1.0};
-    const double u = (KIND && face) ? mac[t] : 0.0;
+    const double* row0 = vel + ((long long)k * g.ny + j) * g.nx;
+    const int im = ic <= 0 ? ic - 1 + g.nx : ic - 1, i0 = ic < 0 ? ic + g.nx : ic, ip = ic + 1 >= g.nx ? ic + 1 - g.nx : ic + 1;
+    const double u = (KIND && face) ? mac[t] : 0.0, ru = rho * u;
     constexpr int nend = KIND == 1 ? 3 : 1;
     for (int n = 0; n < nend; ++n) {
-        const double b = Q(n, ic - 1, j, k), c = Q(n, ic, j, k), e = Q(n, ic + 1, j, k);
-        const double s0 = mc_slope(b, c, e, 0);
+        const double* q = row0 + n * g.N;
+        const double b = q[im], c = q[i0], e = q[ip];
+        const double s0 = mc_slope(b, c, e, c - b, e - c, 0);
         const double sm = __shfl_up_sync(0xffffffffu, s0, 1);
         if (!face) continue;
         const double qmns = b + 0.5 * sm, qpls = c - 0.5 * s0;
         if (KIND == 0) o0[t] = mol_pick(qmns, qpls);
-        else pick3(n, o0, o1, o2)[t] = mol_upwind(u, qmns, qpls) * u;
+        else pick3(n, o0, o1, o2)[t] = mol_upwind(u, qmns, qpls) * ru;
     }
 }
 
-constexpr int MOL_CHUNK = 16;
-
-// y faces: one thread per (i, k, chunk of MOL_CHUNK faces along y)
+// y faces: one thread per (i, k, chunk of faces along y)
 template <int KIND>
-__global__ void k_mol_y(Grid g, const double* vel, double rho, const double* mac, double* o0, double* o1, double* o2) {
-    const int nch = (g.ny + MOL_CHUNK - 1) / MOL_CHUNK;
+__global__ void k_mol_y(Grid g, const double* vel, double rho, const double* mac, double* o0, double* o1, double* o2, int chunk) {
+    const int nch = (g.ny + chunk - 1) / chunk;
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)g.nx * g.nz * nch) return;
     const int i = (int)(t % g.nx);
     const long long r = t / g.nx;
     const int k = (int)(r % g.nz), ch = (int)(r / g.nz);
-    const int j0 = ch * MOL_CHUNK, j1 = min(j0 + MOL_CHUNK, g.ny);
-    const VelFP Q{vel, g, KIND ? rho : 1.0};
+    const int j0 = ch * chunk, j1 = min(j0 + chunk, g.ny);
+    const double* col = vel + (long long)k * g.ny * g.nx + i;
+    auto Q = [&](int n, int j) { return col[n * g.N + (long long)(j < 0 ? j + g.ny : (j >= g.ny ? j - g.ny : j)) * g.nx]; };
     const int nbeg = KIND == 0 ? 1 : 0, nend = KIND == 0 ? 2 : (KIND == 1 ? 3 : 1);
     for (int n = nbeg; n < nend; ++n) {
-        double qb = Q(n, i, j0 - 1, k), qc = Q(n, i, j0, k);
-        double sb = mc_slope(Q(n, i, j0 - 2, k), qb, qc, 0);
+        double qb = Q(n, j0 - 1), qc = Q(n, j0), l = qc - qb;
+        const double qa = Q(n, j0 - 2);
+        double sb = mc_slope(qa, qb, qc, qb - qa, l, 0);
         for (int j = j0; j < j1; ++j) {
-            const double qe = Q(n, i, j + 1, k);
-            const double sc = mc_slope(qb, qc, qe, 0);
+            const double qe = Q(n, j + 1), r1 = qe - qc;
+            const double sc = mc_slope(qb, qc, qe, l, r1, 0);
             const double qmns = qb + 0.5 * sb, qpls = qc - 0.5 * sc;
             const long long f = cidx(g, i, j, k);
-            if (KIND == 0) o0[f] = mol_pick(qmns, qpls);
-            else pick3(n, o0, o1, o2)[f] = mol_upwind(mac[f], qmns, qpls) * mac[f];
+            if (KIND == 0) {
+                o0[f] = mol_pick(qmns, qpls);
+            } else {
+                const double u = mac[f];
+                pick3(n, o0, o1, o2)[f] = mol_upwind(u, qmns, qpls) * (rho * u);
+            }
             qb = qc;
             qc = qe;
             sb = sc;
+            l = r1;
         }
     }
 }
 
-// z faces: one thread per (i, j, chunk of MOL_CHUNK face layers); on a wall
+// z faces: one thread per (i, j, chunk of face layers); on a wall
 // face the normal component takes the ghost (boundary) value 0
 template <int KIND>
-__global__ void k_mol_z(Grid g, const double* vel, double rho, const double* mac, double* o0, double* o1, double* o2) {
+__global__ void k_mol_z(Grid g, const double* vel, double rho, const double* mac, double* o0, double* o1, double* o2, int chunk) {
     const int nzf = nzfaces(g);
-    const int nch = (nzf + MOL_CHUNK - 1) / MOL_CHUNK;
+    const int nch = (nzf + chunk - 1) / chunk;
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)g.nx * g.ny * nch) return;
     const int i = (int)(t % g.nx);
     const long long r = t / g.nx;
     const int j = (int)(r % g.ny), ch = (int)(r / g.ny);
-    const int k0 = ch * MOL_CHUNK, k1 = min(k0 + MOL_CHUNK, nzf);
-    const VelFP Q{vel, g, KIND ? rho : 1.0};
+    const int k0 = ch * chunk, k1 = min(k0 + chunk, nzf);
+    const VelFP G{vel, g, 1.0};
+    const double* col = vel + (long long)j * g.nx + i;
+    const long long sz = (long long)g.nx * g.ny;
     const int nbeg = KIND == 0 ? 2 : 0, nend = KIND == 2 ? 1 : 3;
     for (int n = nbeg; n < nend; ++n) {
-        double qb = Q(n, i, j, k0 - 1), qc = Q(n, i, j, k0);
-        double sb = mc_slope(Q(n, i, j, k0 - 2), qb, qc, z_edge(g, 2, k0 - 1));
+        const double* q = col + n * g.N;
+        const double qa = G(n, i, j, k0 - 2), top = g.zper ? q[0] : (k1 >= g.nz ? G(n, i, j, g.nz) : 0.0);
+        double qb = G(n, i, j, k0 - 1), qc = k0 < g.nz ? q[k0 * sz] : top, l = qc - qb;
+        double sb = mc_slope(qa, qb, qc, qb - qa, l, z_edge(g, 2, k0 - 1));
         for (int k = k0; k < k1; ++k) {
-            const double qe = Q(n, i, j, k + 1);
-            const double sc = mc_slope(qb, qc, qe, z_edge(g, 2, k));
+            const double qe = k + 1 < g.nz ? q[(k + 1) * sz] : top, r1 = qe - qc;
+            const double sc = mc_slope(qb, qc, qe, l, r1, z_edge(g, 2, k));
             const double qmns = qb + 0.5 * sb, qpls = qc - 0.5 * sc;
-            const long long f = fidx(g, 2, i, j, k);
+            const long long f = (long long)k * sz + (long long)j * g.nx + i;
             const bool wall = !g.zper && (k == 0 || k == g.nz);
             if (KIND == 0) {
                 o0[f] = wall ? 0.0 : mol_pick(qmns, qpls);
             } else {
                 const double u = mac[f];
-                pick3(n, o0, o1, o2)[f] = ((wall && n == 2) ? 0.0 : mol_upwind(u, qmns, qpls)) * u;
+                pick3(n, o0, o1, o2)[f] = ((wall && n == 2) ? 0.0 : mol_upwind(u, qmns, qpls)) * (rho * u);
             }
             qb = qc;
             qc = qe;
             sb = sc;
+            l = r1;
         }
     }
 }
@@ -206,8 +222,9 @@ inline long long nfaces_d(const Grid& g, int d) { return (long long)g.nx * g.ny 
 template <int KIND>
 static void mol_faces(Ctx& c, const Grid& g, const double* vel, double rho, const double* const mac[3], double* const out[9]) {
     const double nc = KIND == 1 ? 3.0 : 1.0;  // components read and written per face
-    const long long ty = (long long)g.nx * g.nz * ((g.ny + MOL_CHUNK - 1) / MOL_CHUNK);
-    const long long tz = (long long)g.nx * g.ny * ((nzfaces(g) + MOL_CHUNK - 1) / MOL_CHUNK);
+    const int chunk = march_chunk<double>(g, 1, 16);
+    const long long ty = (long long)g.nx * g.nz * ((g.ny + chunk - 1) / chunk);
+    const long long tz = (long long)g.nx * g.ny * ((nzfaces(g) + chunk - 1) / chunk);
     const double nfz = (double)nfaces_d(g, 2);
     auto o = [&](int d, int n) { return out[KIND == 1 ? 3 * d + n : d]; };
     const double* m0 = KIND ? mac[0] : nullptr;
@@ -215,9 +232,9 @@ static void mol_faces(Ctx& c, const Grid& g, const double* vel, double rho, cons
     const double* m2 = KIND ? mac[2] : nullptr;
     const long long tx = 32LL * g.ny * g.nz * ((g.nx + XSEG - 1) / XSEG);
     KS_LAUNCH(c, k_mol_x<KIND>, nblocks(tx, BS), BS, 8.0 * (2.0 * nc + KIND) * g.N, g, vel, rho, m0, o(0, 0), o(0, 1), o(0, 2));
-    KS_LAUNCH(c, k_mol_y<KIND>, nblocks(ty, BS), BS, 8.0 * (2.0 * nc + KIND) * g.N, g, vel, rho, m1, o(1, 0), o(1, 1), o(1, 2));
+    KS_LAUNCH(c, k_mol_y<KIND>, nblocks(ty, BS), BS, 8.0 * (2.0 * nc + KIND) * g.N, g, vel, rho, m1, o(1, 0), o(1, 1), o(1, 2), chunk);
     KS_LAUNCH(c, k_mol_z<KIND>, nblocks(tz, BS), BS, 8.0 * (nc * g.N + (nc + KIND) * nfz), g, vel, rho, m2, o(2, 0), o(2, 1),
-              o(2, 2));
+              o(2, 2), chunk);
 }
 
 void launch_mol_extrap(Ctx& c, const Grid& g, const double* vel, double* const mac[3]) {

@@ -265,12 +265,14 @@ __global__ void k_modes_setup(SpectralZ Z) {
 }
 
 // The z systems of all modes, in place on the transformed plane pairs C.  A
-// thread marches its column up (elimination, the next pair's loads issued
-// before the current pair's arithmetic) and down (substitution).  The
-// coefficients of the real planes 2m and 2m + 1 are
+// thread marches its column up (elimination) and down (substitution), kAhead
+// pairs at a time whose loads were issued a group earlier: a box has few modes
+// (2080 on 64^3), so the march is a chain of loads unless several are in
+// flight (MODES_MEASURED).  The coefficients of the real planes 2m and 2m + 1 are
 //   A = (C + conj C~) / 2,   B = (C - conj C~) / 2i,
 // C~ the entry of the opposite mode (the factor 1/2 is left to the output's
 // scale); on the way up the pair's two slots hold the eliminated A and B.
+constexpr int kAhead = 4;
 __global__ void __launch_bounds__(128) k_modes_z(SpectralZ Z, double2* C) {
     const int kx = blockIdx.x * blockDim.x + threadIdx.x, ky = blockIdx.y;
     if (kx >= Z.nx) return;
@@ -294,6 +296,7 @@ __global__ void __launch_bounds__(128) k_modes_z(SpectralZ Z, double2* C) {
     if (Z.zper) {
         const double* w = Z.w + md;
         double2 s = make_double2(0.0, 0.0);
+#pragma unroll 4
         for (int m = 0; m < np; ++m) {
             double2 A, B;
             sep(c[m * plane], o[m * plane], A, B);
@@ -304,71 +307,88 @@ __global__ void __launch_bounds__(128) k_modes_z(SpectralZ Z, double2* C) {
         const double q = Z.schur[md];
         last = make_double2(q * s.x, q * s.y);
     }
+    struct Pair {
+        double2 p, q;
+        double da, db;
+    };
+    auto load = [&](int m) {
+        Pair r{};
+        if (m < 0 || m >= np) return r;
+        r.p = c[m * plane];
+        r.q = o[m * plane];
+        r.da = dinv[(long long)(2 * m) * M];
+        r.db = 2 * m + 1 < nu ? dinv[(long long)(2 * m + 1) * M] : 0.0;
+        return r;
+    };
     // up: z_k = b_k - e dinv_{k-1} z_{k-1}
     double2 z = make_double2(0.0, 0.0);
     double di = 0.0;
-    double2 p = c[0], q = o[0];
-    for (int m = 0; m < np; ++m) {
-        double2 pn = p, qn = q;
-        if (m + 1 < np) {
-            pn = c[(m + 1) * plane];
-            qn = o[(m + 1) * plane];
+    Pair cur[kAhead], nxt[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) cur[u] = load(u);
+    for (int m0 = 0; m0 < np; m0 += kAhead) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) nxt[u] = load(m0 + kAhead + u);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int m = m0 + u, k = 2 * m;
+            if (m >= np) break;
+            double2 A, B;
+            sep(cur[u].p, cur[u].q, A, B);
+            if (Z.nodal && !Z.zper) {
+                if (k == 0 || k == nz - 1) A = make_double2(0.5 * A.x, 0.5 * A.y);
+                if (k + 1 == nz - 1) B = make_double2(0.5 * B.x, 0.5 * B.y);
+            }
+            if (Z.zper) {
+                if (k == 0) A = make_double2(fma(-e, last.x, A.x), fma(-e, last.y, A.y));
+                if (k == nu - 1) A = make_double2(fma(-e, last.x, A.x), fma(-e, last.y, A.y));
+            }
+            double l = -e * di;
+            A = make_double2(fma(l, z.x, A.x), fma(l, z.y, A.y));
+            l = -e * cur[u].da;
+            B = make_double2(fma(l, A.x, B.x), fma(l, A.y, B.y));
+            if (self) {  // both planes' coefficients are real here: one slot holds them
+                c[m * plane] = make_double2(A.x, B.x);
+            } else {
+                c[m * plane] = A;
+                o[m * plane] = B;
+            }
+            z = B;
+            di = cur[u].db;
         }
-        const int k = 2 * m;
-        const double da = dinv[(long long)k * M], db = k + 1 < nu ? dinv[(long long)(k + 1) * M] : 0.0;
-        double2 A, B;
-        sep(p, q, A, B);
-        if (Z.nodal && !Z.zper) {
-            if (k == 0 || k == nz - 1) A = make_double2(0.5 * A.x, 0.5 * A.y);
-            if (k + 1 == nz - 1) B = make_double2(0.5 * B.x, 0.5 * B.y);
-        }
-        if (Z.zper) {
-            if (k == 0) A = make_double2(fma(-e, last.x, A.x), fma(-e, last.y, A.y));
-            if (k == nu - 1) A = make_double2(fma(-e, last.x, A.x), fma(-e, last.y, A.y));
-        }
-        double l = -e * di;
-        A = make_double2(fma(l, z.x, A.x), fma(l, z.y, A.y));
-        l = -e * da;
-        B = make_double2(fma(l, A.x, B.x), fma(l, A.y, B.y));
-        if (self) {  // both planes' coefficients are real here: one slot holds them
-            c[m * plane] = make_double2(A.x, B.x);
-        } else {
-            c[m * plane] = A;
-            o[m * plane] = B;
-        }
-        z = B;
-        di = db;
-        p = pn;
-        q = qn;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) cur[u] = nxt[u];
     }
     // down: x_k = dinv_k z_k - e dinv_k x_{k+1}, and C = A + i B, C~ = conj A + i conj B
     double2 x = make_double2(0.0, 0.0);
-    p = c[(np - 1) * plane];
-    q = o[(np - 1) * plane];
-    for (int m = np - 1; m >= 0; --m) {
-        double2 pn = p, qn = q;
-        if (m > 0) {
-            pn = c[(m - 1) * plane];
-            qn = o[(m - 1) * plane];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) cur[u] = load(np - 1 - u);
+    for (int m0 = np - 1; m0 >= 0; m0 -= kAhead) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) nxt[u] = load(m0 - kAhead - u);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int m = m0 - u, k = 2 * m;
+            if (m < 0) break;
+            const double2 p = cur[u].p, q = cur[u].q;
+            double2 A = self ? make_double2(p.x, 0.0) : p, B = self ? make_double2(p.y, 0.0) : q;
+            if (k + 1 < nu) {
+                const double db = cur[u].db, cb = -e * db;
+                B = make_double2(fma(cb, x.x, db * B.x), fma(cb, x.y, db * B.y));
+                x = B;
+            } else if (k + 1 < nz) {
+                B = last;  // cyclic: already folded into rows 0 and nz - 2
+            } else {
+                B = make_double2(0.0, 0.0);  // past the last node plane
+            }
+            const double da = cur[u].da, ca = -e * da;
+            A = make_double2(fma(ca, x.x, da * A.x), fma(ca, x.y, da * A.y));
+            x = A;
+            c[m * plane] = make_double2(A.x - B.y, A.y + B.x);
+            if (!self) o[m * plane] = make_double2(A.x + B.y, B.x - A.y);
         }
-        const int k = 2 * m;
-        double2 A = self ? make_double2(p.x, 0.0) : p, B = self ? make_double2(p.y, 0.0) : q;
-        if (k + 1 < nu) {
-            const double db = dinv[(long long)(k + 1) * M], cb = -e * db;
-            B = make_double2(fma(cb, x.x, db * B.x), fma(cb, x.y, db * B.y));
-            x = B;
-        } else if (k + 1 < nz) {
-            B = last;  // cyclic: already folded into rows 0 and nz - 2
-        } else {
-            B = make_double2(0.0, 0.0);  // past the last node plane
-        }
-        const double da = dinv[(long long)k * M], ca = -e * da;
-        A = make_double2(fma(ca, x.x, da * A.x), fma(ca, x.y, da * A.y));
-        x = A;
-        c[m * plane] = make_double2(A.x - B.y, A.y + B.x);
-        if (!self) o[m * plane] = make_double2(A.x + B.y, B.x - A.y);
-        p = pn;
-        q = qn;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) cur[u] = nxt[u];
     }
 }
 
