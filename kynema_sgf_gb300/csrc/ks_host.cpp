@@ -617,18 +617,22 @@ void Sim::mac_semi_mixed() {
 //     contracts by 0.4 to 0.7 a V-cycle there (256 x 256 x 128 cells of
 //     20 x 20 x 10 m: 76 MAC and 28 nodal V-cycles, 78 and 55 ms a step,
 //     against 1.1 and 1.3 ms for a direct start with its residual);
-//   - on fully periodic boxes of at most 2^18 cells, whose V-cycles are bound by
-//     launches (32^3: 8 V-cycles 0.9 ms, direct 0.1 ms);
+//   - on fully periodic boxes: their V-cycles are bound by launches up to 2^18
+//     cells (32^3: 8 V-cycles 0.9 ms, direct 0.1 ms), are 8 a solve above (two
+//     Taylor-Green steps on 96^3: 17.5 ms, 5.5 direct), and counts that halve
+//     once or twice sweep a large coarsest level (72^3: 118 ms, 3.6 direct);
+//   - in the forward steps of the reverse mode, and in the two reverse solves of
+//     its mixed-precision form (adj_alloc);
 //   - in a nodal projection that is called by itself (ApplyProjection): the
 //     pressure at hand is no guess for another velocity (160 x 96 x 80 cells of
 //     20 m, whose coarsest level takes 100 sweeps: 21.5 ms, direct 0.8 ms).
-// Elsewhere (cubic cells between walls, large boxes) 8 V-cycles reach the
-// tolerance and remain: the mixed form's V-cycles are counted against them.
+// Elsewhere (cubic cells between walls) 8 V-cycles reach the tolerance and
+// remain: the mixed form's V-cycles are counted against them, and they leave
+// 1.4e-9 of the pressure, by which a direct start would change it.
 // So do the multigrid iterates
 //   - of the mixed-precision form, whose FP32 advection turns any change of
 //     an iterate into another trajectory at its rounding level;
-//   - under ks.mg_warm_start = 0 (solves start from zero, as the reference's),
-//     which the reverse mode sets too;
+//   - under ks.mg_warm_start = 0 (solves start from zero, as the reference's);
 //   - of decks that limit the V-cycles (maxiter below MLMG's default of 200)
 //     and so ask for those iterates;
 //   - on counts with a prime factor above 13 or above kSpectralMax.
@@ -695,9 +699,9 @@ bool Sim::spectral_setup(bool nodal) {
 // the rule of the step's solves (see above)
 void Sim::spectral_choose() {
     const double hmin = std::min(g_.dx, std::min(g_.dy, g_.dz)), hmax = std::max(g_.dx, std::max(g_.dy, g_.dz));
-    const bool gains = hmax > 1.25 * hmin || (g_.zper && g_.N <= (1LL << 18));
-    mac_direct_ = gains && spectral_setup(false);
-    nod_direct_ = gains && spectral_setup(true);
+    const bool gains = hmax > 1.25 * hmin || g_.zper;
+    mac_direct_ = (gains || adj_direct_) && spectral_setup(false);
+    nod_direct_ = (gains || adj_direct_) && spectral_setup(true);
 }
 
 // phi = (coef * operator)^-1 rhs, and |rhs|'s block maxima (its caller's last

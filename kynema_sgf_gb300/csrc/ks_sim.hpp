@@ -421,7 +421,9 @@ class Sim {
     int nod_bparts_ = 0;  // block maxima of |rhs| that nd_rhs left in parts_ for the direct start
     bool mac_direct_ = false, nod_direct_ = false;
     bool nod_alone_ = false;  // inside projection_alone, with the nodal factors at hand
-    bool direct_start(bool solve) const { return solve && mg_warm_ && !mixed_; }
+    bool adj_direct_ = false;  // the reverse mode of a handle whose solves may start directly
+    bool reverse_ = false;     // inside the two solves of a reverse step
+    bool direct_start(bool solve) const { return solve && (mixed_ ? reverse_ : !reverse_ && (mg_warm_ || adj_direct_)); }
     SpectralZ zmac_{}, znod_{};
     DevBuf<double> spec_tab_, spec_mac_, spec_nod_;  // roots and eigenvalues; z factors
     const double2 *tw_x_ = nullptr, *tw_y_ = nullptr;

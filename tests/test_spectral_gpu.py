@@ -115,6 +115,28 @@ def test_mac_projection_is_exact(cuda_dev, n, walls):
     assert sim.scalar("mac_divu_rel") <= 1e-12
 
 
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-7), ("mixed", 1e-4)])
+@pytest.mark.parametrize("n", [(32, 32, 16), (48, 20, 24)])
+def test_reverse_step_with_direct_solves(cuda_dev, n, precision, tol):
+    """A reverse step whose forward solves (FP64) or reverse solves (mixed) start
+    directly, against the same step on multigrid iterates from zero.  The
+    multigrid's tolerance of 2e-11 on the residual leaves up to 1e-8 of an
+    adjoint field (condition number below 1e3), FP32 roundings 1e-5.
+    """
+    out = []
+    for warm in (1, 0):
+        d, lo, hi, _ = decks.adjoint_c3(*n, dcells=4, n_disks=2)
+        sim = cuda_dev.Incflo(d + "ks.precision = %s\nks.mg_warm_start = %d\n" % (precision, warm))
+        sim.InitData()
+        sim.set_objective_box(lo, hi)
+        sim.objective(seed=True)
+        sim.adjoint_step()
+        assert (sim.scalar("mac_iters") == 0) == (warm == 1 and precision == "mixed")  # the last MAC solve is the reverse one
+        out.append([sim.get_field("velocity_adjoint"), sim.get_field("gp_adjoint"), sim.ct_gradient()])
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= tol * np.abs(b).max()
+
+
 def test_multigrid_where_it_is_asked_for(cuda_dev):
     """ks.mg_warm_start = 0, a limit on the V-cycles, mixed precision or a count
     with a large prime keep the multigrid solve, to the same fields."""
