@@ -546,30 +546,30 @@ __global__ void k_adj_pm_trans(Grid g, int a, int b, int n, double cb64, const T
     const long long f = t;
     const double ob64 = outb[f];
     if (!(dbits(ob64) & kMag)) return;
-    const A ob = (A)ob64, cb = (A)cb64;
+    const A ob = to<A>(ob64), cb = to<A>(cb64);
     const bool wl = (a == 2 && !g.zper && k == 0), wh = (a == 2 && !g.zper && k == g.nz);
     A lb = A(0), hb = A(0);
     rev_upwind(ad_a[f], ob, lb, hb);
     if (a == 2) zbc_rev(g, k, n, lb, hb);
-    lo_anb[f] += (double)lb;
-    hi_anb[f] += (double)hb;
+    lo_anb[f] += to<double>(lb);
+    hi_anb[f] += to<double>(hb);
     const int e0 = (b == 0), e1 = (b == 1), e2 = (b == 2);
     if (!wh && nonzero(hb)) {
         const long long f0 = fidx(g, b, i, j, k), f1 = fidx(g, b, i + e0, j + e1, k + e2);
         const A S = ad_b[f1] + ad_b[f0], Dd = edge_b[f1] - edge_b[f0];
-        aadd(&ad_bb[f1], (double)(-cb * Dd * hb));
-        aadd(&ad_bb[f0], (double)(-cb * Dd * hb));
-        aadd(&edge_bb[f1], (double)(-cb * S * hb));
-        aadd(&edge_bb[f0], (double)(cb * S * hb));
+        aadd(&ad_bb[f1], to<double>(-cb * Dd * hb));
+        aadd(&ad_bb[f0], to<double>(-cb * Dd * hb));
+        aadd(&edge_bb[f1], to<double>(-cb * S * hb));
+        aadd(&edge_bb[f0], to<double>(cb * S * hb));
     }
     if (!wl && nonzero(lb)) {
         const int ci = i - (a == 0), cj = j - (a == 1), ck = k - (a == 2);
         const long long f0 = fidx(g, b, ci, cj, ck), f1 = fidx(g, b, ci + e0, cj + e1, ck + e2);
         const A S = ad_b[f1] + ad_b[f0], Dd = edge_b[f1] - edge_b[f0];
-        aadd(&ad_bb[f1], (double)(-cb * Dd * lb));
-        aadd(&ad_bb[f0], (double)(-cb * Dd * lb));
-        aadd(&edge_bb[f1], (double)(-cb * S * lb));
-        aadd(&edge_bb[f0], (double)(cb * S * lb));
+        aadd(&ad_bb[f1], to<double>(-cb * Dd * lb));
+        aadd(&ad_bb[f0], to<double>(-cb * Dd * lb));
+        aadd(&edge_bb[f1], to<double>(-cb * S * lb));
+        aadd(&edge_bb[f0], to<double>(cb * S * lb));
     }
 }
 
@@ -761,20 +761,20 @@ __global__ void k_adj_flux_cells(Grid g, int d, double rho64, double dt64, doubl
     if (!face_at(g, 0, t, i, j, k)) return;  // the x-face domain is the cell domain
     const int b1 = (d + 1) % 3, b2 = (d + 2) % 3;
     const long long flo = fidx(g, d, i, j, k), fhi = fidx(g, d, i + (d == 0), j + (d == 1), k + (d == 2));
-    const A ulo = (A)Uf.p[d][flo], uhi = (A)Uf.p[d][fhi];
+    const A ulo = to<A>(Uf.p[d][flo]), uhi = to<A>(Uf.p[d][fhi]);
     const long long p1 = fidx(g, b1, i + (b1 == 0), j + (b1 == 1), k + (b1 == 2)), m1 = fidx(g, b1, i, j, k);
     const long long p2 = fidx(g, b2, i + (b2 == 0), j + (b2 == 1), k + (b2 == 2)), m2 = fidx(g, b2, i, j, k);
-    const A rho = (A)rho64, c1 = (A)c1_64, c2 = (A)c2_64, hdt = A(0.5) * (A)dt64;
-    const A r = rho * (c1 * ((A)Uf.p[b1][p1] - (A)Uf.p[b1][m1]) + c2 * ((A)Uf.p[b2][p2] - (A)Uf.p[b2][m2]));
+    const A rho = to<A>(rho64), c1 = to<A>(c1_64), c2 = to<A>(c2_64), hdt = A(0.5) * to<A>(dt64);
+    const A r = rho * (c1 * (to<A>(Uf.p[b1][p1]) - to<A>(Uf.p[b1][m1])) + c2 * (to<A>(Uf.p[b2][p2]) - to<A>(Uf.p[b2][m2])));
     for (int n = 0; n < 3; ++n) {
         A bl, bh, dl, dh;
-        flux_state_rev(g, d, k, n, ulo, (A)Fb.p[n][flo], dl, bh);
-        flux_state_rev(g, d, k + 1, n, uhi, (A)Fb.p[n][fhi], bl, dh);
+        flux_state_rev(g, d, k, n, ulo, to<A>(Fb.p[n][flo]), dl, bh);
+        flux_state_rev(g, d, k + 1, n, uhi, to<A>(Fb.p[n][fhi]), bl, dh);
         const A cb = bh + bl;
         CB[n * g.N + t] = cb;
         if (nonzero(cb)) {
-            ub[n * g.N + t] += (double)(r * cb);
-            forcesb[n * g.N + t] += (double)(hdt * rho * cb);
+            ub[n * g.N + t] += to<double>(r * cb);
+            forcesb[n * g.N + t] += to<double>(hdt * rho * cb);
         }
     }
 }
@@ -797,17 +797,17 @@ __global__ void k_adj_bfaces(Grid g, int b, const double* u, double rho64, doubl
     const long long f = t;
     const long long cp = hasp ? cidx(g, i, j, k) : 0;
     const long long cm = hasm ? cidx(g, wrapn(i - (b == 0), g.nx), wrapn(j - (b == 1), g.ny), g.zper ? wrapn(k - (b == 2), g.nz) : k - (b == 2)) : 0;
-    const A c = (A)c64, rho = (A)rho64, v = (A)vb[f];
+    const A c = to<A>(c64), rho = to<A>(rho64), v = to<A>(vb[f]);
     A gv = A(0);
     for (int n = 0; n < 3; ++n) {
         const A bp = hasp ? CB[n * g.N + cp] : A(0), bm = hasm ? CB[n * g.N + cm] : A(0);
         if (!nonzero(bp) && !nonzero(bm)) continue;
         const A e = T.p[n][f];
-        Tb.p[n][f] += (double)(c * v * (bp - bm));
-        const A qm = hasm ? rho * (A)u[n * g.N + cm] : A(0), qp = hasp ? rho * (A)u[n * g.N + cp] : A(0);
+        Tb.p[n][f] += to<double>(c * v * (bp - bm));
+        const A qm = hasm ? rho * to<A>(u[n * g.N + cm]) : A(0), qp = hasp ? rho * to<A>(u[n * g.N + cp]) : A(0);
         gv += (c * qm - c * e) * bm + (c * e - c * qp) * bp;
     }
-    if (nonzero(gv)) vbb[f] += (double)gv;
+    if (nonzero(gv)) vbb[f] += to<double>(gv);
 }
 
 // stage 2 for the a-faces, per cell: the adjoints of its two corrections (one
@@ -825,18 +825,18 @@ __global__ void k_adj_trans_cells(Grid g, int a, double rho64, double cb1_64, do
     const int b1 = (a + 1) % 3, b2 = (a + 2) % 3;
     const bool top = a == 2 && !g.zper && k + 1 == g.nz;  // the face above is the top wall face
     const long long flo = fidx(g, a, i, j, k), fhi = fidx(g, a, i + (a == 0), j + (a == 1), k + (a == 2));
-    const A ulo = (A)ua[flo], uhi = (A)ua[fhi];
+    const A ulo = to<A>(ua[flo]), uhi = to<A>(ua[fhi]);
     const long long p1 = fidx(g, b1, i + (b1 == 0), j + (b1 == 1), k + (b1 == 2)), m1 = fidx(g, b1, i, j, k);
     const long long p2 = fidx(g, b2, i + (b2 == 0), j + (b2 == 1), k + (b2 == 2)), m2 = fidx(g, b2, i, j, k);
-    const A rho = (A)rho64;
-    const A w1 = rho * (A)cb1_64 * ((A)v1[p1] - (A)v1[m1]), w2 = rho * (A)cb2_64 * ((A)v2[p2] - (A)v2[m2]);
+    const A rho = to<A>(rho64);
+    const A w1 = rho * to<A>(cb1_64) * (to<A>(v1[p1]) - to<A>(v1[m1])), w2 = rho * to<A>(cb2_64) * (to<A>(v2[p2]) - to<A>(v2[m2]));
     A ubs[3];
     for (int n = 0; n < 3; ++n) {
         A l1 = A(0), h1 = A(0), l2 = A(0), h2 = A(0), L1 = A(0), H1 = A(0), L2 = A(0), H2 = A(0);
-        rev_upwind(ulo, (A)O1b.p[n][flo], l1, h1);  // face below
-        rev_upwind(ulo, (A)O2b.p[n][flo], l2, h2);
-        rev_upwind(uhi, (A)O1b.p[n][fhi], L1, H1);  // face above
-        rev_upwind(uhi, (A)O2b.p[n][fhi], L2, H2);
+        rev_upwind(ulo, to<A>(O1b.p[n][flo]), l1, h1);  // face below
+        rev_upwind(ulo, to<A>(O2b.p[n][flo]), l2, h2);
+        rev_upwind(uhi, to<A>(O1b.p[n][fhi]), L1, H1);  // face above
+        rev_upwind(uhi, to<A>(O2b.p[n][fhi]), L2, H2);
         if (a == 2) {
             zbc_rev(g, k, n, l1, h1);
             zbc_rev(g, k, n, l2, h2);
@@ -844,11 +844,11 @@ __global__ void k_adj_trans_cells(Grid g, int a, double rho64, double cb1_64, do
             zbc_rev(g, k + 1, n, L2, H2);
         }
         const A sl = l1 + l2, sh = h1 + h2;
-        if (nonzero(sl)) LOb.p[n][flo] += (double)sl;
-        if (nonzero(sh)) HIb.p[n][flo] += (double)sh;
+        if (nonzero(sl)) LOb.p[n][flo] += to<double>(sl);
+        if (nonzero(sh)) HIb.p[n][flo] += to<double>(sh);
         if (top) {
-            LOb.p[n][fhi] += (double)(L1 + L2);
-            HIb.p[n][fhi] += (double)(H1 + H2);
+            LOb.p[n][fhi] += to<double>(L1 + L2);
+            HIb.p[n][fhi] += to<double>(H1 + H2);
         }
         const A cb1 = h1 + L1, cb2 = h2 + L2;
         CB[n * g.N + t] = cb1;
@@ -856,7 +856,7 @@ __global__ void k_adj_trans_cells(Grid g, int a, double rho64, double cb1_64, do
         ubs[n] = w1 * cb1 + w2 * cb2;
     }
     for (int n = 0; n < 3; ++n)
-        if (nonzero(ubs[n])) ub[n * g.N + t] += (double)ubs[n];
+        if (nonzero(ubs[n])) ub[n * g.N + t] += to<double>(ubs[n]);
 }
 
 // ---- reverse of conv = -div F on d-faces: Fb(f) = (convb(cell above f) - convb(cell below f)) / h_d
@@ -1161,7 +1161,7 @@ __global__ void k_adj_smag_w(Grid g, const double* vel, const double* mub, doubl
     if (!face_at(g, 0, t, i, j, k)) return;
     const double mb = mub[t];
     A gxb[3] = {A(0), A(0), A(0)}, gyb[3] = {A(0), A(0), A(0)}, gzb[3] = {A(0), A(0), A(0)};
-    const A hx = A(0.5 * g.idx), hy = A(0.5 * g.idy), iz = (A)g.idz;
+    const A hx = A(0.5 * g.idx), hy = A(0.5 * g.idy), iz = to<A>(g.idz);
     if (dbits(mb) & kMag) {
         A a, b, c;
         smag_zcoef(g, k, a, b, c);
@@ -1173,21 +1173,21 @@ __global__ void k_adj_smag_w(Grid g, const double* vel, const double* mub, doubl
         A gx[3], gy[3], gz[3];
         for (int n = 0; n < 3; ++n) {
             const double* v = vel + n * g.N;
-            gx[n] = hx * ((A)v[xp] - (A)v[xm]);
-            gy[n] = hy * ((A)v[yp] - (A)v[ym]);
+            gx[n] = hx * (to<A>(v[xp]) - to<A>(v[xm]));
+            gy[n] = hy * (to<A>(v[yp]) - to<A>(v[ym]));
             // fill-patch ghost (VelFPT): the normal component 0, the others
             // (15 q0 - 10 q1 + 3 q2) / 8 from the three cells next to the wall
             A qm, qp;
-            if (glo) qm = n == 2 ? A(0) : A(0.125) * (A(15) * (A)v[t] - A(10) * (A)v[t + sz] + A(3) * (A)v[t + 2 * sz]);
-            else qm = (A)v[zm];
-            if (ghi) qp = n == 2 ? A(0) : A(0.125) * (A(15) * (A)v[t] - A(10) * (A)v[t - sz] + A(3) * (A)v[t - 2 * sz]);
-            else qp = (A)v[zp];
-            gz[n] = (a * qp + b * (A)v[t] + c * qm) * iz;
+            if (glo) qm = n == 2 ? A(0) : A(0.125) * (A(15) * to<A>(v[t]) - A(10) * to<A>(v[t + sz]) + A(3) * to<A>(v[t + 2 * sz]));
+            else qm = to<A>(v[zm]);
+            if (ghi) qp = n == 2 ? A(0) : A(0.125) * (A(15) * to<A>(v[t]) - A(10) * to<A>(v[t - sz]) + A(3) * to<A>(v[t - 2 * sz]));
+            else qp = to<A>(v[zp]);
+            gz[n] = (a * qp + b * to<A>(v[t]) + c * qm) * iz;
         }
         const A S = sqrt(A(2) * gx[0] * gx[0] + A(2) * gy[1] * gy[1] + A(2) * gz[2] * gz[2] + (gy[0] + gx[1]) * (gy[0] + gx[1]) +
                          (gz[1] + gy[2]) * (gz[1] + gy[2]) + (gx[2] + gz[0]) * (gx[2] + gz[0]));
         if (S > A(0)) {
-            const A q = (A)(rho * fac * mb) / S;
+            const A q = to<A>(rho * fac * mb) / S;
             gxb[0] = A(2) * q * gx[0];
             gyb[1] = A(2) * q * gy[1];
             gzb[2] = A(2) * q * gz[2];

@@ -44,35 +44,46 @@ __host__ __device__ inline long long fidx(const Grid& g, int d, int i, int j, in
     return cidx(g, i, j, k);
 }
 
+#ifdef __CUDACC__
+template <typename To>
+__device__ __forceinline__ To to(double x);
+template <typename To>
+__device__ __forceinline__ To to(float x);
+
 // Cell-centred velocity (or rho*velocity) with fill-patch ghost values:
 // periodic wrap in x, y (and z); at walls the tangential components take the
 // high-order extrapolation to the face, (15 q0 - 10 q1 + 3 q2)/8, in every
 // ghost layer and the normal component is 0.  The field is stored as S
 // (FP64, or its FP32 copy in the mixed-precision advection); the value is
 // returned in the arithmetic type T of the caller.
-template <typename T = double, typename S = double>
+template <typename T = double, typename S = double, bool INT = false>
 struct VelFPT {
     const S* v;
     Grid g;
     T scale;
+    // INT: converted on the integer pipe (to, below)
+    static __device__ inline T cv(S x) {
+        if constexpr (INT) return to<T>(x);
+        else return (T)x;
+    }
     __device__ inline T operator()(int n, int i, int j, int k) const {
         i = wrapn(i, g.nx);
         j = wrapn(j, g.ny);
         const long long N = g.N;
         const S* c = v + n * N;
-        if (g.zper) return scale * (T)c[cidx(g, i, j, wrapn(k, g.nz))];
+        if (g.zper) return scale * cv(c[cidx(g, i, j, wrapn(k, g.nz))]);
         if (k < 0) {
             if (n == 2) return T(0);
-            const T q0 = (T)c[cidx(g, i, j, 0)], q1 = (T)c[cidx(g, i, j, 1)], q2 = (T)c[cidx(g, i, j, 2)];
+            const T q0 = cv(c[cidx(g, i, j, 0)]), q1 = cv(c[cidx(g, i, j, 1)]), q2 = cv(c[cidx(g, i, j, 2)]);
             return scale * (T(0.125) * (T(15) * q0 - T(10) * q1 + T(3) * q2));
         }
         if (k >= g.nz) {
             if (n == 2) return T(0);
             const int t = g.nz - 1;
-            const T q0 = (T)c[cidx(g, i, j, t)], q1 = (T)c[cidx(g, i, j, t - 1)], q2 = (T)c[cidx(g, i, j, t - 2)];
+            const T q0 = cv(c[cidx(g, i, j, t)]), q1 = cv(c[cidx(g, i, j, t - 1)]), q2 = cv(c[cidx(g, i, j, t - 2)]);
             return scale * (T(0.125) * (T(15) * q0 - T(10) * q1 + T(3) * q2));
         }
-        return scale * (T)c[cidx(g, i, j, k)];
+        return scale * cv(c[cidx(g, i, j, k)]);
     }
 };
 using VelFP = VelFPT<double>;
@@ -91,6 +102,8 @@ struct CellFOT {
     }
 };
 using CellFO = CellFOT<double>;
+
+#endif
 
 inline unsigned nblocks(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
@@ -151,6 +164,65 @@ __device__ __forceinline__ bool isame_sign(double a, double b) {
 __device__ __forceinline__ double isign(double m, double s) {
     return hiword(m, (__double2hiint(m) & 0x7fffffff) | (__double2hiint(s) & (int)0x80000000));
 }
+// ---- FP32 <-> FP64 on the integer pipe.  A conversion instruction takes an
+// FP64 issue slot (74 cycles of a warp), these about ten integer instructions,
+// and give the same bits: round to nearest even, FP32 subnormals included; a
+// NaN becomes a quiet NaN.  What is not zero or normal in FP32 takes the call.
+// They pay in kernels bound by FP64 issue (Smagorinsky tile on 256x256x128: 388
+// us with conversions, 285 with these); kernels that wait on memory keep the
+// conversion (k_add_f32 37 us against 41, k_adj_edges_gather 573 against 769).
+static __device__ __noinline__ float d2f_rare(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned m = ((hi & 0xfffffu) << 3) | (lo >> 29), r = lo & 0x1fffffffu;
+    const int e = (int)((hi >> 20) & 0x7ffu) - 896;  // biased FP32 exponent
+    unsigned b = 0u;
+    if (e <= 0) {  // FP32 subnormal or zero
+        const int s = 1 - e;
+        const unsigned f = m | 0x800000u;
+        if (s <= 24) {
+            const unsigned q = f >> s, rem = f & ((1u << s) - 1u), half = 1u << (s - 1);
+            b = q + (rem > half || (rem == half && (r || (q & 1u))));
+        }
+    } else {
+        b = e == 1151 && (m | r) ? 0x7fffffffu : 0x7f800000u;
+    }
+    return __uint_as_float((hi & 0x80000000u) | b);
+}
+__device__ __forceinline__ float d2f(double x) {
+    const int h = __double2hiint(x);
+    if ((unsigned)((h & 0x7ff00000) - 0x38100000) >= 0x0fe00000u && ((h & 0x7fffffff) | __double2loint(x)) != 0) return d2f_rare(x);
+    // round at bit 29, then the exponent's bias: its top bit inverted
+    const long long v = dbits(x), q = v + 0x0fffffff + ((v >> 29) & 1);
+    const unsigned t = ((unsigned)(q >> 29) & 0x7fffffffu) ^ 0x40000000u;
+    return __uint_as_float(((h & 0x7fffffff) == 0 ? 0u : t) | ((unsigned)h & 0x80000000u));
+}
+static __device__ __noinline__ double f2d_rare(float x) {
+    const unsigned b = __float_as_uint(x), sign = b & 0x80000000u;
+    unsigned m = b & 0x7fffffu, e = 1151u;
+    if ((b & 0x7f800000u) == 0u) {
+        const int s = __clz((int)m) - 8;  // normalise
+        m = (m << s) & 0x7fffffu;
+        e = 1u - (unsigned)s;
+    }
+    return __hiloint2double((int)(sign | ((e + 896u) << 20) | (m >> 3)), (int)(m << 29));
+}
+__device__ __forceinline__ double f2d(float x) {
+    const unsigned b = __float_as_uint(x), a = b & 0x7fffffffu;
+    if (a - 0x00800000u >= 0x7f000000u && a != 0u) return f2d_rare(x);
+    const unsigned h = ((unsigned)((int)b >> 3) & 0x8fffffffu) + (a == 0u ? 0u : 0x38000000u);
+    return __hiloint2double((int)h, (int)(b << 29));
+}
+template <typename To>
+__device__ __forceinline__ To to(double x) {
+    if constexpr (sizeof(To) == 8) return x;
+    else return d2f(x);
+}
+template <typename To>
+__device__ __forceinline__ To to(float x) {
+    if constexpr (sizeof(To) == 4) return x;
+    else return f2d(x);
+}
+
 // max that keeps a NaN operand (fmax drops it): a non-finite residual or CFL
 // maximum must reach the host's finiteness checks
 __device__ __forceinline__ double nmax(double a, double b) {

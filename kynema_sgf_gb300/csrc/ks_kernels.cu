@@ -203,12 +203,12 @@ __global__ void __launch_bounds__(128) k_smag_col(Grid g, const double* vel, dou
 // instead of the 18 reads of the thread-per-cell form.
 constexpr int SMX = 32, SMY = 4, SMZ = 4;
 constexpr int SMHX = SMX + 2, SMHY = SMY + 2, SMHZ = SMZ + 2, SMNH = SMHX * SMHY * SMHZ;
-__global__ void __launch_bounds__(SMX* SMY* SMZ) k_smag_tile(Grid g, const double* vel, double* mueff, double mu, double rho, double fac,
+__global__ void __launch_bounds__(SMX* SMY* SMZ) k_smag_tile(Grid g, const double* vel, double* mueff, double mu, double rhofac,
                                                             double* alpha, double mu_pr, double iprt) {
     __shared__ float sV[3 * SMNH];
     const int i0 = blockIdx.x * SMX, j0 = blockIdx.y * SMY, k0 = blockIdx.z * SMZ;
     const int tid = threadIdx.x, nthr = SMX * SMY * SMZ;
-    const VelFPT<float, double> V{vel, g, 1.0f};
+    const VelFPT<float, double, true> V{vel, g, 1.0f};
     for (int h = tid; h < SMNH; h += nthr) {
         const int hx = h % SMHX, hy = (h / SMHX) % SMHY, hz = h / (SMHX * SMHY);
         // a tile may be wider than the grid: wrap x, y (and periodic z) fully
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(SMX* SMY* SMZ) k_smag_tile(Grid g, const doubl
     const int i = i0 + tx, j = j0 + ty, k = k0 + tz;
     if (i >= g.nx || j >= g.ny || k >= g.nz) return;
     const int c = ((tz + 1) * SMHY + ty + 1) * SMHX + tx + 1;
-    const float hx = float(0.5 * g.idx), hy = float(0.5 * g.idy);
+    const float hx = 0.5f * d2f(g.idx), hy = 0.5f * d2f(g.idy);
     float gx[3], gy[3], gz[3];
     for (int n = 0; n < 3; ++n) {
         const float* v = sV + n * SMNH + c;
@@ -232,13 +232,13 @@ __global__ void __launch_bounds__(SMX* SMY* SMZ) k_smag_tile(Grid g, const doubl
     if (!g.zper && (k == 0 || k == g.nz - 1)) {  // one-sided through the wall (ghost) value
         float a = 1.0f / 3.0f, b = 1.0f, cc = -4.0f / 3.0f;
         if (k == g.nz - 1) { a = 4.0f / 3.0f; b = -1.0f; cc = -1.0f / 3.0f; }
-        const float iz = float(g.idz);
+        const float iz = d2f(g.idz);
         for (int n = 0; n < 3; ++n) {
             const float* v = sV + n * SMNH + c;
             gz[n] = (a * v[SMHX * SMHY] + b * v[0] + cc * v[-SMHX * SMHY]) * iz;
         }
     } else {
-        const float hz = float(0.5 * g.idz);
+        const float hz = 0.5f * d2f(g.idz);
         for (int n = 0; n < 3; ++n) {
             const float* v = sV + n * SMNH + c;
             gz[n] = hz * (v[SMHX * SMHY] - v[-SMHX * SMHY]);
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(SMX* SMY* SMZ) k_smag_tile(Grid g, const doubl
     }
     const float sxy = gy[0] + gx[1], syz = gz[1] + gy[2], szx = gx[2] + gz[0];
     const float s = sqrtf(2.0f * (gx[0] * gx[0] + gy[1] * gy[1] + gz[2] * gz[2]) + (sxy * sxy + syz * syz + szx * szx));
-    const double mut = (rho * fac) * (double)s;
+    const double mut = rhofac * f2d(s);
     const long long t = cidx(g, i, j, k);
     mueff[t] = mu + mut;
     if (alpha) alpha[t] = mu_pr + iprt * mut;
@@ -473,11 +473,13 @@ struct TauEpi {
     double* parts;
     double dt, rho, omega;
     double irho;  // 1 / rho, formed on the host
+    double hdr;   // dt / (2 rho)
 };
 
 // FP32 form (mixed precision, modes 0-2): staged values, face fluxes and their
 // arithmetic are FP32, the FP64 inputs rounded once when staged; the epilogue
 // runs in FP64.
+template <int MODE>
 __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const double* vel, const double* mueff, const double* wg, double* out,
                                                                TauEpi E) {
     using T = float;
@@ -499,13 +501,13 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
         const int gi = ((i0 + hx - 1) % g.nx + g.nx) % g.nx, gj = ((j0 + hy - 1) % g.ny + g.ny) % g.ny;
         int gk = k0 + hz - 1;
         if (g.zper) gk = (gk % g.nz + g.nz) % g.nz;
-        for (int n = 0; n < 3; ++n) sV[n * TNH + h] = (T)V(n, gi, gj, gk);
+        for (int n = 0; n < 3; ++n) sV[n * TNH + h] = d2f(V(n, gi, gj, gk));
         const int kk = g.zper ? gk : (gk < 0 ? 0 : (gk >= g.nz ? g.nz - 1 : gk));
-        sM[h] = (T)mueff[cidx(g, gi, gj, kk)];
+        sM[h] = d2f(mueff[cidx(g, gi, gj, kk)]);
     }
     __syncthreads();
-    const T ih[3] = {(T)g.idx, (T)g.idy, (T)g.idz};
-    const T qh[3] = {T(0.25 * g.idx), T(0.25 * g.idy), T(0.25 * g.idz)};
+    const T ih[3] = {d2f(g.idx), d2f(g.idy), d2f(g.idz)};
+    const T qh[3] = {T(0.25) * ih[0], T(0.25) * ih[1], T(0.25) * ih[2]};
     // flux through the d-face at the low side of halo cell (hx, hy, hz)
     auto flux = [&](int d, int hx, int hy, int hz, int gk, T F[3]) {
         const int e0 = (d == 0), e1 = (d == 1), e2 = (d == 2);
@@ -555,7 +557,7 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
     const int tx = tid % TTX, ty = (tid / TTX) % TTY, tz = tid / (TTX * TTY);
     const int i = i0 + tx, j = j0 + ty, k = k0 + tz;
     const bool live = i < g.nx && j < g.ny && k < g.nz;
-    const double dt = E.dt, irho = E.irho;
+    const double irho = E.irho, hdr = E.hdr;
     const long long N = g.N, t = live ? cidx(g, i, j, k) : 0;
     for (int n = 0; n < 3 && live; ++n) {
         const int ax = (tz * TTY + ty) * (TTX + 1) + tx;
@@ -564,15 +566,15 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
         T acc_t = (sFx[n * TNFX + ax + 1] - sFx[n * TNFX + ax]) * ih[0];
         acc_t += (sFy[n * TNFY + ay + TTX] - sFy[n * TNFY + ay]) * ih[1];
         acc_t += (sFz[n * TNFZ + az + TTX * TTY] - sFz[n * TNFZ + az]) * ih[2];
-        const double acc = (double)acc_t;
+        const double acc = f2d(acc_t);
         const long long m = n * N + t;
-        if (E.mode == 0) {
+        if constexpr (MODE == 0) {
             out[m] = acc;
-        } else if (E.mode == 1) {
+        } else if constexpr (MODE == 1) {
             out[m] = acc;
             E.forces[m] = (E.src[m] + acc) * irho;
         } else {
-            out[m] = E.base[m] + 0.5 * dt * (acc - E.dold[m]) * irho;
+            out[m] = E.base[m] + hdr * (acc - E.dold[m]);
         }
     }
 }
@@ -726,7 +728,6 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
     const bool live = mainw && i < g.nx && j < g.ny;
     const int sr = l & 15, sx = l < 16 ? 0 : 33;  // the side warp's row and column
     const bool side = w == TY + 2 && sr < TY;
-    const double hdr = 0.5 * E.dt * E.irho;
     long long rmax = 0;
     for (int k = k0; k < k1; ++k) {
         const int m = k & 1;
@@ -784,7 +785,7 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
                     out[o] = acc;
                     E.forces[o] = (E.src[o] + acc) * E.irho;
                 } else if constexpr (MODE == 2) {
-                    out[o] = E.base[o] + hdr * (acc - E.dold[o]);
+                    out[o] = E.base[o] + E.hdr * (acc - E.dold[o]);
                 } else if constexpr (MODE == 3) {
                     out[o] = (E.rho * E.base[o] + E.dt * (0.5 * (E.conv_o[o] + E.conv_n[o]) + 0.5 * E.dold[o] + 0.5 * acc + E.src[o])) * E.irho;
                 } else {
@@ -1265,7 +1266,7 @@ void launch_smagorinsky(Ctx& c, const Grid& g, const double* vel, double* mueff,
     const double bytes = B8 * ((s.smag ? 4 : 1) + (alpha ? 1 : 0)) * g.N;
     if (fp32 && s.smag) {
         const dim3 grid((g.nx + SMX - 1) / SMX, (g.ny + SMY - 1) / SMY, (g.nz + SMZ - 1) / SMZ);
-        KS_LAUNCH(c, k_smag_tile, grid, SMX * SMY * SMZ, bytes, g, vel, mueff, s.mu, s.rho, s.smag_fac, alpha, s.mu_pr, s.iprt);
+        KS_LAUNCH(c, k_smag_tile, grid, SMX * SMY * SMZ, bytes, g, vel, mueff, s.mu, s.rho * s.smag_fac, alpha, s.mu_pr, s.iprt);
     } else if (fp32)
         KS_LAUNCH(c, k_smag<float>, nblocks(g.N, BS), BS, bytes, g, vel, mueff, s.mu, s.rho, s.smag_fac, s.smag, alpha, s.mu_pr, s.iprt);
     else if (s.smag) {
@@ -1356,17 +1357,18 @@ static_assert(sizeof(TauPlanes<4>) <= 48 * 1024, "needs no shared memory attribu
 void launch_divtau(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, int mode,
                    const double* src, double* forces, const double* base, const double* dold, double dt, double rho, int fp32) {
     const double per_cell = 4 + 3 + (mode == 1 ? 6 : 0) + (mode == 2 ? 6 : 0);
-    TauEpi E{mode, src, base, dold, nullptr, nullptr, nullptr, forces, nullptr, dt, rho, 0.0, 1.0 / rho};
+    TauEpi E{mode, src, base, dold, nullptr, nullptr, nullptr, forces, nullptr, dt, rho, 0.0, 1.0 / rho, 0.5 * dt / rho};
     if (fp32) {
         const dim3 grid((g.nx + TTX - 1) / TTX, (g.ny + TTY - 1) / TTY, (g.nz + TTZ - 1) / TTZ);
-        KS_LAUNCH_SMEM(c, k_divtau_tile, grid, TTX * TTY * TTZ, tau_smem(), B8 * per_cell * g.N, g, vel, mueff, wg, out, E);
+        const auto run = mode == 0 ? k_divtau_tile<0> : (mode == 1 ? k_divtau_tile<1> : k_divtau_tile<2>);
+        KS_LAUNCH_SMEM_NAMED(c, "k_divtau_tile", run, grid, TTX * TTY * TTZ, tau_smem(), B8 * per_cell * g.N, g, vel, mueff, wg, out, E);
     } else {
         launch_divtau_col(c, g, vel, mueff, wg, out, E, B8 * per_cell * g.N);
     }
 }
 void launch_divtau_corrector(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, const double* vel_old,
                              const double* conv_old, const double* conv_new, const double* dold, const double* src, double dt, double rho) {
-    TauEpi E{3, src, vel_old, dold, conv_old, conv_new, nullptr, nullptr, nullptr, dt, rho, 0.0, 1.0 / rho};
+    TauEpi E{3, src, vel_old, dold, conv_old, conv_new, nullptr, nullptr, nullptr, dt, rho, 0.0, 1.0 / rho, 0.5 * dt / rho};
     launch_divtau_col(c, g, vel, mueff, wg, out, E, B8 * 22.0 * g.N);
 }
 int divtau_blocks(const Grid& g) {
@@ -1375,7 +1377,7 @@ int divtau_blocks(const Grid& g) {
 }
 void launch_divtau_jacobi(Ctx& c, const Grid& g, const double* x, const double* mueff, const double* wg, const double* b, const double* dinv,
                           double* out, double rho, double dtd, double omega, double* parts) {
-    TauEpi E{omega > 0.0 ? 7 : 8, nullptr, b, nullptr, nullptr, nullptr, dinv, nullptr, parts, dtd, rho, omega, 1.0 / rho};
+    TauEpi E{omega > 0.0 ? 7 : 8, nullptr, b, nullptr, nullptr, nullptr, dinv, nullptr, parts, dtd, rho, omega, 1.0 / rho, 0.5 * dtd / rho};
     launch_divtau_col(c, g, x, mueff, wg, out, E, B8 * ((omega > 0.0 ? 13.0 : 10.0) * g.N));
 }
 void launch_predictor_rhs(Ctx& c, const Grid& g, const double* vo, const double* conv, const double* src, const double* dtau, double* vel,

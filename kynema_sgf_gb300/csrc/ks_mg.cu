@@ -271,7 +271,7 @@ __global__ void k_cc_resid(CCLevelT<T> L, CCCoef<T> w, int kc, double* parts, fl
             const T v = cur.r - dg * (cur.pc - S);
             cur = nxt;
             if constexpr (TO32) {
-                r32[c] = (float)v;
+                r32[c] = d2f(v);
                 z32[c] = 0.0f;
             } else {
                 L.res[c] = v;
@@ -511,7 +511,7 @@ __global__ void k_nd_col(NDLevelT<T> L, NdCoef<T> w, const T* in, T* out, int kc
                 res = w.c4 * (Cm + Cp) + res;
             }
             if constexpr (MODE == 3) {
-                r32[idx] = (float)res;
+                r32[idx] = d2f(res);
                 z32[idx] = 0.0f;
             } else if constexpr (MODE == 2) {
                 L.res[idx] = res;
@@ -998,7 +998,7 @@ __global__ void k_nd_zero_start(const double* rhs, long long n, double oinv, dou
         mx.add(r);
         if (out) out[t] = oinv * r;
         if (r32) {
-            r32[t] = (float)r;
+            r32[t] = d2f(r);
             z32[t] = 0.0f;
         }
     }
