@@ -33,7 +33,7 @@ __device__ inline void block_max_to(double v, double* out) {
 // tangential components' is fixed (Neumann data), so they carry weight 2 and 0.
 // Also the block maxima of s = 1 - rho / D (off-diagonal weight of a row: the
 // Jacobi iteration contracts by about s per sweep).
-__global__ void k_diff_dinv(Grid g, const double* mu, double rho, double dtd, double* dinv, double* parts) {
+__global__ void k_diff_dinv(Grid g, const double* mu, double rho, double dtd, double* dinv, double* parts, double hx, double hy, double hz) {
     const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const bool live = t0 < g.N;
     const long long t = live ? t0 : 0;
@@ -41,18 +41,20 @@ __global__ void k_diff_dinv(Grid g, const double* mu, double rho, double dtd, do
     const int i = (int)(u - r * (unsigned)g.nx);
     const int k = (int)(r / (unsigned)g.ny), j = (int)(r - (unsigned)k * (unsigned)g.ny);
     const double c0 = mu[t];
-    const double mx = 0.5 * (mu[cidx(g, wrapn(i - 1, g.nx), j, k)] + c0) + 0.5 * (mu[cidx(g, wrapn(i + 1, g.nx), j, k)] + c0);
-    const double my = 0.5 * (mu[cidx(g, i, wrapn(j - 1, g.ny), k)] + c0) + 0.5 * (mu[cidx(g, i, wrapn(j + 1, g.ny), k)] + c0);
+    // sums over a direction's two faces, in units of 1 / (2 h^2); the direction's
+    // own component adds a third, and z walls carry the weights above
+    const double mx = (mu[cidx(g, wrapn(i - 1, g.nx), j, k)] + mu[cidx(g, wrapn(i + 1, g.nx), j, k)]) + 2.0 * c0;
+    const double my = (mu[cidx(g, i, wrapn(j - 1, g.ny), k)] + mu[cidx(g, i, wrapn(j + 1, g.ny), k)]) + 2.0 * c0;
     const bool wlo = !g.zper && k == 0, whi = !g.zper && k == g.nz - 1;
-    const double zlo = wlo ? c0 : 0.5 * (mu[cidx(g, i, j, g.zper ? wrapn(k - 1, g.nz) : k - 1)] + c0);
-    const double zhi = whi ? c0 : 0.5 * (mu[cidx(g, i, j, g.zper ? wrapn(k + 1, g.nz) : k + 1)] + c0);
-    const double ix2 = g.idx * g.idx, iy2 = g.idy * g.idy, iz2 = g.idz * g.idz;
+    const double zlo = mu[cidx(g, i, j, wlo ? k : (g.zper ? wrapn(k - 1, g.nz) : k - 1))] + c0;
+    const double zhi = mu[cidx(g, i, j, whi ? k : (g.zper ? wrapn(k + 1, g.nz) : k + 1))] + c0;
+    const double mz = (wlo ? 0.0 : zlo) + (whi ? 0.0 : zhi);                          // tangential components
+    const double nz = wlo || whi ? (wlo ? 2.0 * zlo : zlo) + (whi ? 2.0 * zhi : zhi) : mz;  // the normal one
+    const double X = hx * mx, Y = hy * my, XY = X + Y, S = XY + hz * mz;
+    const double sn[3] = {S + (1.0 / 3.0) * X, S + (1.0 / 3.0) * Y, XY + (4.0 / 3.0 * hz) * nz};
     double smax = 0.0;
     for (int n = 0; n < 3 && live; ++n) {
-        const double w = n == 2 ? 2.0 : 0.0;
-        const double sz = (wlo ? w * zlo : zlo) + (whi ? w * zhi : zhi);
-        const double s = (n == 0 ? 4.0 / 3.0 : 1.0) * mx * ix2 + (n == 1 ? 4.0 / 3.0 : 1.0) * my * iy2 + (n == 2 ? 4.0 / 3.0 : 1.0) * sz * iz2;
-        const double d = 1.0 / (rho + dtd * s);
+        const double d = 1.0 / (rho + dtd * sn[n]);
         dinv[n * g.N + t] = d;
         smax = nmax(smax, 1.0 - rho * d);
     }
@@ -93,7 +95,7 @@ __global__ void k_rhs_b(Grid g, const double* u, double rho, double* b, double* 
         for (int n = 0; n < 3; ++n) {
             const double v = rho * u[n * g.N + t];
             b[n * g.N + t] = v;
-            m = nmax(m, fabs(v));
+            m = nmax(m, iabs(v));
         }
     block_max_to(m, parts + blockIdx.x);
 }
@@ -102,7 +104,8 @@ __global__ void k_rhs_b(Grid g, const double* u, double rho, double* b, double* 
 
 int diff_cell_blocks(const Grid& g) { return (int)nblocks(g.N, BS); }
 void launch_diff_dinv(Ctx& c, const Grid& g, const double* mueff, double rho, double dtd, double* dinv, double* parts) {
-    KS_LAUNCH(c, k_diff_dinv, nblocks(g.N, BS), BS, 8.0 * 4.0 * g.N, g, mueff, rho, dtd, dinv, parts);
+    KS_LAUNCH(c, k_diff_dinv, nblocks(g.N, BS), BS, 8.0 * 4.0 * g.N, g, mueff, rho, dtd, dinv, parts, 0.5 * g.idx * g.idx,
+              0.5 * g.idy * g.idy, 0.5 * g.idz * g.idz);
 }
 void launch_avg8(Ctx& c, const Grid& fine, const Grid& coarse, const double* f, double* cr, int ncomp) {
     KS_LAUNCH(c, k_avg8, nblocks(coarse.N, BS), BS, 8.0 * ncomp * (fine.N + coarse.N), fine, coarse, f, cr, ncomp);

@@ -25,6 +25,7 @@
 // memory directly, the passes between exchange through shared memory.
 #include <algorithm>
 
+#include "ks_decide.cuh"
 #include "ks_launch.hpp"
 
 namespace ks {
@@ -264,49 +265,57 @@ __global__ void k_modes_setup(SpectralZ Z) {
     Z.schur[t] = t == 0 ? 0.0 : 1.0 / (d + e * (Z.w[t] + Z.w[(long long)(nu - 1) * M + t]));
 }
 
-// The z systems of all modes, in place on the transformed plane pairs C.  A
-// thread marches its column up (elimination) and down (substitution), kAhead
-// pairs at a time whose loads were issued a group earlier: a box has few modes
-// (2080 on 64^3), so the march is a chain of loads unless several are in
-// flight (64^3: 66 us with one pair ahead, 56 with four).  The coefficients of
+// The z systems of all modes, in place on the transformed plane pairs C: the
+// elimination marches a column up, the substitution down.  The coefficients of
 // the real planes 2m and 2m + 1 are
 //   A = (C + conj C~) / 2,   B = (C - conj C~) / 2i,
 // C~ the entry of the opposite mode (the factor 1/2 is left to the output's
 // scale); on the way up the pair's two slots hold the eliminated A and B.
+//
+// A box has few modes (2080 on 64^3), each a serial chain whose length is its
+// FP64 instructions, so two neighbouring lanes share a mode: the systems of the
+// real and the imaginary parts are independent.  Lane part 0 holds (Re A, Re B),
+// part 1 (Im A, Im B), and they exchange B where C is merged again.  kAhead
+// pairs are loaded a group before they are used, and the column's kind is a
+// template argument (a branch not taken costs its FP64 issue slots):
+// a solve on 64^3 66 -> 40 us, 32^3 30 -> 20, 128x128x64 52 -> 30, 256x256x128
+// 131 -> 108.
 constexpr int kAhead = 4;
-__global__ void __launch_bounds__(128) k_modes_z(SpectralZ Z, double2* C) {
-    const int kx = blockIdx.x * blockDim.x + threadIdx.x, ky = blockIdx.y;
-    if (kx >= Z.nx) return;
+template <int NODAL, int ZPER>
+__global__ void __launch_bounds__(64) k_modes_z(SpectralZ Z, double2* C) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, kx = t >> 1, part = t & 1, ky = blockIdx.y;
     const int ox = kx == 0 ? 0 : Z.nx - kx, oy = ky == 0 ? 0 : Z.ny - ky;
-    if (oy == ky && kx > ox) return;  // the other half of a self-conjugate row
+    // the pairs of a warp stay together to its end (the exchange below): lanes
+    // past the row, and on the other half of a self-conjugate row, idle
+    const bool live = kx < Z.nx && !(oy == ky && kx > ox);
+    if (!__any_sync(0xffffffffu, live)) return;
     const bool self = oy == ky && ox == kx;
-    const int ax = min(kx, Z.nx - kx), na = Z.nx / 2 + 1, M = na * (Z.ny / 2 + 1), md = ky * na + ax;
+    const int ax = live ? min(kx, Z.nx - kx) : 0, na = Z.nx / 2 + 1, M = na * (Z.ny / 2 + 1), md = ky * na + ax;
     const long long plane = (long long)Z.nx * Z.ny;
-    const int nz = Z.nz, np = (nz + 1) / 2;
-    double2* c = C + (long long)ky * Z.nx + kx;
-    double2* o = C + (long long)oy * Z.nx + ox;
+    const int nz = Z.nz, np = (nz + 1) / 2, nu = ZPER ? nz - 1 : nz;
+    double2* c = C + (long long)ky * Z.nx + (live ? kx : 0);
+    double2* o = C + (long long)oy * Z.nx + (live ? ox : 0);
     double d, e;
     mode_coef(Z, ax, ky, d, e);
     const double* dinv = Z.dinv + md;
-    auto sep = [](double2 p, double2 q, double2& A, double2& B) {
-        A = make_double2(p.x + q.x, p.y - q.y);
-        B = make_double2(p.y + q.y, q.x - p.x);
+    // the lane's part of A and B from the entries p of the mode and q of its opposite
+    auto sep = [&](double2 p, double2 q, double& a, double& b) {
+        a = (part ? p.y : p.x) + (part ? ineg(q.y) : q.x);
+        b = (part ? q.x : p.y) + (part ? ineg(p.x) : q.y);
     };
-    double2 last = make_double2(0.0, 0.0);  // cyclic: the eliminated unknown x(nz - 1)
-    const int nu = Z.zper ? nz - 1 : nz;
-    if (Z.zper) {
+    double last = 0.0;  // cyclic: the eliminated unknown x(nz - 1)
+    if (ZPER && live) {
         const double* w = Z.w + md;
-        double2 s = make_double2(0.0, 0.0);
+        double s = 0.0;
 #pragma unroll 4
         for (int m = 0; m < np; ++m) {
-            double2 A, B;
-            sep(c[m * plane], o[m * plane], A, B);
-            const double w0 = w[(long long)(2 * m) * M], w1 = 2 * m + 1 < nu ? w[(long long)(2 * m + 1) * M] : 1.0;
-            s = make_double2(fma(w0, A.x, s.x), fma(w0, A.y, s.y));
-            s = make_double2(fma(w1, B.x, s.x), fma(w1, B.y, s.y));
+            double a, b;
+            sep(c[m * plane], o[m * plane], a, b);
+            const double w0 = 2 * m < nu ? w[(long long)(2 * m) * M] : 1.0, w1 = 2 * m + 1 < nu ? w[(long long)(2 * m + 1) * M] : 1.0;
+            s = fma(w0, a, s);
+            s = fma(w1, b, s);
         }
-        const double q = Z.schur[md];
-        last = make_double2(q * s.x, q * s.y);
+        last = Z.schur[md] * s;
     }
     struct Pair {
         double2 p, q;
@@ -314,7 +323,7 @@ __global__ void __launch_bounds__(128) k_modes_z(SpectralZ Z, double2* C) {
     };
     auto load = [&](int m) {
         Pair r{};
-        if (m < 0 || m >= np) return r;
+        if (!live || m < 0 || m >= np) return r;
         r.p = c[m * plane];
         r.q = o[m * plane];
         r.da = dinv[(long long)(2 * m) * M];
@@ -322,74 +331,105 @@ __global__ void __launch_bounds__(128) k_modes_z(SpectralZ Z, double2* C) {
         return r;
     };
     // up: z_k = b_k - e dinv_{k-1} z_{k-1}
-    double2 z = make_double2(0.0, 0.0);
-    double di = 0.0;
+    double z = 0.0, di = 0.0;
     Pair cur[kAhead], nxt[kAhead];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) cur[u] = load(u);
     for (int m0 = 0; m0 < np; m0 += kAhead) {
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) nxt[u] = load(m0 + kAhead + u);
+        __syncwarp();  // both lanes of a mode have read what one of them overwrites
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
             const int m = m0 + u, k = 2 * m;
             if (m >= np) break;
-            double2 A, B;
-            sep(cur[u].p, cur[u].q, A, B);
-            if (Z.nodal && !Z.zper) {
-                if (k == 0 || k == nz - 1) A = make_double2(0.5 * A.x, 0.5 * A.y);
-                if (k + 1 == nz - 1) B = make_double2(0.5 * B.x, 0.5 * B.y);
+            double a, b;
+            sep(cur[u].p, cur[u].q, a, b);
+            if (NODAL && !ZPER) {  // the mirrored end rows are halved
+                a = k == 0 || k == nz - 1 ? half_of(a) : a;
+                b = k + 1 == nz - 1 ? half_of(b) : b;
             }
-            if (Z.zper) {
-                if (k == 0) A = make_double2(fma(-e, last.x, A.x), fma(-e, last.y, A.y));
-                if (k == nu - 1) A = make_double2(fma(-e, last.x, A.x), fma(-e, last.y, A.y));
+            if (ZPER && (m == 0 || m >= np - 2)) {  // first and last row
+                if (k == 0) a = fma(-e, last, a);
+                if (k == nu - 1) a = fma(-e, last, a);
+                if (k + 1 == nu - 1) b = fma(-e, last, b);
             }
-            double l = -e * di;
-            A = make_double2(fma(l, z.x, A.x), fma(l, z.y, A.y));
-            l = -e * cur[u].da;
-            B = make_double2(fma(l, A.x, B.x), fma(l, A.y, B.y));
-            if (self) {  // both planes' coefficients are real here: one slot holds them
-                c[m * plane] = make_double2(A.x, B.x);
-            } else {
-                c[m * plane] = A;
-                o[m * plane] = B;
+            a = fma(-e * di, z, a);
+            b = fma(-e * cur[u].da, a, b);
+            if (live) {
+                double* cc = reinterpret_cast<double*>(c + m * plane);
+                double* oo = reinterpret_cast<double*>(o + m * plane);
+                if (self) {  // both planes' coefficients are real: part 0 keeps them in one slot
+                    if (part == 0) {
+                        cc[0] = a;
+                        cc[1] = b;
+                    }
+                } else {
+                    cc[part] = a;
+                    oo[part] = b;
+                }
             }
-            z = B;
+            z = b;
             di = cur[u].db;
         }
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) cur[u] = nxt[u];
     }
     // down: x_k = dinv_k z_k - e dinv_k x_{k+1}, and C = A + i B, C~ = conj A + i conj B
-    double2 x = make_double2(0.0, 0.0);
+    double x = 0.0;
+    struct Row {
+        double a, b, da, db;
+    };
+    auto down = [&](int m) {
+        Row r{};
+        if (!live || m < 0) return r;
+        const double* cc = reinterpret_cast<const double*>(c + m * plane);
+        const double* oo = reinterpret_cast<const double*>(o + m * plane);
+        if (self) {
+            r.a = part == 0 ? cc[0] : 0.0;
+            r.b = part == 0 ? cc[1] : 0.0;
+        } else {
+            r.a = cc[part];
+            r.b = oo[part];
+        }
+        r.da = dinv[(long long)(2 * m) * M];
+        r.db = 2 * m + 1 < nu ? dinv[(long long)(2 * m + 1) * M] : 0.0;
+        return r;
+    };
+    Row rc[kAhead], rn[kAhead];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) cur[u] = load(np - 1 - u);
+    for (int u = 0; u < kAhead; ++u) rc[u] = down(np - 1 - u);
     for (int m0 = np - 1; m0 >= 0; m0 -= kAhead) {
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) nxt[u] = load(m0 - kAhead - u);
+        for (int u = 0; u < kAhead; ++u) rn[u] = down(m0 - kAhead - u);
+        __syncwarp();
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
             const int m = m0 - u, k = 2 * m;
             if (m < 0) break;
-            const double2 p = cur[u].p, q = cur[u].q;
-            double2 A = self ? make_double2(p.x, 0.0) : p, B = self ? make_double2(p.y, 0.0) : q;
+            double a = rc[u].a, b = rc[u].b;
             if (k + 1 < nu) {
-                const double db = cur[u].db, cb = -e * db;
-                B = make_double2(fma(cb, x.x, db * B.x), fma(cb, x.y, db * B.y));
-                x = B;
-            } else if (k + 1 < nz) {
-                B = last;  // cyclic: already folded into rows 0 and nz - 2
+                b = rc[u].db * fma(-e, x, b);
+                x = b;
             } else {
-                B = make_double2(0.0, 0.0);  // past the last node plane
+                b = ZPER && k + 1 < nz ? last : 0.0;  // folded into rows 0 and nz - 2; past the last node plane
             }
-            const double da = cur[u].da, ca = -e * da;
-            A = make_double2(fma(ca, x.x, da * A.x), fma(ca, x.y, da * A.y));
-            x = A;
-            c[m * plane] = make_double2(A.x - B.y, A.y + B.x);
-            if (!self) o[m * plane] = make_double2(A.x + B.y, B.x - A.y);
+            if (!ZPER || k < nu) {
+                a = rc[u].da * fma(-e, x, a);
+                x = a;
+            } else {
+                a = last;
+            }
+            const double y = __shfl_xor_sync(0xffffffffu, b, 1);
+            if (live) {
+                double* cc = reinterpret_cast<double*>(c + m * plane);
+                double* oo = reinterpret_cast<double*>(o + m * plane);
+                cc[part] = a + (part ? y : ineg(y));
+                if (!self) oo[part] = y + (part ? ineg(a) : a);
+            }
         }
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) cur[u] = nxt[u];
+        for (int u = 0; u < kAhead; ++u) rc[u] = rn[u];
     }
 }
 
@@ -449,8 +489,9 @@ void launch_spectral_solve(Ctx& c, const SpectralZ& Z, const double2* tw_x, cons
     const int tiles = (Z.nx + ly - 1) / ly, gx = (rows + lx - 1) / lx;
     KS_LAUNCH_SMEM(c, k_fft_x<false>, gx, 128, sx, 8.0 * pts + cb, X, Z.ny, Z.nz, rows, lx, rhs, C, (double*)nullptr, 1.0);
     KS_LAUNCH_SMEM(c, k_fft_y, np * tiles, 128, sy, 2.0 * cb, Y, Z.nx, tiles, ly, C, 0);
-    const dim3 gz((unsigned)((Z.nx + 127) / 128), (unsigned)(Z.ny / 2 + 1));
-    KS_LAUNCH(c, k_modes_z, gz, 128, 4.0 * cb + 8.0 * 2.0 * (Z.nx / 2 + 1) * (Z.ny / 2 + 1) * Z.nz, Z, C);
+    const dim3 gz((unsigned)((2 * Z.nx + 63) / 64), (unsigned)(Z.ny / 2 + 1));
+    const auto modes = Z.nodal ? (Z.zper ? k_modes_z<1, 1> : k_modes_z<1, 0>) : (Z.zper ? k_modes_z<0, 1> : k_modes_z<0, 0>);
+    KS_LAUNCH_NAMED(c, "k_modes_z", modes, gz, 64, 4.0 * cb + 8.0 * 2.0 * (Z.nx / 2 + 1) * (Z.ny / 2 + 1) * Z.nz, Z, C);
     KS_LAUNCH_SMEM(c, k_fft_y, np * tiles, 128, sy, 2.0 * cb, Y, Z.nx, tiles, ly, C, 1);
     KS_LAUNCH_SMEM(c, k_fft_x<true>, gx, 128, sx, 8.0 * pts + cb, X, Z.ny, Z.nz, rows, lx, (const double*)nullptr, C, phi, scale);
 }

@@ -100,82 +100,87 @@ __global__ void k_theta_wall_grad(Grid g, const double* vel, const double* theta
 
 struct TdiffArgs {
     ScalarBC bc;
-    int mode;
     const double *base, *dold, *b, *dinv;
     double* parts;
     double dt, rho, omega;
+    double hdr;         // dt / (2 rho)
+    double hx, hy, hz;  // 1 / (2 h^2)
+    double top;         // offset of the ghost value above a z-hi wall
 };
 
-// face diffusivity: mean of the two cells, the cell value on a z wall
+// The cell's neighbours along z with the boundary data folded in: across a wall
+// face the gradient gw gives the value q0 -+ gw dz at the cell's diffusivity.
+__device__ inline void z_side(const Grid& g, const double* th, const double* al, int i, int j, int k, bool high, double q0, double a0, double wall,
+                              double& q, double& a) {
+    const int kk = high ? k + 1 : k - 1;
+    if (!g.zper && (kk < 0 || kk >= g.nz)) {
+        q = q0 + wall;
+        a = a0;
+        return;
+    }
+    const long long z = cidx(g, i, j, g.zper ? wrapn(kk, g.nz) : kk);
+    q = th[z];
+    a = al[z];
+}
+
+// div(alpha grad theta) = sum_d (1 / 2h^2) [(a+ + a0) (q+ - q0) + (a- + a0) (q- - q0)]
+// and MODE's epilogue, face diffusivity the mean of the two cells (the cell
+// value on a z wall).  24 FP64 instructions a cell and the epilogue's; with a
+// half, a difference and a spacing formed for each of six fluxes and every
+// boundary form and mode predicated off, about 75 (96^3: 100 us, 50 now).
+template <int MODE>
 __global__ void k_tdiff(Grid g, const double* th, const double* al, double* out, TdiffArgs A) {
     const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const bool live = t0 < g.N;
     const long long t = live ? t0 : 0;
-    const int i = (int)(t % g.nx);
-    const long long r = t / g.nx;
-    const int j = (int)(r % g.ny), k = (int)(r / g.ny);
+    const unsigned u = (unsigned)t, r = u / (unsigned)g.nx;
+    const int i = (int)(u - r * (unsigned)g.nx);
+    const int k = (int)(r / (unsigned)g.ny), j = (int)(r - (unsigned)k * (unsigned)g.ny);
     const double q0 = th[t], a0 = al[t];
     const long long xm = cidx(g, wrapn(i - 1, g.nx), j, k), xp = cidx(g, wrapn(i + 1, g.nx), j, k);
     const long long ym = cidx(g, i, wrapn(j - 1, g.ny), k), yp = cidx(g, i, wrapn(j + 1, g.ny), k);
-    const double fxl = 0.5 * (al[xm] + a0) * (q0 - th[xm]) * g.idx, fxh = 0.5 * (a0 + al[xp]) * (th[xp] - q0) * g.idx;
-    const double fyl = 0.5 * (al[ym] + a0) * (q0 - th[ym]) * g.idy, fyh = 0.5 * (a0 + al[yp]) * (th[yp] - q0) * g.idy;
-    double fzl, fzh;
-    if (g.zper) {
-        const long long zm = cidx(g, i, j, wrapn(k - 1, g.nz)), zp = cidx(g, i, j, wrapn(k + 1, g.nz));
-        fzl = 0.5 * (al[zm] + a0) * (q0 - th[zm]) * g.idz;
-        fzh = 0.5 * (a0 + al[zp]) * (th[zp] - q0) * g.idz;
-    } else {
-        if (k == 0) {
-            const double gw = A.bc.zlo == 1 ? A.bc.gz[(long long)j * g.nx + i] : 0.0;
-            const double ghost = q0 - gw * g.dz;
-            fzl = a0 * (q0 - ghost) * g.idz;
-        } else {
-            const long long zm = cidx(g, i, j, k - 1);
-            fzl = 0.5 * (al[zm] + a0) * (q0 - th[zm]) * g.idz;
-        }
-        if (k == g.nz - 1) {
-            const double ghost = q0 + (A.bc.zhi == 2 ? A.bc.gtop : 0.0) * g.dz;
-            fzh = a0 * (ghost - q0) * g.idz;
-        } else {
-            const long long zp = cidx(g, i, j, k + 1);
-            fzh = 0.5 * (a0 + al[zp]) * (th[zp] - q0) * g.idz;
-        }
-    }
-    const double acc = (fxh - fxl) * g.idx + (fyh - fyl) * g.idy + (fzh - fzl) * g.idz;
+    double wl = 0.0, wh = 0.0;  // the ghost values' offsets: - gz dz below, + gtop dz above
+    if (!g.zper && k == 0 && A.bc.zlo == 1) wl = -A.bc.gz[(long long)j * g.nx + i] * g.dz;
+    if (!g.zper && k == g.nz - 1) wh = A.top;
+    double qm, am, qp, ap;
+    z_side(g, th, al, i, j, k, false, q0, a0, wl, qm, am);
+    z_side(g, th, al, i, j, k, true, q0, a0, wh, qp, ap);
+    const double X = (al[xp] + a0) * (th[xp] - q0) + (al[xm] + a0) * (th[xm] - q0);
+    const double Y = (al[yp] + a0) * (th[yp] - q0) + (al[ym] + a0) * (th[ym] - q0);
+    const double Zs = (ap + a0) * (qp - q0) + (am + a0) * (qm - q0);
+    const double acc = A.hx * X + (A.hy * Y + A.hz * Zs);
     double rmax = 0.0;
     if (live) {
-        if (A.mode == 0) {
+        if constexpr (MODE == 0) {
             out[t] = acc;
-        } else if (A.mode == 2) {
-            out[t] = A.base[t] + 0.5 * A.dt * (acc - A.dold[t]) / A.rho;
+        } else if constexpr (MODE == 2) {
+            out[t] = A.base[t] + A.hdr * (acc - A.dold[t]);
         } else {
             const double res = A.b[t] - A.rho * q0 + A.dt * acc;
-            rmax = fabs(res);
-            out[t] = A.mode == 7 ? q0 + A.omega * A.dinv[t] * res : res;
+            rmax = iabs(res);
+            out[t] = MODE == 7 ? q0 + A.omega * A.dinv[t] * res : res;
         }
     }
-    if (A.parts) block_max(rmax, A.parts + blockIdx.x);
+    if constexpr (MODE >= 7) {
+        if (A.parts) block_max(rmax, A.parts + blockIdx.x);
+    }
 }
 
-__global__ void k_tdiff_dinv(Grid g, const double* al, double rho, double dtd, double* dinv, double* parts) {
+__global__ void k_tdiff_dinv(Grid g, const double* al, double rho, double dtd, double* dinv, double* parts, double hx, double hy, double hz) {
     const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const bool live = t0 < g.N;
     const long long t = live ? t0 : 0;
-    const int i = (int)(t % g.nx);
-    const long long r = t / g.nx;
-    const int j = (int)(r % g.ny), k = (int)(r / g.ny);
-    const double a0 = al[t];
-    double s = (0.5 * (al[cidx(g, wrapn(i - 1, g.nx), j, k)] + a0) + 0.5 * (al[cidx(g, wrapn(i + 1, g.nx), j, k)] + a0)) * g.idx * g.idx +
-               (0.5 * (al[cidx(g, i, wrapn(j - 1, g.ny), k)] + a0) + 0.5 * (al[cidx(g, i, wrapn(j + 1, g.ny), k)] + a0)) * g.idy * g.idy;
-    double zl, zh;
-    if (g.zper) {
-        zl = 0.5 * (al[cidx(g, i, j, wrapn(k - 1, g.nz))] + a0);
-        zh = 0.5 * (al[cidx(g, i, j, wrapn(k + 1, g.nz))] + a0);
-    } else {  // the wall faces' gradients are boundary data: no diagonal weight
-        zl = k == 0 ? 0.0 : 0.5 * (al[cidx(g, i, j, k - 1)] + a0);
-        zh = k == g.nz - 1 ? 0.0 : 0.5 * (al[cidx(g, i, j, k + 1)] + a0);
-    }
-    s += (zl + zh) * g.idz * g.idz;
+    const unsigned u = (unsigned)t, r = u / (unsigned)g.nx;
+    const int i = (int)(u - r * (unsigned)g.nx);
+    const int k = (int)(r / (unsigned)g.ny), j = (int)(r - (unsigned)k * (unsigned)g.ny);
+    const double a0 = al[t], a2 = a0 + a0;
+    // the wall faces' gradients are boundary data: no diagonal weight
+    const bool lo = g.zper || k > 0, hi = g.zper || k < g.nz - 1;
+    const double zl = lo ? al[cidx(g, i, j, g.zper ? wrapn(k - 1, g.nz) : k - 1)] : 0.0, zh = hi ? al[cidx(g, i, j, g.zper ? wrapn(k + 1, g.nz) : k + 1)] : 0.0;
+    const double X = (al[cidx(g, wrapn(i - 1, g.nx), j, k)] + al[cidx(g, wrapn(i + 1, g.nx), j, k)]) + a2;
+    const double Y = (al[cidx(g, i, wrapn(j - 1, g.ny), k)] + al[cidx(g, i, wrapn(j + 1, g.ny), k)]) + a2;
+    const double Zs = (zl + zh) + (lo && hi ? a2 : (lo || hi ? a0 : 0.0));
+    const double s = hx * X + (hy * Y + hz * Zs);
     const double d = 1.0 / (rho + dtd * s);
     if (live) dinv[t] = d;
     if (parts) block_max(live ? 1.0 - rho * d : 0.0, parts + blockIdx.x);
@@ -186,7 +191,7 @@ __global__ void k_scalar_rhs(Grid g, const double* th, double rho, double* b, do
     double m = 0.0;
     if (t < g.N) {
         b[t] = rho * th[t];
-        m = fabs(b[t]);
+        m = iabs(b[t]);
     }
     block_max(m, parts + blockIdx.x);
 }
@@ -233,13 +238,16 @@ void launch_theta_wall_grad(Ctx& c, const Grid& g, const double* vel_old, const 
 int tdiff_blocks(const Grid& g) { return (int)nblocks(g.N, BS); }
 void launch_tdiff(Ctx& c, const Grid& g, const double* th, const double* alpha, const ScalarBC& bc, double* out, int mode, const double* base,
                   const double* dold, const double* b, const double* dinv, double* parts, double dt, double rho, double omega) {
-    TdiffArgs A{bc, mode, base, dold, b, dinv, parts, dt, rho, omega};
+    const TdiffArgs A{bc, base, dold, b, dinv, parts, dt, rho, omega, 0.5 * dt / rho, 0.5 * g.idx * g.idx, 0.5 * g.idy * g.idy, 0.5 * g.idz * g.idz,
+                      bc.zhi == 2 ? bc.gtop * g.dz : 0.0};
     const double per = 3.0 + (mode == 2 ? 2.0 : 0.0) + (mode >= 7 ? 1.0 + (mode == 7 ? 1.0 : 0.0) : 0.0);
-    KS_LAUNCH(c, k_tdiff, nblocks(g.N, BS), BS, 8.0 * per * g.N, g, th, alpha, out, A);
+    const auto run = mode == 0 ? k_tdiff<0> : (mode == 2 ? k_tdiff<2> : (mode == 7 ? k_tdiff<7> : k_tdiff<8>));
+    KS_LAUNCH_NAMED(c, "k_tdiff", run, nblocks(g.N, BS), BS, 8.0 * per * g.N, g, th, alpha, out, A);
 }
 void launch_tdiff_dinv(Ctx& c, const Grid& g, const double* alpha, const ScalarBC& bc, double rho, double dtd, double* dinv, double* parts) {
     (void)bc;
-    KS_LAUNCH(c, k_tdiff_dinv, nblocks(g.N, BS), BS, 8.0 * 2.0 * g.N, g, alpha, rho, dtd, dinv, parts);
+    KS_LAUNCH(c, k_tdiff_dinv, nblocks(g.N, BS), BS, 8.0 * 2.0 * g.N, g, alpha, rho, dtd, dinv, parts, 0.5 * g.idx * g.idx, 0.5 * g.idy * g.idy,
+              0.5 * g.idz * g.idz);
 }
 void launch_scalar_rhs(Ctx& c, const Grid& g, const double* th, double rho, double* b, double* parts) {
     KS_LAUNCH(c, k_scalar_rhs, nblocks(g.N, BS), BS, 8.0 * 2.0 * g.N, g, th, rho, b, parts);
