@@ -75,6 +75,11 @@ __device__ inline float vls3(float l, float r, float d) {
     return mag_sign(m, dsc);
 }
 
+// unlimited PPM edge value between cells with values a0, a1 = a0 + l and
+// slopes s0, s1 (before the clip to the two cells)
+__device__ inline double edge_value(double a0, double, double l, double s0, double s1) { return fma(-1.0 / 6.0, s1 - s0, fma(0.5, l, a0)); }
+__device__ inline float edge_value(float a0, float a1, float, float s0, float s1) { return 0.5f * (a0 + a1) - float(1.0 / 6.0) * (s1 - s0); }
+
 #endif
 
 }  // namespace ks

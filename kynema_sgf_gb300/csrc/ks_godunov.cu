@@ -37,13 +37,11 @@ inline long long nfaces(const Grid& g, int d) { return (long long)g.nx * g.ny * 
 // are the same bits as the plain forms; edges and traces differ in their last
 // bit or two.
 //
-// unlimited PPM edge value between cells with values a0, a1 = a0 + l and
-// slopes s0, s1, clipped to the two cells
-__device__ inline double ppm_edge(double a0, double a1, double l, double s0, double s1) {
-    return clip2(fma(-1.0 / 6.0, s1 - s0, fma(0.5, l, a0)), a0, a1);
-}
-__device__ inline float ppm_edge(float a0, float a1, float, float s0, float s1) {
-    return clip2(0.5f * (a0 + a1) - float(1.0 / 6.0) * (s1 - s0), a0, a1);
+// PPM edge value between cells with values a0, a1 = a0 + l and slopes s0, s1,
+// clipped to the two cells
+template <typename T>
+__device__ inline T ppm_edge(T a0, T a1, T l, T s0, T s1) {
+    return clip2(edge_value(a0, a1, l, s0, s1), a0, a1);
 }
 
 // Edge value on the face with index k along d from the cell values
