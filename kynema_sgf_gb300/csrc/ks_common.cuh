@@ -45,45 +45,35 @@ __host__ __device__ inline long long fidx(const Grid& g, int d, int i, int j, in
 }
 
 #ifdef __CUDACC__
-template <typename To>
-__device__ __forceinline__ To to(double x);
-template <typename To>
-__device__ __forceinline__ To to(float x);
-
 // Cell-centred velocity (or rho*velocity) with fill-patch ghost values:
 // periodic wrap in x, y (and z); at walls the tangential components take the
 // high-order extrapolation to the face, (15 q0 - 10 q1 + 3 q2)/8, in every
 // ghost layer and the normal component is 0.  The field is stored as S
 // (FP64, or its FP32 copy in the mixed-precision advection); the value is
 // returned in the arithmetic type T of the caller.
-template <typename T = double, typename S = double, bool INT = false>
+template <typename T = double, typename S = double>
 struct VelFPT {
     const S* v;
     Grid g;
     T scale;
-    // INT: converted on the integer pipe (to, below)
-    static __device__ inline T cv(S x) {
-        if constexpr (INT) return to<T>(x);
-        else return (T)x;
-    }
     __device__ inline T operator()(int n, int i, int j, int k) const {
         i = wrapn(i, g.nx);
         j = wrapn(j, g.ny);
         const long long N = g.N;
         const S* c = v + n * N;
-        if (g.zper) return scale * cv(c[cidx(g, i, j, wrapn(k, g.nz))]);
+        if (g.zper) return scale * (T)(c[cidx(g, i, j, wrapn(k, g.nz))]);
         if (k < 0) {
             if (n == 2) return T(0);
-            const T q0 = cv(c[cidx(g, i, j, 0)]), q1 = cv(c[cidx(g, i, j, 1)]), q2 = cv(c[cidx(g, i, j, 2)]);
+            const T q0 = (T)(c[cidx(g, i, j, 0)]), q1 = (T)(c[cidx(g, i, j, 1)]), q2 = (T)(c[cidx(g, i, j, 2)]);
             return scale * (T(0.125) * (T(15) * q0 - T(10) * q1 + T(3) * q2));
         }
         if (k >= g.nz) {
             if (n == 2) return T(0);
             const int t = g.nz - 1;
-            const T q0 = cv(c[cidx(g, i, j, t)]), q1 = cv(c[cidx(g, i, j, t - 1)]), q2 = cv(c[cidx(g, i, j, t - 2)]);
+            const T q0 = (T)(c[cidx(g, i, j, t)]), q1 = (T)(c[cidx(g, i, j, t - 1)]), q2 = (T)(c[cidx(g, i, j, t - 2)]);
             return scale * (T(0.125) * (T(15) * q0 - T(10) * q1 + T(3) * q2));
         }
-        return scale * cv(c[cidx(g, i, j, k)]);
+        return scale * (T)(c[cidx(g, i, j, k)]);
     }
 };
 using VelFP = VelFPT<double>;
@@ -168,8 +158,8 @@ __device__ __forceinline__ double isign(double m, double s) {
 // FP64 issue slot (74 cycles of a warp), these about ten integer instructions,
 // and give the same bits: round to nearest even, FP32 subnormals included; a
 // NaN becomes a quiet NaN.  What is not zero or normal in FP32 takes the call.
-// They pay in kernels bound by FP64 issue (Smagorinsky tile on 256x256x128: 388
-// us with conversions, 285 with these); kernels that wait on memory keep the
+// They pay in kernels bound by FP64 issue (viscous tile on 256x256x128: 520 us
+// with conversions, 450 with these); kernels that wait on memory keep the
 // conversion (k_add_f32 37 us against 41, k_adj_edges_gather 573 against 769).
 static __device__ __noinline__ float d2f_rare(double x) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);

@@ -997,10 +997,11 @@ static void to_single(Ctx& c, const double* a, float* b, long long n) {
     KS_LAUNCH(c, k_to_single, (unsigned)(nb < 152 * 16 ? nb : 152 * 16), BS, 12.0 * n, a, b, n);
 }
 
+void launch_vel_single(Ctx& c, const Grid& g, const double* vel, GodunovIn32& in32) { to_single(c, vel, in32.vel, 3 * g.N); }
+
 void launch_premac(Ctx& c, const Grid& g, const double* vel, const double* forces, double dt, GodunovBufs& B, double* mac[3], int fp32,
                    GodunovIn32* in32, int edges) {
     if (fp32) {
-        to_single(c, vel, in32->vel, 3 * g.N);
         to_single(c, forces, in32->forces, 3 * g.N);
         premac_t<float>(c, g, in32->vel, in32->forces, dt, B, mac, edges);
     } else {
@@ -1011,7 +1012,7 @@ void launch_premac(Ctx& c, const Grid& g, const double* vel, const double* force
 void launch_advection(Ctx& c, const Grid& g, const double* vel, const double* forces, const double* mac[3], double dt, double rho,
                       GodunovBufs& B, double* conv, int fp32, GodunovIn32* in32) {
     if (fp32) {
-        // vel and forces: the FP32 copies made by launch_premac of the same step
+        // vel and forces: the FP32 copies of the same step
         for (int d = 0; d < 3; ++d) to_single(c, mac[d], in32->mac[d], nfaces(g, d));
         const float* m32[3] = {in32->mac[0], in32->mac[1], in32->mac[2]};
         advection_t<float>(c, g, in32->vel, in32->forces, m32, dt, rho, B, conv);

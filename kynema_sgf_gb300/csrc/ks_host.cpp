@@ -922,7 +922,7 @@ void Sim::compute_dt() {
 // oscillatory BodyForce takes its factor at the mid-step time (BodyForce.cpp:145-160)
 void Sim::sources(const double* vel, const double* theta) {
     S_.t_nph = 0.5 * (t_.cur + t_.next);
-    launch_sources(ctx_, g_, vel, gp_.p, act_.p, src_.p, S_, theta);
+    launch_sources(ctx_, g_, vel, gp_.p, act_.p, src_.p, S_, theta, mixed_);
 }
 
 // ---------------------------------------------------------------- ABL
@@ -1337,7 +1337,7 @@ void Sim::mac_project() {
     if (rn > target && !mac_.fixed_iters) throw KsError(KS_ERR_NOT_CONVERGED, "MAC projection did not converge in mac_proj.maxiter V-cycles");
     mac_it_ = it;
     mac_r_ = rn;
-    launch_mac_correct(ctx_, g_, L.phi, umac_[0].p, umac_[1].p, umac_[2].p, beta);
+    launch_mac_correct(ctx_, g_, L.phi, umac_[0].p, umac_[1].p, umac_[2].p, beta, mixed_);
     if (direct) {  // nothing but the next MAC solve writes L.phi
         mac_phi_last_ = L.phi;
         mac_prev_ok_ = true;
@@ -1653,10 +1653,12 @@ void Sim::apply_predictor(bool incremental) {
         return;
     }
     const double dt = t_.dt[0];
-    launch_smagorinsky(ctx_, g_, vel_old_.p, mueff_.p, S_, alpha_.p, mixed_);
+    const float* v32 = mixed_ ? in32_.vel : nullptr;
+    if (mixed_) launch_vel_single(ctx_, g_, vel_old_.p, in32_);
+    launch_smagorinsky(ctx_, g_, vel_old_.p, mueff_.p, S_, alpha_.p, mixed_, v32);
     sources(vel_old_.p, theta_old_.p);  // BoussinesqBuoyancy: theta at Old
     if (wallmodel_) launch_wall_grad(ctx_, g_, vel_old_.p, mueff_.p, wg_.p, shear_, utau_ * utau_, um_[0], um_[1], vmag_, rho_);
-    launch_divtau(ctx_, g_, vel_old_.p, mueff_.p, wg_.p, divtau_.p, 1, src_.p, forces_.p, nullptr, nullptr, dt, rho_, mixed_);
+    launch_divtau(ctx_, g_, vel_old_.p, mueff_.p, wg_.p, divtau_.p, 1, src_.p, forces_.p, nullptr, nullptr, dt, rho_, mixed_, v32);
     if (temp_) {  // the temperature's diff_term(Old) (no temperature sources)
         if (tzlo_ == 1)
             launch_theta_wall_grad(ctx_, g_, vel_old_.p, theta_old_.p, alpha_.p, tgz_.p, shear_, utau_, kappa_, std::log(zref_ / z0t_), vmag_,
@@ -1673,7 +1675,7 @@ void Sim::apply_predictor(bool incremental) {
     // unchanged, so only BoussinesqBuoyancy (theta at n+1/2) changes src;
     // compute_diffusion_term(Old) reproduces divtau.
     if (S_.bous) sources(vel_old_.p, theta_nph_.p);
-    launch_predictor_rhs(ctx_, g_, vel_old_.p, conv_.p, src_.p, divtau_.p, vel_.p, dt, rho_, diff_fac());
+    launch_predictor_rhs(ctx_, g_, vel_old_.p, conv_.p, src_.p, divtau_.p, vel_.p, dt, rho_, diff_fac(), mixed_);
     if (diff_type_ == 0) {  // explicit RK2 correction (incflo_advance.cpp:388-400)
         launch_divtau(ctx_, g_, vel_.p, mueff_.p, wg_.p, vel_tmp_.p, 2, nullptr, nullptr, vel_.p, divtau_.p, dt, rho_, mixed_);
         std::swap(vel_.p, vel_tmp_.p);

@@ -203,12 +203,12 @@ __global__ void __launch_bounds__(128) k_smag_col(Grid g, const double* vel, dou
 // instead of the 18 reads of the thread-per-cell form.
 constexpr int SMX = 32, SMY = 4, SMZ = 4;
 constexpr int SMHX = SMX + 2, SMHY = SMY + 2, SMHZ = SMZ + 2, SMNH = SMHX * SMHY * SMHZ;
-__global__ void __launch_bounds__(SMX* SMY* SMZ) k_smag_tile(Grid g, const double* vel, double* mueff, double mu, double rhofac,
+__global__ void __launch_bounds__(SMX* SMY* SMZ) k_smag_tile(Grid g, const float* vel, double* mueff, double mu, double rhofac,
                                                             double* alpha, double mu_pr, double iprt) {
     __shared__ float sV[3 * SMNH];
     const int i0 = blockIdx.x * SMX, j0 = blockIdx.y * SMY, k0 = blockIdx.z * SMZ;
     const int tid = threadIdx.x, nthr = SMX * SMY * SMZ;
-    const VelFPT<float, double, true> V{vel, g, 1.0f};
+    const VelFPT<float, float> V{vel, g, 1.0f};
     for (int h = tid; h < SMNH; h += nthr) {
         const int hx = h % SMHX, hy = (h / SMHX) % SMHY, hz = h / (SMHX * SMHY);
         // a tile may be wider than the grid: wrap x, y (and periodic z) fully
@@ -267,8 +267,8 @@ struct SrcCoef {
 };
 // Which terms run is a template argument: as a run-time flag each absent term
 // still took its FP64 issue slots, predicated off (22 for 12 a cell: 351 us on
-// 256x256x128, 247 now).
-template <int COR, int ACT, int BOUS>
+// 256x256x128, 200 now).
+template <int COR, int ACT, int BOUS, int PLAIN>
 __global__ void k_sources(Grid g, const double* vel, const double* gp, const double* act, double* src, SrcCoef s, const double* theta) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= g.N) return;
@@ -277,7 +277,10 @@ __global__ void k_sources(Grid g, const double* vel, const double* gp, const dou
     for (int n = 0; n < 3; ++n) f[n] = s.c[n] - gp[n * N + t];
     if (COR) {
         const double u0 = vel[t], u1 = vel[N + t], u2 = vel[2 * N + t];
-        for (int n = 0; n < 3; ++n) f[n] += s.M[n][0] * u0 + s.M[n][1] * u1 + s.M[n][2] * u2;
+        for (int n = 0; n < 3; ++n) {
+            if constexpr (PLAIN) f[n] += s.M[n][0] * u0 + s.M[n][1] * u1 + s.M[n][2] * u2;
+            else f[n] = fma(s.M[n][2], u2, fma(s.M[n][1], u1, fma(s.M[n][0], u0, f[n])));
+        }
     }
     if (ACT)
         for (int n = 0; n < 3; ++n) f[n] += s.rho * act[n * N + t];
@@ -474,13 +477,14 @@ struct TauEpi {
     double dt, rho, omega;
     double irho;  // 1 / rho, formed on the host
     double hdr;   // dt / (2 rho)
+    double hdt;   // dt / 2
 };
 
 // FP32 form (mixed precision, modes 0-2): staged values, face fluxes and their
 // arithmetic are FP32, the FP64 inputs rounded once when staged; the epilogue
 // runs in FP64.
-template <int MODE>
-__global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const double* vel, const double* mueff, const double* wg, double* out,
+template <int MODE, int V32>
+__global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const double* vel, const float* vel32, const double* mueff, const double* wg, double* out,
                                                                TauEpi E) {
     using T = float;
     extern __shared__ __align__(16) unsigned char sm_raw[];
@@ -501,7 +505,12 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
         const int gi = ((i0 + hx - 1) % g.nx + g.nx) % g.nx, gj = ((j0 + hy - 1) % g.ny + g.ny) % g.ny;
         int gk = k0 + hz - 1;
         if (g.zper) gk = (gk % g.nz + g.nz) % g.nz;
-        for (int n = 0; n < 3; ++n) sV[n * TNH + h] = d2f(V(n, gi, gj, gk));
+        if (V32 && gk >= 0 && gk < g.nz) {
+            const long long c = cidx(g, gi, gj, gk);
+            for (int n = 0; n < 3; ++n) sV[n * TNH + h] = vel32[n * g.N + c];
+        } else {  // no FP32 copy, or a ghost across a wall (formed in FP64)
+            for (int n = 0; n < 3; ++n) sV[n * TNH + h] = d2f(V(n, gi, gj, gk));
+        }
         const int kk = g.zper ? gk : (gk < 0 ? 0 : (gk >= g.nz ? g.nz - 1 : gk));
         sM[h] = d2f(mueff[cidx(g, gi, gj, kk)]);
     }
@@ -557,7 +566,7 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
     const int tx = tid % TTX, ty = (tid / TTX) % TTY, tz = tid / (TTX * TTY);
     const int i = i0 + tx, j = j0 + ty, k = k0 + tz;
     const bool live = i < g.nx && j < g.ny && k < g.nz;
-    const double irho = E.irho, hdr = E.hdr;
+    const double irho = E.irho, hdt = E.hdt;
     const long long N = g.N, t = live ? cidx(g, i, j, k) : 0;
     for (int n = 0; n < 3 && live; ++n) {
         const int ax = (tz * TTY + ty) * (TTX + 1) + tx;
@@ -574,7 +583,7 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
             out[m] = acc;
             E.forces[m] = (E.src[m] + acc) * irho;
         } else {
-            out[m] = E.base[m] + hdr * (acc - E.dold[m]);
+            out[m] = E.base[m] + hdt * (acc - E.dold[m]) * irho;
         }
     }
 }
@@ -853,11 +862,16 @@ inline TauShape tau_shape(const Grid& g) {
 
 // predictor_rhs (src/equation_systems/CompRHSOps.H:32-141); fac = 1 explicit,
 // 1/2 Crank-Nicolson, 0 implicit
-__global__ void k_pred_rhs(long long N3, const double* vo, const double* conv, const double* src, const double* dt_, double* vel, double dtr,
-                           double fac) {
+// PLAIN (here, in k_sources and in k_mac_correct): the products as they stand,
+// for the mixed-precision form, whose FP32 advection turns a change of the last
+// bit into another trajectory; the FP64 form folds them (dtr = dt / rho).
+template <int PLAIN>
+__global__ void k_pred_rhs(long long N3, const double* vo, const double* conv, const double* src, const double* dt_, double* vel, double dt,
+                           double rho, double irho, double fac, double dtr) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= N3) return;
-    vel[t] = vo[t] + dtr * ((conv[t] + src[t]) + fac * dt_[t]);  // dtr = dt / rho, formed on the host
+    if constexpr (PLAIN) vel[t] = (rho * vo[t] + dt * (conv[t] + src[t] + fac * dt_[t])) * irho;
+    else vel[t] = vo[t] + dtr * ((conv[t] + src[t]) + fac * dt_[t]);
 }
 
 // ---------------------------------------------------------------- projection
@@ -1064,15 +1078,23 @@ __global__ void k_mac_divmax(Grid g, const double* um, const double* vm, const d
 }
 
 // bx = beta / dx, ...
-__global__ void k_mac_correct(Grid g, const double* phi, double* um, double* vm, double* wm, double bx, double by, double bz) {
+template <int PLAIN>
+__global__ void k_mac_correct(Grid g, const double* phi, double* um, double* vm, double* wm, double beta, double bx, double by, double bz) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= g.N) return;
     int i, j, k;
     cell_of(g, t, i, j, k);
     const double p0 = phi[t];
-    um[t] -= bx * (p0 - phi[cidx(g, wrapn(i - 1, g.nx), j, k)]);
-    vm[t] -= by * (p0 - phi[cidx(g, i, wrapn(j - 1, g.ny), k)]);
-    if (g.zper || k > 0) wm[t] -= bz * (p0 - phi[cidx(g, i, j, k == 0 ? g.nz - 1 : k - 1)]);
+    const double px = phi[cidx(g, wrapn(i - 1, g.nx), j, k)], py = phi[cidx(g, i, wrapn(j - 1, g.ny), k)];
+    if constexpr (PLAIN) {
+        um[t] -= beta * (p0 - px) * g.idx;
+        vm[t] -= beta * (p0 - py) * g.idy;
+        if (g.zper || k > 0) wm[t] -= beta * (p0 - phi[cidx(g, i, j, k == 0 ? g.nz - 1 : k - 1)]) * g.idz;
+    } else {
+        um[t] -= bx * (p0 - px);
+        vm[t] -= by * (p0 - py);
+        if (g.zper || k > 0) wm[t] -= bz * (p0 - phi[cidx(g, i, j, k == 0 ? g.nz - 1 : k - 1)]);
+    }
 }
 
 // ---------------------------------------------------------------- reductions
@@ -1261,12 +1283,13 @@ void launch_init_abl(Ctx& c, const Grid& g, double* vel, int loglaw, const doubl
 }
 void launch_fill(Ctx& c, double* p, double v, long long n) { KS_LAUNCH(c, k_fill, nblocks(n, BS), BS, B8 * n, p, v, n); }
 void launch_copy(Ctx& c, double* d, const double* s, long long n) { KS_LAUNCH(c, k_copy, nblocks(n, BS), BS, B8 * 2 * n, d, s, n); }
-void launch_smagorinsky(Ctx& c, const Grid& g, const double* vel, double* mueff, const Scalars& s, double* alpha, int fp32) {
+void launch_smagorinsky(Ctx& c, const Grid& g, const double* vel, double* mueff, const Scalars& s, double* alpha, int fp32,
+                        const float* vel32) {
     if (!s.temp) alpha = nullptr;
     const double bytes = B8 * ((s.smag ? 4 : 1) + (alpha ? 1 : 0)) * g.N;
     if (fp32 && s.smag) {
         const dim3 grid((g.nx + SMX - 1) / SMX, (g.ny + SMY - 1) / SMY, (g.nz + SMZ - 1) / SMZ);
-        KS_LAUNCH(c, k_smag_tile, grid, SMX * SMY * SMZ, bytes, g, vel, mueff, s.mu, s.rho * s.smag_fac, alpha, s.mu_pr, s.iprt);
+        KS_LAUNCH(c, k_smag_tile, grid, SMX * SMY * SMZ, bytes - 12.0 * g.N, g, vel32, mueff, s.mu, s.rho * s.smag_fac, alpha, s.mu_pr, s.iprt);
     } else if (fp32)
         KS_LAUNCH(c, k_smag<float>, nblocks(g.N, BS), BS, bytes, g, vel, mueff, s.mu, s.rho, s.smag_fac, s.smag, alpha, s.mu_pr, s.iprt);
     else if (s.smag) {
@@ -1284,7 +1307,7 @@ void launch_smagorinsky(Ctx& c, const Grid& g, const double* vel, double* mueff,
 // (e, n, u the east / north / up unit vectors, ue = e.u etc., f = corfac, h = hfac) is the linear map
 //   M = f sin (e n^T - n e^T) + f h cos (u e^T - e u^T).
 void launch_sources(Ctx& c, const Grid& g, const double* vel_old, const double* gp, const double* act, double* src, const Scalars& s,
-                    const double* theta) {
+                    const double* theta, int plain) {
     SrcCoef k{};
     k.rho = s.rho;
     k.T_ref = s.T_ref;
@@ -1300,9 +1323,11 @@ void launch_sources(Ctx& c, const Grid& g, const double* vel_old, const double* 
                         (s.sinphi * (s.east[n] * s.north[m] - s.north[n] * s.east[m]) + s.hfac * s.cosphi * (s.up[n] * s.east[m] - s.east[n] * s.up[m]));
     }
     using Kern = void (*)(Grid, const double*, const double*, const double*, double*, SrcCoef, const double*);
-    static const Kern kern[8] = {k_sources<0, 0, 0>, k_sources<1, 0, 0>, k_sources<0, 1, 0>, k_sources<1, 1, 0>,
-                                 k_sources<0, 0, 1>, k_sources<1, 0, 1>, k_sources<0, 1, 1>, k_sources<1, 1, 1>};
-    const Kern run = kern[(s.cor ? 1 : 0) + (s.act ? 2 : 0) + (s.bous ? 4 : 0)];
+    static const Kern kern[2][8] = {{k_sources<0, 0, 0, 0>, k_sources<1, 0, 0, 0>, k_sources<0, 1, 0, 0>, k_sources<1, 1, 0, 0>,
+                                     k_sources<0, 0, 1, 0>, k_sources<1, 0, 1, 0>, k_sources<0, 1, 1, 0>, k_sources<1, 1, 1, 0>},
+                                    {k_sources<0, 0, 0, 1>, k_sources<1, 0, 0, 1>, k_sources<0, 1, 0, 1>, k_sources<1, 1, 0, 1>,
+                                     k_sources<0, 0, 1, 1>, k_sources<1, 0, 1, 1>, k_sources<0, 1, 1, 1>, k_sources<1, 1, 1, 1>}};
+    const Kern run = kern[plain ? 1 : 0][(s.cor ? 1 : 0) + (s.act ? 2 : 0) + (s.bous ? 4 : 0)];
     KS_LAUNCH_NAMED(c, "k_sources", run, nblocks(g.N, BS), BS, B8 * (6 + 3 * s.cor + 3 * s.act + s.bous) * g.N, g, vel_old, gp, act, src, k, theta);
 }
 void launch_plane_sums(Ctx& c, const Grid& g, const double* vel, double* parts, int* np) {
@@ -1355,20 +1380,22 @@ static void launch_divtau_col(Ctx& c, const Grid& g, const double* vel, const do
 }
 static_assert(sizeof(TauPlanes<4>) <= 48 * 1024, "needs no shared memory attribute");
 void launch_divtau(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, int mode,
-                   const double* src, double* forces, const double* base, const double* dold, double dt, double rho, int fp32) {
+                   const double* src, double* forces, const double* base, const double* dold, double dt, double rho, int fp32,
+                   const float* vel32) {
     const double per_cell = 4 + 3 + (mode == 1 ? 6 : 0) + (mode == 2 ? 6 : 0);
-    TauEpi E{mode, src, base, dold, nullptr, nullptr, nullptr, forces, nullptr, dt, rho, 0.0, 1.0 / rho, 0.5 * dt / rho};
+    TauEpi E{mode, src, base, dold, nullptr, nullptr, nullptr, forces, nullptr, dt, rho, 0.0, 1.0 / rho, 0.5 * dt / rho, 0.5 * dt};
     if (fp32) {
         const dim3 grid((g.nx + TTX - 1) / TTX, (g.ny + TTY - 1) / TTY, (g.nz + TTZ - 1) / TTZ);
-        const auto run = mode == 0 ? k_divtau_tile<0> : (mode == 1 ? k_divtau_tile<1> : k_divtau_tile<2>);
-        KS_LAUNCH_SMEM_NAMED(c, "k_divtau_tile", run, grid, TTX * TTY * TTZ, tau_smem(), B8 * per_cell * g.N, g, vel, mueff, wg, out, E);
+        const auto run = vel32 ? (mode == 0 ? k_divtau_tile<0, 1> : (mode == 1 ? k_divtau_tile<1, 1> : k_divtau_tile<2, 1>))
+                               : (mode == 0 ? k_divtau_tile<0, 0> : (mode == 1 ? k_divtau_tile<1, 0> : k_divtau_tile<2, 0>));
+        KS_LAUNCH_SMEM_NAMED(c, "k_divtau_tile", run, grid, TTX * TTY * TTZ, tau_smem(), B8 * per_cell * g.N, g, vel, vel32, mueff, wg, out, E);
     } else {
         launch_divtau_col(c, g, vel, mueff, wg, out, E, B8 * per_cell * g.N);
     }
 }
 void launch_divtau_corrector(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, const double* vel_old,
                              const double* conv_old, const double* conv_new, const double* dold, const double* src, double dt, double rho) {
-    TauEpi E{3, src, vel_old, dold, conv_old, conv_new, nullptr, nullptr, nullptr, dt, rho, 0.0, 1.0 / rho, 0.5 * dt / rho};
+    TauEpi E{3, src, vel_old, dold, conv_old, conv_new, nullptr, nullptr, nullptr, dt, rho, 0.0, 1.0 / rho, 0.5 * dt / rho, 0.5 * dt};
     launch_divtau_col(c, g, vel, mueff, wg, out, E, B8 * 22.0 * g.N);
 }
 int divtau_blocks(const Grid& g) {
@@ -1377,12 +1404,13 @@ int divtau_blocks(const Grid& g) {
 }
 void launch_divtau_jacobi(Ctx& c, const Grid& g, const double* x, const double* mueff, const double* wg, const double* b, const double* dinv,
                           double* out, double rho, double dtd, double omega, double* parts) {
-    TauEpi E{omega > 0.0 ? 7 : 8, nullptr, b, nullptr, nullptr, nullptr, dinv, nullptr, parts, dtd, rho, omega, 1.0 / rho, 0.5 * dtd / rho};
+    TauEpi E{omega > 0.0 ? 7 : 8, nullptr, b, nullptr, nullptr, nullptr, dinv, nullptr, parts, dtd, rho, omega, 1.0 / rho, 0.5 * dtd / rho, 0.5 * dtd};
     launch_divtau_col(c, g, x, mueff, wg, out, E, B8 * ((omega > 0.0 ? 13.0 : 10.0) * g.N));
 }
 void launch_predictor_rhs(Ctx& c, const Grid& g, const double* vo, const double* conv, const double* src, const double* dtau, double* vel,
-                          double dt, double rho, double fac) {
-    KS_LAUNCH(c, k_pred_rhs, nblocks(3 * g.N, BS), BS, B8 * 15 * g.N, 3 * g.N, vo, conv, src, dtau, vel, dt / rho, fac);
+                          double dt, double rho, double fac, int plain) {
+    const auto run = plain ? k_pred_rhs<1> : k_pred_rhs<0>;
+    KS_LAUNCH_NAMED(c, "k_pred_rhs", run, nblocks(3 * g.N, BS), BS, B8 * 15 * g.N, 3 * g.N, vo, conv, src, dtau, vel, dt, rho, 1.0 / rho, fac, dt / rho);
 }
 void launch_proj_pre(Ctx& c, const Grid& g, double* vel, const double* vo, const double* gp, double scaling, double rho, int add_gp,
                      int sub_old) {
@@ -1417,8 +1445,9 @@ void launch_mac_divmax(Ctx& c, const Grid& g, const double* um, const double* vm
     *np = parts_for(g.N);
     KS_LAUNCH(c, k_mac_divmax, *np, BS, B8 * (2 * g.N + g.NFz), g, um, vm, wm, parts, *np);
 }
-void launch_mac_correct(Ctx& c, const Grid& g, const double* phi, double* um, double* vm, double* wm, double beta) {
-    KS_LAUNCH(c, k_mac_correct, nblocks(g.N, BS), BS, B8 * 7 * g.N, g, phi, um, vm, wm, beta * g.idx, beta * g.idy, beta * g.idz);
+void launch_mac_correct(Ctx& c, const Grid& g, const double* phi, double* um, double* vm, double* wm, double beta, int plain) {
+    const auto run = plain ? k_mac_correct<1> : k_mac_correct<0>;
+    KS_LAUNCH_NAMED(c, "k_mac_correct", run, nblocks(g.N, BS), BS, B8 * 7 * g.N, g, phi, um, vm, wm, beta, beta * g.idx, beta * g.idy, beta * g.idz);
 }
 void launch_cfl(Ctx& c, const Grid& g, const double* vel, const double* src, const double* mu, double rho, double* parts, int* np) {
     *np = parts_for(g.N);

@@ -160,12 +160,13 @@ void launch_init_abl(Ctx& c, const Grid& g, double* vel, int loglaw, const doubl
                      double amp, double zmax_rel, unsigned long long seed);
 // mu_eff (and alpha_eff when s.temp is set and alpha is not null)
 // fp32 = 1: strain rate in FP32 arithmetic (mixed-precision form), mu_eff stored in FP64
-void launch_smagorinsky(Ctx& c, const Grid& g, const double* vel, double* mueff, const Scalars& s, double* alpha = nullptr, int fp32 = 0);
+void launch_smagorinsky(Ctx& c, const Grid& g, const double* vel, double* mueff, const Scalars& s, double* alpha = nullptr, int fp32 = 0,
+                        const float* vel32 = nullptr);  // vel32: the velocity's FP32 copy (fp32)
 void launch_fill(Ctx& c, double* p, double v, long long n);
 void launch_copy(Ctx& c, double* dst, const double* src, long long n);
 // src = rho (-gp / rho + sources); theta: the temperature state BoussinesqBuoyancy reads
 void launch_sources(Ctx& c, const Grid& g, const double* vel_old, const double* gp, const double* act, double* src, const Scalars& s,
-                    const double* theta = nullptr);
+                    const double* theta = nullptr, int plain = 0);  // plain: k_pred_rhs
 void launch_plane_sums(Ctx& c, const Grid& g, const double* vel, double* partials, int* nparts);
 void launch_wall_grad(Ctx& c, const Grid& g, const double* vel_old, const double* mueff, double* wg, int shear_type, double ut2,
                       double um0, double um1, double vmag, double rho);
@@ -174,7 +175,8 @@ void launch_wall_grad(Ctx& c, const Grid& g, const double* vel_old, const double
 // Fused: no face arrays touch memory.
 // fp32 = 1 (modes 0-2): staging, face fluxes and divergence in FP32 (mixed-precision form), epilogue in FP64
 void launch_divtau(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, int mode,
-                   const double* src, double* forces, const double* base, const double* dold, double dt, double rho, int fp32 = 0);
+                   const double* src, double* forces, const double* base, const double* dold, double dt, double rho, int fp32 = 0,
+                   const float* vel32 = nullptr);  // vel32: the velocity's FP32 copy, where there is one (fp32)
 // the same result through face-flux arrays in caller-provided scratch (9 arrays:
 // N cells for x and y faces, nx*ny*(nz+1) for z faces) and a divergence pass
 void launch_divtau_faces(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, int mode,
@@ -192,7 +194,7 @@ void launch_divtau_jacobi(Ctx& c, const Grid& g, const double* x, const double* 
                           double* out, double rho, double dtd, double omega, double* parts);
 // predictor_rhs: vel = (rho vel_old + dt (conv + src + fac divtau)) / rho
 void launch_predictor_rhs(Ctx& c, const Grid& g, const double* vel_old, const double* conv, const double* src, const double* divtau,
-                          double* vel, double dt, double rho, double fac);
+                          double* vel, double dt, double rho, double fac, int plain = 0);
 void launch_proj_pre(Ctx& c, const Grid& g, double* vel, const double* vel_old, const double* gp, double scaling, double rho,
                      int add_gp, int sub_old);
 void launch_nodal_rhs(Ctx& c, const Grid& g, const double* vel, double* rhs, double* partials, int* nparts);
@@ -204,7 +206,7 @@ void launch_mac_rhs(Ctx& c, const Grid& g, const double* um, const double* vm, c
                     int* nparts);
 // per-block maxima of |div u_mac| (parts[0..np)) and of the face speeds (parts[np..2np))
 void launch_mac_divmax(Ctx& c, const Grid& g, const double* um, const double* vm, const double* wm, double* partials, int* nparts);
-void launch_mac_correct(Ctx& c, const Grid& g, const double* phi, double* um, double* vm, double* wm, double beta);
+void launch_mac_correct(Ctx& c, const Grid& g, const double* phi, double* um, double* vm, double* wm, double beta, int plain = 0);
 void launch_cfl(Ctx& c, const Grid& g, const double* vel, const double* src, const double* mueff, double rho, double* partials,
                 int* nparts);
 void launch_ke(Ctx& c, const Grid& g, const double* vel, double rho, double* partials, int* nparts);
@@ -245,13 +247,15 @@ struct GodunovBufs {
     void* tr[3][3][3];  // transverse-corrected states tr[a][b][n]
     void* flux[3][3];   // fluxes flux[d][n]
 };
-// FP32 copies of the advection inputs for the mixed-precision form: launch_premac fills vel and
-// forces, launch_advection (same step) the MAC velocities
+// FP32 copies of the advection inputs for the mixed-precision form: launch_vel_single fills vel (read
+// by the Smagorinsky and viscous tiles too), launch_premac (same step) forces, launch_advection the
+// MAC velocities
 struct GodunovIn32 {
     float* vel;     // 3 N
     float* forces;  // 3 N
     float* mac[3];  // face arrays
 };
+void launch_vel_single(Ctx& c, const Grid& g, const double* vel, GodunovIn32& in32);
 // edges: also store the unlimited PPM edges (a reverse step reads them)
 void launch_premac(Ctx& c, const Grid& g, const double* vel_old, const double* forces, double dt, GodunovBufs& B, double* mac[3],
                    int fp32, GodunovIn32* in32, int edges);
