@@ -29,6 +29,33 @@ __host__ __device__ inline long long cidx(const Grid& g, int i, int j, int k) {
     return ((long long)k * g.ny + j) * g.nx + i;
 }
 __host__ __device__ inline int wrapn(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
+// any i: a tile or a warp's segment may be wider than the grid, but one period is the
+// rule, and the two remainders take some 40 instructions (a loop in their place is
+// slower still)
+__device__ inline int wrap_tile(int i, int n) {
+    i = wrapn(i, n);
+    if ((unsigned)i >= (unsigned)n) i = (i % n + n) % n;
+    return i;
+}
+// Marches of a thread per column, up to 128 columns of a row a block: the column,
+// the launch, and 16 layers a march or fewer where that leaves less than `warps`.
+#ifdef __CUDACC__
+__device__ inline bool column_of(const Grid& g, int& i, int& j) {
+    const unsigned nb = ((unsigned)g.nx + blockDim.x - 1) / blockDim.x, b = blockIdx.x / nb;
+    i = (int)((blockIdx.x - b * nb) * blockDim.x + threadIdx.x);
+    j = (int)b;
+    return i < g.nx;
+}
+#endif
+inline int column_threads(const Grid& g) { return g.nx > 96 ? 128 : 32 * ((g.nx + 31) / 32); }
+inline dim3 column_grid(const Grid& g, int kc) {
+    const int t = column_threads(g);
+    return dim3((unsigned)((g.nx + t - 1) / t) * (unsigned)g.ny, (unsigned)((g.nz + kc - 1) / kc));
+}
+inline int march_layers(const Grid& g, int warps) {
+    const long long kc = g.N / (32LL * warps);
+    return kc < 1 ? 1 : (kc > 16 ? 16 : (int)kc);
+}
 __host__ __device__ inline double hd(const Grid& g, int d) { return d == 0 ? g.dx : (d == 1 ? g.dy : g.dz); }
 __host__ __device__ inline double ihd(const Grid& g, int d) { return d == 0 ? g.idx : (d == 1 ? g.idy : g.idz); }
 __host__ __device__ inline int nd(const Grid& g, int d) { return d == 0 ? g.nx : (d == 1 ? g.ny : g.nz); }

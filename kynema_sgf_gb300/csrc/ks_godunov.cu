@@ -436,10 +436,10 @@ __global__ void __launch_bounds__(256) k_ppm_x(PpmArgs<T> A, T s, T rho, PpmOut<
     const int lane = threadIdx.x & 31;
     const long long rows = (long long)g.ny * g.nz;
     if (w >= rows * nseg) return;  // whole warps leave together
-    const int row = (int)(w / nseg), seg = (int)(w % nseg);
+    const int row = (int)((unsigned)w / (unsigned)nseg), seg = (int)((unsigned)w - (unsigned)row * (unsigned)nseg);
     const int c = seg * XF + lane - H;
     const bool own = lane >= H && lane <= (LOADE ? 31 : 30) && c < g.nx;
-    auto wx = [&](int x) { return ((x % g.nx) + g.nx) % g.nx; };
+    auto wx = [&](int x) { return wrap_tile(x, g.nx); };
     const long long rb = (long long)row * g.nx;  // row base: cells and x faces share the index
     const long long fc = rb + wx(c);
     auto ld = [&](int n, int x) -> T { return (T)A.vel[n * g.N + rb + wx(x)]; };

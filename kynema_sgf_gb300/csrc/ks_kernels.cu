@@ -153,9 +153,9 @@ __global__ void k_smag(Grid g, const double* vel, double* mueff, double mu, doub
 // of the thread-per-cell form (256x256x128: 1400 us, 575 now).
 __global__ void __launch_bounds__(128) k_smag_col(Grid g, const double* vel, double* mueff, double mu, double rhofac, double* alpha, double mu_pr,
                                                   double iprt, int kc) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
-    if (i >= g.nx) return;
-    const int k0 = blockIdx.z * kc, k1 = min(k0 + kc, g.nz);
+    int i, j;
+    if (!column_of(g, i, j)) return;
+    const int k0 = blockIdx.y * kc, k1 = min(k0 + kc, g.nz);
     const long long N = g.N;
     const int sz = g.nx * g.ny;
     const int xp = i + 1 == g.nx ? 1 - g.nx : 1, xm = i == 0 ? g.nx - 1 : -1;
@@ -197,59 +197,57 @@ __global__ void __launch_bounds__(128) k_smag_col(Grid g, const double* vel, dou
     }
 }
 
-// Mixed-precision form: the same FP32 strain rate from a shared-memory tile of
-// 32 x 4 x 4 cells whose one-cell halo (fill-patch ghosts included) is staged
-// once, so each velocity value is loaded and rounded about 2.4 times per cell
-// instead of the 18 reads of the thread-per-cell form.
-constexpr int SMX = 32, SMY = 4, SMZ = 4;
-constexpr int SMHX = SMX + 2, SMHY = SMY + 2, SMHZ = SMZ + 2, SMNH = SMHX * SMHY * SMHZ;
-__global__ void __launch_bounds__(SMX* SMY* SMZ) k_smag_tile(Grid g, const float* vel, double* mueff, double mu, double rhofac,
-                                                            double* alpha, double mu_pr, double iprt) {
-    __shared__ float sV[3 * SMNH];
-    const int i0 = blockIdx.x * SMX, j0 = blockIdx.y * SMY, k0 = blockIdx.z * SMZ;
-    const int tid = threadIdx.x, nthr = SMX * SMY * SMZ;
+// Mixed-precision form: the same march over the FP32 copy of the velocity.  Its
+// values come from L1 (15 loads a cell), the strain rate is FP32 throughout, and
+// mu_eff is formed in FP64.  The sums are written out operation by operation: the
+// FP32 advection's branches follow every bit of the step, so the bits are kept
+// whatever the compiler would contract.  256x256x128: 230 us as tiles of 32 x 4 x 4
+// cells, whose staging spent four integer remainders on each of 2.4 values a
+// cell, 72 now; 512x512x256 1798 and 473.
+__global__ void __launch_bounds__(128) k_smag_march(Grid g, const float* vel, double* mueff, double mu, double rhofac, double* alpha,
+                                                    double mu_pr, double iprt, int kc) {
+    int i, j;
+    if (!column_of(g, i, j)) return;
+    const int k0 = blockIdx.y * kc, k1 = min(k0 + kc, g.nz);
+    const long long N = g.N;
+    const int sz = g.nx * g.ny;
+    const int xp = i + 1 == g.nx ? 1 - g.nx : 1, xm = i == 0 ? g.nx - 1 : -1;
+    const int yp = (j + 1 == g.ny ? 1 - g.ny : 1) * g.nx, ym = (j == 0 ? g.ny - 1 : -1) * g.nx;
     const VelFPT<float, float> V{vel, g, 1.0f};
-    for (int h = tid; h < SMNH; h += nthr) {
-        const int hx = h % SMHX, hy = (h / SMHX) % SMHY, hz = h / (SMHX * SMHY);
-        // a tile may be wider than the grid: wrap x, y (and periodic z) fully
-        const int gi = ((i0 + hx - 1) % g.nx + g.nx) % g.nx, gj = ((j0 + hy - 1) % g.ny + g.ny) % g.ny;
-        int gk = k0 + hz - 1;
-        if (g.zper) gk = (gk % g.nz + g.nz) % g.nz;
-        for (int n = 0; n < 3; ++n) sV[n * SMNH + h] = V(n, gi, gj, gk);
-    }
-    __syncthreads();
-    const int tx = tid % SMX, ty = (tid / SMX) % SMY, tz = tid / (SMX * SMY);
-    const int i = i0 + tx, j = j0 + ty, k = k0 + tz;
-    if (i >= g.nx || j >= g.ny || k >= g.nz) return;
-    const int c = ((tz + 1) * SMHY + ty + 1) * SMHX + tx + 1;
-    const float hx = 0.5f * d2f(g.idx), hy = 0.5f * d2f(g.idy);
-    float gx[3], gy[3], gz[3];
+    const float hx = 0.5f * d2f(g.idx), hy = 0.5f * d2f(g.idy), hz = 0.5f * d2f(g.idz), iz = d2f(g.idz);
+    const float* p = vel + (long long)k0 * sz + j * g.nx + i;
+    long long t = (long long)k0 * sz + j * g.nx + i;
+    float dn[3], at[3];
     for (int n = 0; n < 3; ++n) {
-        const float* v = sV + n * SMNH + c;
-        gx[n] = hx * (v[1] - v[-1]);
-        gy[n] = hy * (v[SMHX] - v[-SMHX]);
+        dn[n] = V(n, i, j, k0 - 1);
+        at[n] = p[n * N];
     }
-    if (!g.zper && (k == 0 || k == g.nz - 1)) {  // one-sided through the wall (ghost) value
-        float a = 1.0f / 3.0f, b = 1.0f, cc = -4.0f / 3.0f;
-        if (k == g.nz - 1) { a = 4.0f / 3.0f; b = -1.0f; cc = -1.0f / 3.0f; }
-        const float iz = d2f(g.idz);
+    for (int k = k0; k < k1; ++k, p += sz, t += sz) {
+        float up[3], gx[3], gy[3], gz[3];
+        for (int n = 0; n < 3; ++n) up[n] = k + 1 < g.nz ? p[n * N + sz] : V(n, i, j, k + 1);
         for (int n = 0; n < 3; ++n) {
-            const float* v = sV + n * SMNH + c;
-            gz[n] = (a * v[SMHX * SMHY] + b * v[0] + cc * v[-SMHX * SMHY]) * iz;
+            const float* v = p + n * N;
+            gx[n] = hx * (v[xp] - v[xm]);
+            gy[n] = hy * (v[yp] - v[ym]);
         }
-    } else {
-        const float hz = 0.5f * d2f(g.idz);
+        if (!g.zper && (k == 0 || k == g.nz - 1)) {  // one-sided through the wall (ghost) value
+            float a = 1.0f / 3.0f, b = 1.0f, c = -4.0f / 3.0f;
+            if (k == g.nz - 1) { a = 4.0f / 3.0f; b = -1.0f; c = -1.0f / 3.0f; }
+            for (int n = 0; n < 3; ++n) gz[n] = fmaf(c, dn[n], fmaf(a, up[n], b * at[n])) * iz;
+        } else {
+            for (int n = 0; n < 3; ++n) gz[n] = hz * (up[n] - dn[n]);
+        }
+        const float sxy = __fadd_rn(gy[0], gx[1]), syz = __fadd_rn(gz[1], gy[2]), szx = __fadd_rn(gx[2], gz[0]);
+        const float s2 = fmaf(gz[2], gz[2], fmaf(gx[0], gx[0], gy[1] * gy[1])), t2 = fmaf(szx, szx, fmaf(sxy, sxy, syz * syz));
+        const float s = sqrtf(fmaf(2.0f, s2, t2));
+        const double mut = rhofac * f2d(s);
+        mueff[t] = __dadd_rn(mu, mut);
+        if (alpha) alpha[t] = fma(iprt, mut, mu_pr);
         for (int n = 0; n < 3; ++n) {
-            const float* v = sV + n * SMNH + c;
-            gz[n] = hz * (v[SMHX * SMHY] - v[-SMHX * SMHY]);
+            dn[n] = at[n];
+            at[n] = up[n];
         }
     }
-    const float sxy = gy[0] + gx[1], syz = gz[1] + gy[2], szx = gx[2] + gz[0];
-    const float s = sqrtf(2.0f * (gx[0] * gx[0] + gy[1] * gy[1] + gz[2] * gz[2]) + (sxy * sxy + syz * syz + szx * szx));
-    const double mut = rhofac * f2d(s);
-    const long long t = cidx(g, i, j, k);
-    mueff[t] = mu + mut;
-    if (alpha) alpha[t] = mu_pr + iprt * mut;
 }
 
 // ---------------------------------------------------------------- sources
@@ -455,6 +453,10 @@ __global__ void k_tau_div(Grid g, Flux9 F, double* out, int mode, const double* 
 // shared memory, computes every face flux the tile needs once (the same
 // arithmetic as tensor_flux) into shared memory, then forms the divergence
 // and the mode epilogue of k_tau_div for its cells.  No face arrays touch HBM.
+// Bound by instruction issue and shared memory: with wrap_tile in place of four
+// remainders for each of 2.4 staged values a cell 395 -> 328 us on 256x256x128,
+// 3.20 -> 2.62 ms on 512x512x256 (a z march over 32 x 8 columns took 468 us and
+// 3.68 ms: its larger blocks leave too few warps to hide a layer's latency).
 constexpr int TTX = 32, TTY = 4, TTZ = 4;
 constexpr int THX = TTX + 2, THY = TTY + 2, THZ = TTZ + 2;
 constexpr int TNH = THX * THY * THZ;
@@ -502,9 +504,9 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
     for (int h = tid; h < TNH; h += nthr) {
         const int hx = h % THX, hy = (h / THX) % THY, hz = h / (THX * THY);
         // a tile may be wider than the grid (nx < TTX): wrap x, y (and periodic z) fully
-        const int gi = ((i0 + hx - 1) % g.nx + g.nx) % g.nx, gj = ((j0 + hy - 1) % g.ny + g.ny) % g.ny;
+        const int gi = wrap_tile(i0 + hx - 1, g.nx), gj = wrap_tile(j0 + hy - 1, g.ny);
         int gk = k0 + hz - 1;
-        if (g.zper) gk = (gk % g.nz + g.nz) % g.nz;
+        if (g.zper) gk = wrap_tile(gk, g.nz);
         if (V32 && gk >= 0 && gk < g.nz) {
             const long long c = cidx(g, gi, gj, gk);
             for (int n = 0; n < 3; ++n) sV[n * TNH + h] = vel32[n * g.N + c];
@@ -1288,15 +1290,16 @@ void launch_smagorinsky(Ctx& c, const Grid& g, const double* vel, double* mueff,
     if (!s.temp) alpha = nullptr;
     const double bytes = B8 * ((s.smag ? 4 : 1) + (alpha ? 1 : 0)) * g.N;
     if (fp32 && s.smag) {
-        const dim3 grid((g.nx + SMX - 1) / SMX, (g.ny + SMY - 1) / SMY, (g.nz + SMZ - 1) / SMZ);
-        KS_LAUNCH(c, k_smag_tile, grid, SMX * SMY * SMZ, bytes - 12.0 * g.N, g, vel32, mueff, s.mu, s.rho * s.smag_fac, alpha, s.mu_pr, s.iprt);
+        // layers a march: 16, fewer where that leaves less than 4096 warps
+        const int kc = march_layers(g, 4096);
+        KS_LAUNCH(c, k_smag_march, column_grid(g, kc), column_threads(g), bytes - 12.0 * g.N, g, vel32, mueff, s.mu, s.rho * s.smag_fac,
+                  alpha, s.mu_pr, s.iprt, kc);
     } else if (fp32)
         KS_LAUNCH(c, k_smag<float>, nblocks(g.N, BS), BS, bytes, g, vel, mueff, s.mu, s.rho, s.smag_fac, s.smag, alpha, s.mu_pr, s.iprt);
     else if (s.smag) {
         // layers a march: 16, fewer where that leaves less than 2048 warps
-        const int kc = (int)std::min<long long>(16, std::max<long long>(1, g.N / 65536));
-        const dim3 grid((unsigned)((g.nx + 127) / 128), (unsigned)g.ny, (unsigned)((g.nz + kc - 1) / kc));
-        KS_LAUNCH(c, k_smag_col, grid, std::min(128, 32 * ((g.nx + 31) / 32)), bytes, g, vel, mueff, s.mu, s.rho * s.smag_fac, alpha, s.mu_pr, s.iprt, kc);
+        const int kc = march_layers(g, 2048);
+        KS_LAUNCH(c, k_smag_col, column_grid(g, kc), column_threads(g), bytes, g, vel, mueff, s.mu, s.rho * s.smag_fac, alpha, s.mu_pr, s.iprt, kc);
     } else
         KS_LAUNCH(c, k_smag<double>, nblocks(g.N, BS), BS, bytes, g, vel, mueff, s.mu, s.rho, s.smag_fac, s.smag, alpha, s.mu_pr, s.iprt);
 }
