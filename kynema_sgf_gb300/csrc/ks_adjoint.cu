@@ -1048,10 +1048,10 @@ __global__ void __launch_bounds__(ATX* ATY* ATZ) k_adj_tau_tile(Grid g, const do
     const A sA = (A)s;
     for (int h = tid; h < ANH; h += nthr) {
         const int hx = h % AHX, hy = (h / AHX) % AHY, hz = h / (AHX * AHY);
-        const int gi = ((i0 + hx - 1) % g.nx + g.nx) % g.nx, gj = ((j0 + hy - 1) % g.ny + g.ny) % g.ny;
+        const int gi = wrap_tile(i0 + hx - 1, g.nx), gj = wrap_tile(j0 + hy - 1, g.ny);
         int gk = k0 + hz - 1;
         const bool inz = g.zper || (gk >= 0 && gk < g.nz);
-        if (g.zper) gk = (gk % g.nz + g.nz) % g.nz;
+        if (g.zper) gk = wrap_tile(gk, g.nz);
         for (int n = 0; n < 3; ++n) sV[n * ANH + h] = (A)Vd(g, vel, wg, n, gi, gj, gk);
         const int kk = g.zper ? gk : (gk < 0 ? 0 : (gk >= g.nz ? g.nz - 1 : gk));
         const long long c = cidx(g, gi, gj, kk);
@@ -1161,11 +1161,11 @@ __global__ void __launch_bounds__(ATX* ATY* ATZ) k_adj_tau_tile(Grid g, const do
     // flush: box positions to cells (ghost positions through the diffusion ghost rules)
     for (int h = tid; h < ANH; h += nthr) {
         const int hx = h % AHX, hy = (h / AHX) % AHY, hz = h / (AHX * AHY);
-        const int gi = ((i0 + hx - 1) % g.nx + g.nx) % g.nx, gj = ((j0 + hy - 1) % g.ny + g.ny) % g.ny;
+        const int gi = wrap_tile(i0 + hx - 1, g.nx), gj = wrap_tile(j0 + hy - 1, g.ny);
         const int gk = k0 + hz - 1;
         for (int n = 0; n < 3; ++n) Vdb(g, ub, wgb, n, gi, gj, gk, (double)aU[n * ANH + h]);
         if (mub && nonzero(aM[h])) {
-            if (g.zper || (gk >= 0 && gk < g.nz)) atomicAdd(&mub[cidx(g, gi, gj, g.zper ? (gk % g.nz + g.nz) % g.nz : gk)], (double)aM[h]);
+            if (g.zper || (gk >= 0 && gk < g.nz)) atomicAdd(&mub[cidx(g, gi, gj, g.zper ? wrap_tile(gk, g.nz) : gk)], (double)aM[h]);
         }
     }
 }
@@ -1406,42 +1406,48 @@ __global__ void k_adj_wall_global(Grid g, const double* vel, double bu, double b
     ub[g.N + t] += bv + bm * v * iws;
 }
 
-// ---- reverse of the Coriolis source src = rho (C u): u_bar += rho C^T src_bar
-__global__ void k_adj_coriolis(Grid g, const double* srcb, Scalars s, double* ub) {
+// ---- reverse of the Coriolis source src = M u (coriolis_map): u_bar += M^T src_bar.
+// Folded to 9 FP64 instructions a cell as the forward's, where the components
+// along east, north and up took about 45: 256x256x128 531 us, 152 now.
+struct Map3 {
+    double m[3][3];
+};
+__global__ void k_adj_coriolis(long long N, const double* srcb, Map3 M, double* ub) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N) return;
-    const long long N = g.N;
-    double fb[3];
-    for (int n = 0; n < 3; ++n) fb[n] = s.rho * srcb[n * N + t];
-    const double aeb = fb[0] * s.east[0] + fb[1] * s.east[1] + fb[2] * s.east[2];
-    const double anb = fb[0] * s.north[0] + fb[1] * s.north[1] + fb[2] * s.north[2];
-    const double aub = fb[0] * s.up[0] + fb[1] * s.up[1] + fb[2] * s.up[2];
-    const double unb = s.corfac * s.sinphi * aeb;
-    const double uub = -s.hfac * s.corfac * s.cosphi * aeb;
-    const double ueb = -s.corfac * s.sinphi * anb + s.hfac * s.corfac * s.cosphi * aub;
-    for (int n = 0; n < 3; ++n) ub[n * N + t] += ueb * s.east[n] + unb * s.north[n] + uub * s.up[n];
+    if (t >= N) return;
+    const double a = srcb[t], b = srcb[N + t], c = srcb[2 * N + t];
+    for (int m = 0; m < 3; ++m) ub[m * N + t] = fma(M.m[2][m], c, fma(M.m[1][m], b, fma(M.m[0][m], a, ub[m * N + t])));
 }
 
-// ---- nodal projection adjoint: out = ub + Gn psi
-__global__ void k_adj_nodal_post(Grid g, const double* psi, const double* ub, double* out) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N) return;
-    const int i = (int)(t % g.nx);
-    const long long r = t / g.nx;
-    const int j = (int)(r % g.ny), k = (int)(r / g.ny);
-    auto P = [&](int a, int b, int c) {
-        return psi[((long long)(g.zper ? wrapn(c, g.nz) : c) * g.ny + wrapn(b, g.ny)) * g.nx + wrapn(a, g.nx)];
-    };
-    double gx = 0, gy = 0, gz = 0;
-    for (int c = 0; c < 2; ++c)
-        for (int b = 0; b < 2; ++b) {
-            gx += P(i + 1, j + b, k + c) - P(i, j + b, k + c);
-            gy += P(i + b, j + 1, k + c) - P(i + b, j, k + c);
-            gz += P(i + b, j + c, k + 1) - P(i + b, j + c, k);
-        }
-    out[t] = ub[t] + 0.25 * gx * g.idx;
-    out[g.N + t] = ub[g.N + t] + 0.25 * gy * g.idy;
-    out[2 * g.N + t] = ub[2 * g.N + t] + 0.25 * gz * g.idz;
+// ---- nodal projection adjoint: out = ub + Gn psi.  Bound by FP64 issue: a column is
+// marched in z, a node layer's x and y differences are formed once for the two cell
+// layers they border, q = 1 / (4 h): 18 FP64 instructions a cell, 30 when every
+// cell formed its own (256x256x128: 486 us, 307 now).
+__global__ void __launch_bounds__(128) k_adj_nodal_post(Grid g, const double* psi, const double* ub, double* out, double qx, double qy, double qz,
+                                                        int kc) {
+    int i, j;
+    if (!column_of(g, i, j)) return;
+    const int k0 = blockIdx.y * kc, k1 = min(k0 + kc, g.nz);
+    const int sz = g.nx * g.ny;
+    const int xp = i + 1 == g.nx ? 1 - g.nx : 1, yp = (j + 1 == g.ny ? 1 - g.ny : 1) * g.nx;
+    const double* p = psi + (long long)k0 * sz + j * g.nx + i;
+    double a = p[0], b = p[xp], c = p[yp], d = p[xp + yp];
+    double gx = (b - a) + (d - c), gy = (c - a) + (d - b);
+    long long t = (long long)k0 * sz + j * g.nx + i;
+    for (int k = k0; k < k1; ++k, t += sz) {
+        p = psi + (long long)(g.zper && k + 1 == g.nz ? 0 : k + 1) * sz + j * g.nx + i;
+        const double a1 = p[0], b1 = p[xp], c1 = p[yp], d1 = p[xp + yp];
+        const double gx1 = (b1 - a1) + (d1 - c1), gy1 = (c1 - a1) + (d1 - b1), gz = ((a1 - a) + (b1 - b)) + ((c1 - c) + (d1 - d));
+        out[t] = fma(qx, gx + gx1, ub[t]);
+        out[g.N + t] = fma(qy, gy + gy1, ub[g.N + t]);
+        out[2 * g.N + t] = fma(qz, gz, ub[2 * g.N + t]);
+        a = a1;
+        b = b1;
+        c = c1;
+        d = d1;
+        gx = gx1;
+        gy = gy1;
+    }
 }
 
 // ---- elementwise helpers
@@ -1456,9 +1462,8 @@ __global__ void k_objective(Grid g, const double* u, int lo0, int lo1, int lo2, 
     __shared__ double sh[256];
     double s = 0.0;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < g.N; t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t % g.nx);
-        const long long r = t / g.nx;
-        const int j = (int)(r % g.ny), k = (int)(r / g.ny);
+        int i, j, k;
+        face_at(g, 0, t, i, j, k);
         const bool in = i >= lo0 && i <= hi0 && j >= lo1 && j <= hi1 && k >= lo2 && k <= hi2;
         for (int n = 0; n < 3; ++n) {
             const double v = u[n * g.N + t];
@@ -1682,10 +1687,15 @@ void launch_adj_wall_global(Ctx& c, const Grid& g, const double* vel, double bu,
     KS_LAUNCH(c, k_adj_wall_global, nblocks(M, BS), BS, B8 * 6.0 * M, g, vel, bu, bv, bm, ub);
 }
 void launch_adj_coriolis(Ctx& c, const Grid& g, const double* srcb, const Scalars& s, double* ub) {
-    KS_LAUNCH(c, k_adj_coriolis, nblocks(g.N, BS), BS, B8 * 9.0 * g.N, g, srcb, s, ub);
+    Map3 M;
+    for (int n = 0; n < 3; ++n)
+        for (int m = 0; m < 3; ++m) M.m[n][m] = coriolis_map(s, n, m);
+    KS_LAUNCH(c, k_adj_coriolis, nblocks(g.N, BS), BS, B8 * 9.0 * g.N, g.N, srcb, M, ub);
 }
 void launch_adj_nodal_post(Ctx& c, const Grid& g, const double* psi, const double* ub, double* out) {
-    KS_LAUNCH(c, k_adj_nodal_post, nblocks(g.N, BS), BS, B8 * 7.0 * g.N, g, psi, ub, out);
+    const int kc = march_layers(g, 2048);
+    KS_LAUNCH(c, k_adj_nodal_post, column_grid(g, kc), column_threads(g), B8 * 7.0 * g.N, g, psi, ub, out, 0.25 * g.idx, 0.25 * g.idy,
+              0.25 * g.idz, kc);
 }
 void launch_axpby(Ctx& c, long long n, double a, const double* x, double b, const double* y, double* out) {
     KS_LAUNCH(c, k_axpby, nblocks(n, BS), BS, B8 * 3.0 * n, n, a, x, b, y, out);

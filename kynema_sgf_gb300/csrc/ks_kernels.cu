@@ -1322,8 +1322,7 @@ void launch_sources(Ctx& c, const Grid& g, const double* vel_old, const double* 
         k.c[n] = s.rho * a;
         k.bous_g[n] = s.rho * s.grav[n] * s.beta_T;
         for (int m = 0; m < 3; ++m)
-            k.M[n][m] = s.rho * s.corfac *
-                        (s.sinphi * (s.east[n] * s.north[m] - s.north[n] * s.east[m]) + s.hfac * s.cosphi * (s.up[n] * s.east[m] - s.east[n] * s.up[m]));
+            k.M[n][m] = coriolis_map(s, n, m);
     }
     using Kern = void (*)(Grid, const double*, const double*, const double*, double*, SrcCoef, const double*);
     static const Kern kern[2][8] = {{k_sources<0, 0, 0, 0>, k_sources<1, 0, 0, 0>, k_sources<0, 1, 0, 0>, k_sources<1, 1, 0, 0>,

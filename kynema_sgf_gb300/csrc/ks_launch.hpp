@@ -371,6 +371,11 @@ void launch_adj_smag(Ctx& c, const Grid& g, const double* vel, const double* mub
 void launch_adj_wall_local(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wgb, double ut2, double um0, double um1,
                            double vm, double rho, double* ub, double* mub, double* parts, int* np);
 void launch_adj_wall_global(Ctx& c, const Grid& g, const double* vel, double bu, double bv, double bm, double* ub);
+// entry of the linear map rho (Coriolis acceleration), see launch_sources
+inline double coriolis_map(const Scalars& s, int n, int m) {
+    return s.rho * s.corfac *
+           (s.sinphi * (s.east[n] * s.north[m] - s.north[n] * s.east[m]) + s.hfac * s.cosphi * (s.up[n] * s.east[m] - s.east[n] * s.up[m]));
+}
 void launch_adj_coriolis(Ctx& c, const Grid& g, const double* srcb, const Scalars& s, double* ub);
 void launch_adj_nodal_post(Ctx& c, const Grid& g, const double* psi, const double* ub, double* out);
 void launch_axpby(Ctx& c, long long n, double a, const double* x, double b, const double* y, double* out);
