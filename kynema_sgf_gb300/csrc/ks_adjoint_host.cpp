@@ -245,9 +245,9 @@ void Sim::adjoint_step_impl(bool seed) {
     } restore{*this, t_};
     // The linearisation point is the handle's own forward step, recomputed
     // at its precision: a mixed-precision handle's reverse kernels read the
-    // FP32 Godunov intermediates its forward used (and accumulate in FP64);
-    // its multigrid keeps FP32 cycles under the FP64 defect correction, here
-    // and in the two reverse solves.  The post-MAC pass writes its own
+    // FP32 Godunov intermediates its forward used (and accumulate in FP64); its
+    // forward solves keep FP32 cycles under the FP64 defect correction, its two
+    // reverse solves start from the direct solution.  The post-MAC pass writes its own
     // buffers so that the pre-MAC intermediates survive for the reverse.
     adv_bufs_ = &S.gb2;
     const int fp32 = mixed_;
