@@ -258,8 +258,13 @@ __device__ inline T sel(const T (&a)[NC], int n) {
 
 // y (d = 1) and z (d = 2) faces: one thread per (i, transverse index, chunk of
 // faces along d).  Face m lies between cells m-1 and m.
+// Six blocks of 128 threads on an SM (80 registers, 24 bytes of spills in the FP64
+// pre-MAC form): a march is one dependent chain of FP64 instructions, and with 116
+// registers and half the warps it left a fifth of the FP64 issue slots empty
+// (256x256x128, mean of the four passes: 763 us with blocks of 256 and no bound,
+// 741, 676, 663 with 4, 5, 6 blocks; FP32 211 and 208).
 template <typename T, int NC, int MODE, int EDGES>
-__global__ void __launch_bounds__(256) k_ppm_col(PpmArgs<T> A, T s, T rho, PpmOut<T, NC> O, int chunk) {
+__global__ void __launch_bounds__(128, 6) k_ppm_col(PpmArgs<T> A, T s, T rho, PpmOut<T, NC> O, int chunk) {
     const Grid& g = A.g;
     const int d = A.d;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -855,7 +860,7 @@ static void launch_ppm(Ctx& c, const Grid& g, int d, const T* vel, const T* umac
         const int nf = (d == 2) ? nzfaces(g) : g.ny;
         const int most = march_chunk<T>(g, 2, 32);
         const int nch = (nf + most - 1) / most, chunk = (nf + nch - 1) / nch;
-        const int bx = g.nx >= BS ? BS : 32 * ((g.nx + 31) / 32);
+        const int bx = g.nx >= 128 ? 128 : 32 * ((g.nx + 31) / 32);
         const dim3 grid((unsigned)((g.nx + bx - 1) / bx), (unsigned)((d == 1 ? g.nz : g.ny) * nch));
         KS_LAUNCH(c, (k_ppm_col<T, NC, MODE, EDGES>), grid, bx, bytes, A, s, T(rho), O, chunk);
     }
