@@ -239,8 +239,9 @@ __device__ const double kEdgeW[34] = {
 // thread re-evaluates those four faces' slopes and clips from the seven cells
 // c - 3 .. c + 3 (cheap in the pass precision) and owns the cell's adjoint.
 // With a wall-bounded z only the faces 2 .. nz - 2 are gathered.
+// 128x128x64 FP64: 203 us with two blocks an SM, 196 with three (80 registers).
 template <typename TI>
-__global__ void __launch_bounds__(256, 2) k_adj_edges_gather(Grid g, int d, const double* u, const double* Eb0, const double* Eb1, const double* Eb2, double* ub) {
+__global__ void __launch_bounds__(256, 3) k_adj_edges_gather(Grid g, int d, const double* u, const double* Eb0, const double* Eb1, const double* Eb2, double* ub) {
     using A = TI;
     int i, j, k;
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -556,8 +557,11 @@ __device__ inline void face_state_rev(const Grid& g, int d, long long f, int kf,
         for (int n = 0; n < 3; ++n) zbc_rev(g, kf, n, lb[n], hb[n]);
 }
 
+// FP64 issue of long dependent chains: 128x128x64 FP64, before and after the MAC
+// projection 309 and 303 us with two blocks an SM, 271 and 281 with three (80
+// registers); FP32 takes 64 to 72 registers either way.
 template <int MODE, typename TI>
-__global__ void __launch_bounds__(256, 2) k_adj_faces_cells(Grid g, int d, const double* u, KI<TI> E, double s, double rho, const double* umac_d,
+__global__ void __launch_bounds__(256, 3) k_adj_faces_cells(Grid g, int d, const double* u, KI<TI> E, double s, double rho, const double* umac_d,
                                                             KI<TI> LO, KI<TI> HI, const TI* ad, K3 LOb, K3 HIb, const double* adb, K3 TEb,
                                                             double* ub, TI* G) {
     using A = TI;
