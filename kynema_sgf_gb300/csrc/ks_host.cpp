@@ -638,24 +638,35 @@ void Sim::mac_semi_mixed() {
 //   - on counts with a prime factor above 13 or above kSpectralMax.
 // The start depends on the right-hand side alone, so a restart repeats it bit
 // for bit.
+//
+// znod_ / zmac_ (their dinv) are set when the factors are complete and at no
+// other time: a set-up that fails, for want of memory or because the runtime
+// refuses a call (a device-wide wait while a stream is captured), keeps nothing,
+// the solves take the multigrid, and the next set-up starts anew.
 bool Sim::spectral_setup(bool nodal) {
-    SpectralZ& Z = nodal ? znod_ : zmac_;
-    DevBuf<double>& F = nodal ? spec_nod_ : spec_mac_;
-    if (F.p) return true;
+    if ((nodal ? znod_ : zmac_).dinv) return true;
     int np, r[12];
     if (!mg_warm_ || (nodal ? nod_ : mac_).maxiter < MGParams().maxiter || !spectral_radices(g_.nx, np, r) || !spectral_radices(g_.ny, np, r))
         return false;
+    try {
+        spectral_factors(nodal);
+        return true;
+    } catch (const KsError&) {
+    } catch (const std::bad_alloc&) {
+    }
+    (void)cudaGetLastError();
+    (nodal ? spec_nod_ : spec_mac_).reset();
+    return false;
+}
+
+void Sim::spectral_factors(bool nodal) {
+    SpectralZ Z{};
+    DevBuf<double>& F = nodal ? spec_nod_ : spec_mac_;
     const int nx = g_.nx, ny = g_.ny, na = nx / 2 + 1, nk = ny / 2 + 1;
     const size_t M = (size_t)na * nk, nz = nodal ? nd_[0].nz : g_.nz;
-    try {
-        if (!spectral_prepare_device()) throw KsError(KS_ERR_CUDA, "shared memory of the transforms");
-        if (!spec_tab_.p) spec_tab_.alloc(2 * (size_t)(nx + ny + na + nk));
-        F.alloc(nz * M * (g_.zper ? 2 : 1) + (g_.zper ? M : 0));
-    } catch (const KsError&) {  // no room for the factors: the multigrid solves need none
-        (void)cudaGetLastError();
-        F.reset();
-        return false;
-    }
+    if (!spectral_prepare_device()) throw KsError(KS_ERR_CUDA, "shared memory of the transforms");
+    if (!spec_tab_.p) spec_tab_.alloc(2 * (size_t)(nx + ny + na + nk));
+    F.alloc(nz * M * (g_.zper ? 2 : 1) + (g_.zper ? M : 0));
     // roots exp(-2 pi i q / n), then (2 - 2 cos) / h^2 and (2 + cos) / 3 per direction
     const double pi = 3.14159265358979323846;
     std::vector<double> t;
@@ -691,9 +702,11 @@ bool Sim::spectral_setup(bool nodal) {
     Z.dinv = F.p;
     Z.w = g_.zper ? F.p + nz * M : nullptr;
     Z.schur = g_.zper ? F.p + 2 * nz * M : nullptr;
+    (void)cudaGetLastError();  // an older call's, reported there
     launch_spectral_setup(ctx_, Z);
+    ck(cudaGetLastError(), "spectral factors");
     sync();  // t is read by the copy
-    return true;
+    (nodal ? znod_ : zmac_) = Z;
 }
 
 // the rule of the step's solves (see above)

@@ -415,6 +415,7 @@ class Sim {
     // direct start of the Poisson solves: the factors of one operator (false: not available),
     // and the solves of a step that take it
     bool spectral_setup(bool nodal);
+    void spectral_factors(bool nodal);
     void spectral_choose();
     void spectral_start(const SpectralZ& Z, const double* rhs, double* phi, double coef, int np);
     void spectral_norms(int np, double& bnorm, double& rnorm);
