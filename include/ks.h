@@ -89,6 +89,9 @@ int ks_step(ks_handle* h);
 int ks_field_layout(ks_handle* h, const char* name, ks_layout* layout);
 int ks_get_field(ks_handle* h, const char* name, void* dst, ks_memory where);
 int ks_set_field(ks_handle* h, const char* name, const void* src, ks_memory where);
+/* "mac_direct" / "nodal_direct": 1 where the last Poisson solve began at the direct solution (by
+ * transforms), 0 where V-cycles began at an older result or at zero; a handle whose factors find no room
+ * in device memory goes on with the latter, whose fields differ within the solver tolerance. */
 int ks_get_scalar(ks_handle* h, const char* name, double* value);
 int ks_last_solver_stats(const ks_handle* h, ks_mg_stats* stats);
 int ks_set_precision(ks_handle* h, int precision);

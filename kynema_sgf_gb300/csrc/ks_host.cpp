@@ -637,7 +637,8 @@ void Sim::mac_semi_mixed() {
 //     and so ask for those iterates;
 //   - on counts with a prime factor above 13 or above kSpectralMax.
 // The start depends on the right-hand side alone, so a restart repeats it bit
-// for bit.
+// for bit where its handle starts directly too: the scalars "mac_direct" and
+// "nodal_direct" say whether the last solve did.
 //
 // znod_ / zmac_ (their dinv) are set when the factors are complete and at no
 // other time: a set-up that fails, for want of memory or because the runtime
@@ -1350,6 +1351,7 @@ void Sim::mac_project() {
     if (rn > target && !mac_.fixed_iters) throw KsError(KS_ERR_NOT_CONVERGED, "MAC projection did not converge in mac_proj.maxiter V-cycles");
     mac_it_ = it;
     mac_r_ = rn;
+    mac_started_ = direct;
     launch_mac_correct(ctx_, g_, L.phi, umac_[0].p, umac_[1].p, umac_[2].p, beta, mixed_);
     if (direct) {  // nothing but the next MAC solve writes L.phi
         mac_phi_last_ = L.phi;
@@ -1420,7 +1422,8 @@ void Sim::nd_solve(double sigma) {
     int np = 0;
     for (auto& Lv : nd_) Lv.inv_diag = 1.0 / (sigma * Lv.W[13]);
     for (size_t l = 0; l < nd32_.size(); ++l) nd32_[l].inv_diag = (float)nd_[l].inv_diag;
-    if (direct_start(nod_direct_ || nod_alone_)) {
+    nod_started_ = direct_start(nod_direct_ || nod_alone_);
+    if (nod_started_) {
         spectral_start(znod_, L.rhs, L.phi, sigma, nod_bparts_);
         launch_nd_resid(ctx_, L, sigma, parts_.p, &np);
         spectral_norms(np, nod_bnorm_, nod_r_);
@@ -2007,6 +2010,8 @@ double Sim::scalar(const std::string& n) {
     if (n == "step") return t_.step;
     if (n == "mac_iters") return mac_it_;
     if (n == "nodal_iters") return nod_it_;
+    if (n == "mac_direct") return mac_started_;      // 1: the last solve began at the direct solution
+    if (n == "nodal_direct") return nod_started_;
     if (n == "mac_levels") return (double)(mac_semi_ ? ccs_ : cc_).size();
     if (n.rfind("mac_level:", 0) == 0) {  // mac_level:l:d, cells of MAC level l in direction d
         const std::vector<CCLevelDev>& M = mac_semi_ ? ccs_ : cc_;

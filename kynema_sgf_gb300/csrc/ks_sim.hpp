@@ -421,6 +421,7 @@ class Sim {
     void spectral_norms(int np, double& bnorm, double& rnorm);
     int nod_bparts_ = 0;  // block maxima of |rhs| that nd_rhs left in parts_ for the direct start
     bool mac_direct_ = false, nod_direct_ = false;
+    bool mac_started_ = false, nod_started_ = false;  // the last solves did
     bool nod_alone_ = false;  // inside projection_alone, with the nodal factors at hand
     bool adj_direct_ = false;  // the reverse mode of a handle whose solves may start directly
     bool reverse_ = false;     // inside the two solves of a reverse step

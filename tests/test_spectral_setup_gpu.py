@@ -42,9 +42,23 @@ def test_setup_that_fails_half_way(cuda_dev):
     finally:
         cu.cuStreamEndCapture(stream, ctypes.byref(graph))
         cu.cuStreamDestroy_v2(stream)
-    assert sim.scalar("nodal_iters") > 0
+    assert sim.scalar("nodal_iters") > 0 and sim.scalar("nodal_direct") == 0
     after = project(sim, u)
-    assert sim.scalar("nodal_iters") == 0
+    assert sim.scalar("nodal_iters") == 0 and sim.scalar("nodal_direct") == 1
     # the same operations on the same input: the same bits; the multigrid stops at 2.2e-11 of the right-hand side
     assert np.array_equal(after, want)
     assert np.abs(during - want).max() <= 1e-8 * np.abs(want).max()
+
+
+def test_scalars_tell_the_start(cuda_dev):
+    cubic, flat = cuda_dev.Incflo(decks.abl(*N, steps=2)), cuda_dev.Incflo(decks.abl(*N, steps=2, dz=10.0))
+    for sim in (cubic, flat):
+        sim.InitData()
+        assert sim.step()
+        for s in ("mac_direct", "nodal_direct"):
+            assert sim.scalar(s) == float(sim is flat)
+    cubic.ApplyProjection(0.0, 0.7, False)
+    assert cubic.scalar("mac_direct") == 0 and cubic.scalar("nodal_direct") == 1
+    flat.set_precision(1)
+    assert flat.step()
+    assert flat.scalar("mac_direct") == 0 and flat.scalar("nodal_direct") == 0
