@@ -187,7 +187,7 @@ __device__ __forceinline__ double isign(double m, double s) {
 // NaN becomes a quiet NaN.  What is not zero or normal in FP32 takes the call.
 // They pay in kernels bound by FP64 issue (viscous tile on 256x256x128: 520 us
 // with conversions, 450 with these); kernels that wait on memory keep the
-// conversion (k_add_f32 37 us against 41, k_adj_edges_gather 573 against 769).
+// conversion (k_adj_edges_gather 573 us, 769 with these).
 static __device__ __noinline__ float d2f_rare(double x) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     const unsigned m = ((hi & 0xfffffu) << 3) | (lo >> 29), r = lo & 0x1fffffffu;
@@ -220,6 +220,8 @@ static __device__ __noinline__ double f2d_rare(float x) {
         const int s = __clz((int)m) - 8;  // normalise
         m = (m << s) & 0x7fffffu;
         e = 1u - (unsigned)s;
+    } else if (m) {
+        m |= 0x400000u;
     }
     return __hiloint2double((int)(sign | ((e + 896u) << 20) | (m >> 3)), (int)(m << 29));
 }

@@ -44,11 +44,13 @@ __device__ inline bool nonzero(double x) { return (dbits(x) & kMag) != 0; }
 __device__ inline bool nonzero(float x) { return x != 0.0f; }
 
 // The FP64 forms below spend fewer FP64 instructions: scaling by a power of two
-// is an addition to the exponent field (a result below the normal range becomes
-// zero), and a choice is made before the arithmetic it selects, for an
-// instruction that is predicated off still takes its FP64 issue slot.
+// is an addition to the exponent field, and a choice is made before the
+// arithmetic it selects, for an instruction that is predicated off still takes
+// its FP64 issue slot.  At the ends of the range a half below the normal numbers
+// becomes zero, twice a subnormal a normal number of at most 2^-1021, and twice
+// 2^1023 or more no infinity.
 constexpr long long kExp1 = 1LL << 52;
-__device__ inline double twice(double x) { return hiword(x, __double2hiint(x) + 0x00100000); }  // x finite, not 0
+__device__ inline double twice(double x) { return hiword(x, __double2hiint(x) + 0x00100000); }  // x normal, below 2^1023
 __device__ inline double half_fin(double x) {  // x finite
     const int h = __double2hiint(x);
     return (h & 0x7fffffff) >= 0x00200000 ? hiword(x, h - 0x00100000) : 0.0;
