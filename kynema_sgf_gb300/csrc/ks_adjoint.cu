@@ -673,7 +673,7 @@ __global__ void k_adj_pm_trans(Grid g, int a, int b, int n, double cb64, const T
     }
 }
 
-// forces with the first-order extrapolated ghosts of CellFOT and the adjoint
+// cell of a field with first-order extrapolated ghosts in z (forces)
 __device__ inline long long cell_fo(const Grid& g, int i, int j, int k) {
     i = wrapn(i, g.nx);
     j = wrapn(j, g.ny);

@@ -105,21 +105,6 @@ struct VelFPT {
 };
 using VelFP = VelFPT<double>;
 
-// Cell field with first-order extrapolation ghosts in z (forces, viscosity).
-template <typename T = double, typename S = double>
-struct CellFOT {
-    const S* v;
-    Grid g;
-    __device__ inline T operator()(int n, int i, int j, int k) const {
-        i = wrapn(i, g.nx);
-        j = wrapn(j, g.ny);
-        if (g.zper) k = wrapn(k, g.nz);
-        else k = k < 0 ? 0 : (k >= g.nz ? g.nz - 1 : k);
-        return (T)v[n * g.N + cidx(g, i, j, k)];
-    }
-};
-using CellFO = CellFOT<double>;
-
 #endif
 
 inline unsigned nblocks(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }

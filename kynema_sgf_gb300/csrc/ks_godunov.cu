@@ -18,8 +18,6 @@
 // taken on the integer pipe (ks_common.cuh).  Post-MAC states of rho*u are rho
 // times the traces of u (the PPM limiter and the traces are homogeneous of
 // degree one in the advected field).
-#include <algorithm>
-
 #include "ks_decide.cuh"
 #include "ks_launch.hpp"
 

@@ -108,43 +108,13 @@ __global__ void k_copy(double* d, const double* s, long long n) {
 // mu_eff = mu + rho Cs^2 Delta^2 |S| (src/turbulence/LES/Smagorinsky.cpp:22-62,
 // strain rate src/fvm/strainrate.H:24-86, one-sided z stencils at walls
 // src/fvm/stencils.H:166-330).
-// alpha_eff = mu / Pr + mu_t / Pr_t (TurbModelBase.H:28-35) when alpha is set
-// T is the arithmetic type: double, or float in the mixed-precision form (the
-// strain rate of the FP64 velocity read once per cell and rounded; mu_eff is
-// stored in FP64).
-template <typename T>
-__global__ void k_smag(Grid g, const double* vel, double* mueff, double mu, double rho, double fac, int smag, double* alpha, double mu_pr,
-                       double iprt) {
+// alpha_eff = mu / Pr + mu_t / Pr_t (TurbModelBase.H:28-35) when alpha is set.
+// Where the model is off both are the molecular values.
+__global__ void k_mu_molecular(long long N, double* mueff, double mu, double* alpha, double mu_pr) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N) return;
-    if (!smag) {
-        mueff[t] = mu;
-        if (alpha) alpha[t] = mu_pr;
-        return;
-    }
-    int i, j, k;
-    cell_of(g, t, i, j, k);
-    VelFPT<T, double> V{vel, g, T(1)};
-    const T hx = T(0.5 * g.idx), hy = T(0.5 * g.idy);
-    T gx[3], gy[3], gz[3];
-    for (int n = 0; n < 3; ++n) {
-        gx[n] = hx * (V(n, i + 1, j, k) - V(n, i - 1, j, k));
-        gy[n] = hy * (V(n, i, j + 1, k) - V(n, i, j - 1, k));
-    }
-    if (!g.zper && (k == 0 || k == g.nz - 1)) {  // one-sided through the wall (ghost) value
-        T a = T(1.0 / 3.0), b = T(1), c = T(-4.0 / 3.0);
-        if (k == g.nz - 1) { a = T(4.0 / 3.0); b = T(-1); c = T(-1.0 / 3.0); }
-        const T iz = T(g.idz);
-        for (int n = 0; n < 3; ++n) gz[n] = (a * V(n, i, j, k + 1) + b * V(n, i, j, k) + c * V(n, i, j, k - 1)) * iz;
-    } else {
-        const T hz = T(0.5 * g.idz);
-        for (int n = 0; n < 3; ++n) gz[n] = hz * (V(n, i, j, k + 1) - V(n, i, j, k - 1));
-    }
-    const T sxy = gy[0] + gx[1], syz = gz[1] + gy[2], szx = gx[2] + gz[0];
-    const T s = sqrt(T(2) * (gx[0] * gx[0] + gy[1] * gy[1] + gz[2] * gz[2]) + (sxy * sxy + syz * syz + szx * szx));
-    const double mut = (rho * fac) * (double)s;
-    mueff[t] = mu + mut;
-    if (alpha) alpha[t] = mu_pr + iprt * mut;
+    if (t >= N) return;
+    mueff[t] = mu;
+    if (alpha) alpha[t] = mu_pr;
 }
 
 // FP64 form: columns marched in z, the column's own values carried and the
@@ -1289,19 +1259,18 @@ void launch_smagorinsky(Ctx& c, const Grid& g, const double* vel, double* mueff,
                         const float* vel32) {
     if (!s.temp) alpha = nullptr;
     const double bytes = B8 * ((s.smag ? 4 : 1) + (alpha ? 1 : 0)) * g.N;
-    if (fp32 && s.smag) {
+    if (!s.smag) {
+        KS_LAUNCH(c, k_mu_molecular, nblocks(g.N, BS), BS, bytes, g.N, mueff, s.mu, alpha, s.mu_pr);
+    } else if (fp32) {
         // layers a march: 16, fewer where that leaves less than 4096 warps
         const int kc = march_layers(g, 4096);
         KS_LAUNCH(c, k_smag_march, column_grid(g, kc), column_threads(g), bytes - 12.0 * g.N, g, vel32, mueff, s.mu, s.rho * s.smag_fac,
                   alpha, s.mu_pr, s.iprt, kc);
-    } else if (fp32)
-        KS_LAUNCH(c, k_smag<float>, nblocks(g.N, BS), BS, bytes, g, vel, mueff, s.mu, s.rho, s.smag_fac, s.smag, alpha, s.mu_pr, s.iprt);
-    else if (s.smag) {
+    } else {
         // layers a march: 16, fewer where that leaves less than 2048 warps
         const int kc = march_layers(g, 2048);
         KS_LAUNCH(c, k_smag_col, column_grid(g, kc), column_threads(g), bytes, g, vel, mueff, s.mu, s.rho * s.smag_fac, alpha, s.mu_pr, s.iprt, kc);
-    } else
-        KS_LAUNCH(c, k_smag<double>, nblocks(g.N, BS), BS, bytes, g, vel, mueff, s.mu, s.rho, s.smag_fac, s.smag, alpha, s.mu_pr, s.iprt);
+    }
 }
 // src = rho (-gp/rho + geostrophic + Coriolis(u_old) + body + actuator + Boussinesq + ABLForcing)
 // (icns_ops.H:78-124, PDEOps.H:94-145, GeostrophicForcing.cpp:103-, CoriolisForcing.cpp:60-108,

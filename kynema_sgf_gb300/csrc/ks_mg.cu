@@ -455,15 +455,6 @@ __global__ void k_bottom_direct(const T* __restrict__ binv, int n, const T* rhs,
 }
 
 // ---------------------------------------------------------------- nodal
-template <typename T>
-__device__ inline T nd_at(const NDLevelT<T>& L, const T* p, int i, int j, int k) {
-    i = i < 0 ? i + L.nx : (i >= L.nx ? i - L.nx : i);
-    j = j < 0 ? j + L.ny : (j >= L.ny ? j - L.ny : j);
-    if (L.zper) k = k < 0 ? k + L.nz : (k >= L.nz ? k - L.nz : k);
-    else k = k < 0 ? -k : (k >= L.nz ? 2 * (L.nz - 1) - k : k);
-    return p[(k * L.ny + j) * L.nx + i];
-}
-
 // sigma * (27-point Q1 stencil) at node (i,j,k); the weights are symmetric in
 // each direction, so neighbours are summed by weight class first.
 template <typename T>
