@@ -579,13 +579,19 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
 // faces need, and the upper row's faces); one for the columns left (lanes 0 ..)
 // and right (lanes 16 ..) of the block.
 // On 256x256x128: 2.25 ms as tiles (96 % of the FP64 issue rate), 1.50 ms now.
-template <int TY>
+//
+// WX < 32 (boxes of at most 16 columns in x, MODE 0): a warp holds 32 / WX rows
+// of WX columns, a block one such warp and the three of the halo.  On 32 lanes
+// a row of 4 leaves 28 idle: 4x256x256 351 us and 4x4x16384 621, where fluxes
+// formed face by face take 158 and 146 (193 and 183 under walls); 66 and 129 now.
+template <int TY, int WX>
 struct TauPlanes {
-    double V[3][3][TY + 2][34];   // [layer mod 3][component]: row and column 0 are the halo
-    double M[2][TY + 2][34];      // [layer mod 2]
-    double QX[3][TY][34];         // cell differences for x faces: divergence part, du/dy, du/dz
-    double QY[3][TY + 2][32];     // for y faces: divergence part, dv/dx, dv/dz
-    double FX[3][TY][33], FY[3][TY + 1][32];
+    static constexpr int NR = TY * (32 / WX);  // rows of a block
+    double V[3][3][NR + 2][WX + 2];  // [layer mod 3][component]: row and column 0 are the halo
+    double M[2][NR + 2][WX + 2];     // [layer mod 2]
+    double QX[3][NR][WX + 2];        // cell differences for x faces: divergence part, du/dy, du/dz
+    double QY[3][NR + 2][WX];        // for y faces: divergence part, dv/dx, dv/dz
+    double FX[3][NR][WX + 1], FY[3][NR + 1][WX];
 };
 struct TauCoef {                  // spacing ratios (see k_divtau_col)
     double gx, gy, gz;            // 1 / (2 h^2)
@@ -599,21 +605,25 @@ inline TauCoef tau_coef(const Grid& g) {
                    0.25 * z / x,        0.25 * z / y,        -0.125 * x / y,      -0.125 * y / x, -0.125 * z / x, y / z, x / z, x / y};
 }
 
+constexpr int kNarrowBlocks = 6;  // blocks of the narrow forms on an SM
+
 // MODE (TauEpi) is a template argument: the other modes' instructions, predicated
 // off, took 7 of 92 FP64 issue slots a cell.
-template <int TY, int MODE>
-__global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef K, const double* vel, const double* mueff, const double* wg, double* out,
-                                                             TauEpi E, int kc) {
+template <int TY, int MODE, int WX>
+__global__ void __launch_bounds__(32 * (TY + 3), WX == 32 ? 2 : kNarrowBlocks) k_divtau_col(Grid g, TauCoef K, const double* vel, const double* mueff,
+                                                                                           const double* wg, double* out, TauEpi E, int kc) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
-    TauPlanes<TY>& S = *reinterpret_cast<TauPlanes<TY>*>(sm_raw);
+    TauPlanes<TY, WX>& S = *reinterpret_cast<TauPlanes<TY, WX>*>(sm_raw);
+    constexpr int NR = TauPlanes<TY, WX>::NR;
+    static_assert((NR + 2) * (WX + 2) <= 32 * (TY + 3), "a thread stages one column");
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
-    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * TY, k0 = blockIdx.z * kc, k1 = min(k0 + kc, g.nz);
+    const int i0 = blockIdx.x * WX, j0 = blockIdx.y * NR, k0 = blockIdx.z * kc, k1 = min(k0 + kc, g.nz);
     const long long N = g.N;
     const int sz = g.nx * g.ny;
-    // ---- staging: thread tid loads one column of the (TY + 2) x 34 footprint
+    // ---- staging: thread tid loads one column of the (NR + 2) x (WX + 2) footprint
     // (a block may be wider than the grid: x and y wrap fully)
-    const bool loads = tid < (TY + 2) * 34;
-    const int lx = tid % 34, ly = tid / 34;
+    const bool loads = tid < (NR + 2) * (WX + 2);
+    const int lx = tid % (WX + 2), ly = tid / (WX + 2);
     const int col = loads ? (((j0 + ly - 1) % g.ny + g.ny) % g.ny) * g.nx + ((i0 + lx - 1) % g.nx + g.nx) % g.nx : 0;
     struct Cell {
         double v[3], m;
@@ -643,7 +653,15 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
     }
     __syncthreads();
     const bool mainw = w < TY;
-    const int y = w + 1, x = l + 1;
+    const int y = w * (32 / WX) + l / WX + 1, x = l % WX + 1;
+    // the halo's warps: lanes of the rows below and above, then of the columns
+    // left and right of the block
+    constexpr int kSide = 2 * WX < 32 ? 32 : 2 * WX, kHalf = NR < 16 ? 16 : NR;
+    static_assert(kSide + 2 * kHalf <= 96, "three warps hold the halo");
+    const int h = tid - 32 * TY, hq = h - kSide;
+    const int yh = h < WX ? 0 : NR + 1, xh = h % WX + 1;
+    const int sr = hq % kHalf, sx = hq < kHalf ? 0 : WX + 1;
+    const bool side = hq >= 0 && hq < 2 * kHalf && sr < NR;
     if (mainw) mu = S.M[(k0 - 1) & 1][y][x];
     __syncthreads();
     if (loads) {
@@ -705,10 +723,8 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
         zflux(pm, pc, mu + m0, fz);
         mu = m0;
     }
-    const int i = i0 + l, j = j0 + w;
+    const int i = i0 + x - 1, j = j0 + y - 1;
     const bool live = mainw && i < g.nx && j < g.ny;
-    const int sr = l & 15, sx = l < 16 ? 0 : 33;  // the side warp's row and column
-    const bool side = w == TY + 2 && sr < TY;
     long long rmax = 0;
     for (int k = k0; k < k1; ++k) {
         const int m = k & 1;
@@ -724,13 +740,12 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
             zflux(pc, pn, mu + mn, fzn);
             mu = mn;
             xcell(y, x, pc.dy, q);
-            for (int n = 0; n < 3; ++n) S.QX[n][w][x] = q[n];
+            for (int n = 0; n < 3; ++n) S.QX[n][y - 1][x] = q[n];
             ycell(y, x, pc.dx, q);
-            for (int n = 0; n < 3; ++n) S.QY[n][y][l] = q[n];
-        } else if (w < TY + 2) {
-            const int yy = w == TY ? 0 : TY + 1;
-            ycell(yy, x, S.V[sc][0][yy][x + 1] - S.V[sc][0][yy][x - 1], q);
-            for (int n = 0; n < 3; ++n) S.QY[n][yy][l] = q[n];
+            for (int n = 0; n < 3; ++n) S.QY[n][y][x - 1] = q[n];
+        } else if (h < 2 * WX) {
+            ycell(yh, xh, S.V[sc][0][yh][xh + 1] - S.V[sc][0][yh][xh - 1], q);
+            for (int n = 0; n < 3; ++n) S.QY[n][yh][xh - 1] = q[n];
         } else if (side) {
             xcell(sr + 1, sx, S.V[sc][1][sr + 2][sx] - S.V[sc][1][sr][sx], q);
             for (int n = 0; n < 3; ++n) S.QX[n][sr][sx] = q[n];
@@ -742,15 +757,15 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
             xflux(y, x, m, fx);
             yflux(y, x, m, fy);
             for (int n = 0; n < 3; ++n) {
-                S.FX[n][w][l] = fx[n];
-                S.FY[n][w][l] = fy[n];
+                S.FX[n][y - 1][x - 1] = fx[n];
+                S.FY[n][y - 1][x - 1] = fy[n];
             }
-        } else if (w == TY + 1) {
-            yflux(TY + 1, x, m, fy);
-            for (int n = 0; n < 3; ++n) S.FY[n][TY][l] = fy[n];
+        } else if (h >= WX && h < 2 * WX) {
+            yflux(NR + 1, xh, m, fy);
+            for (int n = 0; n < 3; ++n) S.FY[n][NR][xh - 1] = fy[n];
         } else if (side && sx) {
-            xflux(sr + 1, 33, m, fx);
-            for (int n = 0; n < 3; ++n) S.FX[n][sr][32] = fx[n];
+            xflux(sr + 1, WX + 1, m, fx);
+            for (int n = 0; n < 3; ++n) S.FX[n][sr][WX] = fx[n];
         }
         __syncthreads();
         // ---- divergence and the mode's epilogue
@@ -758,7 +773,7 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
             const long long t = ((long long)k * g.ny + j) * g.nx + i;
 #pragma unroll
             for (int n = 0; n < 3; ++n) {
-                const double acc = ((S.FX[n][w][l + 1] - fx[n]) + (S.FY[n][w + 1][l] - fy[n])) + (fzn[n] - fz[n]);
+                const double acc = ((S.FX[n][y - 1][x] - fx[n]) + (S.FY[n][y][x - 1] - fy[n])) + (fzn[n] - fz[n]);
                 const long long o = n * N + t;
                 if constexpr (MODE == 0) {
                     out[o] = acc;
@@ -806,23 +821,29 @@ __global__ void __launch_bounds__(32 * (TY + 3), 2) k_divtau_col(Grid g, TauCoef
 // Launch shape: rows a block and layers a march.  A march does about 0.6
 // layers' work more than its layers (the low z face and two staged layers), and
 // an SM runs two blocks at a time, so the march is the one whose blocks, dealt
-// to 304 places, finish first: 96^3 takes 12 layers (177 us; 210 at 1, 232 at
-// 16), 128x128x64 16 (232; 217 at 4), 64^3 4 (66; 101 at
-// 12, 253 at 32), 256x256x128 16 (1571; 1544 at 8, 1886 at 1).  Blocks of 4
-// rows only where those of 8 leave places empty: 32x32x16 12 us against 16.
+// to 304 places, finish first: 96^3 takes 12 layers (169 us; 203 at 1, 222 at
+// 16), 64^3 4 (64; 68 at 1, 92 at 12, 229 at 32), 192x160x96 10 (548; 657 at 1,
+// 576 at 12), 256x256x128 16 (1498; 1471 at 10, 1847 at 1).  It is within 2 % of
+// the best of them but on 128x128x64, where it takes 16 layers (223 us) and 4
+// take 206.  Blocks of 4 rows only where those of 8 leave places empty: 32x32x16
+// 12 us against 15.  `narrow`: the forms of at most 16 columns, six blocks an SM.
 struct TauShape {
-    int ty, kc;
+    int ty, wx, kc;
     dim3 grid;
 };
-inline TauShape tau_shape(const Grid& g) {
-    TauShape s{8, 1, dim3(1, 1, 1)};
-    const int bx = (g.nx + 31) / 32;
-    if ((long long)bx * ((g.ny + 7) / 8) * g.nz < 304) s.ty = 4;  // small grids: more blocks
-    const int by = (g.ny + s.ty - 1) / s.ty;
+inline TauShape tau_shape(const Grid& g, bool narrow = false) {
+    TauShape s{8, 32, 1, dim3(1, 1, 1)};
+    if (narrow && g.nx <= 16) {
+        s.ty = 1;
+        s.wx = g.nx <= 4 ? 4 : (g.nx <= 8 ? 8 : 16);
+    }
+    const int bx = (g.nx + s.wx - 1) / s.wx;
+    if (s.wx == 32 && (long long)bx * ((g.ny + 7) / 8) * g.nz < 304) s.ty = 4;  // small grids: more blocks
+    const int rows = s.ty * (32 / s.wx), by = (g.ny + rows - 1) / rows, places = 152 * (s.wx == 32 ? 2 : kNarrowBlocks);
     double best = 0.0;
     for (int kc = 1; kc <= 16 && kc <= g.nz; ++kc) {
         const long long blocks = (long long)bx * by * ((g.nz + kc - 1) / kc);
-        const double cost = (double)((blocks + 303) / 304) * (kc + 0.6);
+        const double cost = (double)((blocks + places - 1) / places) * (kc + 0.6);
         if (kc == 1 || cost < best) {
             best = cost;
             s.kc = kc;
@@ -1327,15 +1348,23 @@ void launch_divtau_faces(Ctx& c, const Grid& g, const double* vel, const double*
 template <int MODE>
 static void launch_divtau_mode(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, const TauEpi& E,
                                double bytes) {
-    const TauShape s = tau_shape(g);
+    const TauShape s = tau_shape(g, MODE == 0);
     const TauCoef K = tau_coef(g);
-    const auto k4 = k_divtau_col<4, MODE>;
-    const auto k8 = k_divtau_col<8, MODE>;
+    if constexpr (MODE == 0) {
+        if (s.wx < 32) {
+            const auto run = s.wx == 4 ? k_divtau_col<1, 0, 4> : (s.wx == 8 ? k_divtau_col<1, 0, 8> : k_divtau_col<1, 0, 16>);
+            const size_t smem = s.wx == 4 ? sizeof(TauPlanes<1, 4>) : (s.wx == 8 ? sizeof(TauPlanes<1, 8>) : sizeof(TauPlanes<1, 16>));
+            KS_LAUNCH_SMEM_NAMED(c, "k_divtau_col", run, s.grid, 32 * 4, smem, bytes, g, K, vel, mueff, wg, out, E, s.kc);
+            return;
+        }
+    }
+    const auto k4 = k_divtau_col<4, MODE, 32>;
+    const auto k8 = k_divtau_col<8, MODE, 32>;
     if (s.ty == 4) {
-        KS_LAUNCH_SMEM_NAMED(c, "k_divtau_col", k4, s.grid, 32 * 7, sizeof(TauPlanes<4>), bytes, g, K, vel, mueff, wg, out, E, s.kc);
+        KS_LAUNCH_SMEM_NAMED(c, "k_divtau_col", k4, s.grid, 32 * 7, sizeof(TauPlanes<4, 32>), bytes, g, K, vel, mueff, wg, out, E, s.kc);
     } else {
-        cudaFuncSetAttribute(k8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TauPlanes<8>));
-        KS_LAUNCH_SMEM_NAMED(c, "k_divtau_col", k8, s.grid, 32 * 11, sizeof(TauPlanes<8>), bytes, g, K, vel, mueff, wg, out, E, s.kc);
+        cudaFuncSetAttribute(k8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TauPlanes<8, 32>));
+        KS_LAUNCH_SMEM_NAMED(c, "k_divtau_col", k8, s.grid, 32 * 11, sizeof(TauPlanes<8, 32>), bytes, g, K, vel, mueff, wg, out, E, s.kc);
     }
 }
 static void launch_divtau_col(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, const TauEpi& E,
@@ -1349,7 +1378,7 @@ static void launch_divtau_col(Ctx& c, const Grid& g, const double* vel, const do
         default: launch_divtau_mode<8>(c, g, vel, mueff, wg, out, E, bytes); break;
     }
 }
-static_assert(sizeof(TauPlanes<4>) <= 48 * 1024, "needs no shared memory attribute");
+static_assert(sizeof(TauPlanes<4, 32>) <= 48 * 1024, "needs no shared memory attribute");
 void launch_divtau(Ctx& c, const Grid& g, const double* vel, const double* mueff, const double* wg, double* out, int mode,
                    const double* src, double* forces, const double* base, const double* dold, double dt, double rho, int fp32,
                    const float* vel32) {
