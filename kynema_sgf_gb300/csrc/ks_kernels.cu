@@ -570,8 +570,9 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
 //   viscosity carries 1 / h^2 of the flux's own direction, so a flux enters the
 //   divergence by a subtraction alone;
 // - a march keeps the z faces and the in-plane differences of the next layer.
-// 72 FP64 instructions a cell and 6 for the halo, where the tile kernel's
-// per-face differences, repeated on the tile's halo, took about 130.
+// 79 FP64 instructions a cell with an epilogue, 5.6 for the halo and 26 a column
+// at the start of a march (counters, 256x256x64: 90.2 a cell), where the tile
+// kernel's per-face differences, repeated on the tile's halo, took about 130.
 // A block owns 32 x TY columns and keeps three layers of the velocity (with a
 // one-cell halo) and two of the viscosity in shared memory; the layer after
 // next is loaded while the current one is computed.  Its warps: one per row of
@@ -583,7 +584,7 @@ __global__ void __launch_bounds__(TTX* TTY* TTZ) k_divtau_tile(Grid g, const dou
 // WX < 32 (boxes of at most 16 columns in x, MODE 0): a warp holds 32 / WX rows
 // of WX columns, a block one such warp and the three of the halo.  On 32 lanes
 // a row of 4 leaves 28 idle: 4x256x256 351 us and 4x4x16384 621, where fluxes
-// formed face by face take 158 and 146 (193 and 183 under walls); 66 and 129 now.
+// formed face by face take 158 and 146 (193 and 183 under walls); 72 and 129 now.
 template <int TY, int WX>
 struct TauPlanes {
     static constexpr int NR = TY * (32 / WX);  // rows of a block

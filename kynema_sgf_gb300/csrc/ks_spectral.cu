@@ -481,9 +481,9 @@ void launch_spectral_solve(Ctx& c, const SpectralZ& Z, const double2* tw_x, cons
     const int np = (Z.nz + 1) / 2, rows = np * Z.ny;
     const double pts = (double)Z.nx * Z.ny * Z.nz, cb = 16.0 * np * Z.nx * Z.ny;
     // rows a block: about one radix-8 butterfly per thread of 128; columns a
-    // block: 8 neighbouring complex values are one 128-byte segment.  Both
-    // stay within 98 KB of shared memory (two blocks a SM) up to 3072 points
-    // a line, 131 KB at most.
+    // block: 8 neighbouring complex values are one 128-byte segment.  Shared
+    // memory up to 3072 points a line, two blocks an SM: 98 KB (y), 111 KB (x,
+    // whose rows are padded); at 4096 points 131 and 147 KB.
     const int lx = std::max(1, std::min(16, 1024 / X.n)), ly = Y.n <= 384 ? 8 : (Y.n <= 768 ? 4 : (Y.n <= 1536 ? 2 : 1));
     const size_t sx = 2 * sizeof(double2) * (size_t)lx * (X.n + X.n / 8 + 1), sy = 2 * sizeof(double2) * (size_t)ly * Y.n;
     const int tiles = (Z.nx + ly - 1) / ly, gx = (rows + lx - 1) / lx;
